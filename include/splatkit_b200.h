@@ -268,7 +268,7 @@ sk_status sk_get_stats(sk_context* ctx, sk_stats* out);
  * frame in flight first. */
 sk_status sk_set_timing(sk_context* ctx, uint32_t time_stages);
 /* How each binning cell's front-to-back list is built. SK_BINNING_AUTO: written in place from
- * per-block cell counts when the target has at most 4096 cells (32 x 32 pixels each), else by
+ * per-block counts (targets of up to 8192 x 8192 pixels at least), else by
  * a stable sort of (cell, splat) pairs; SK_BINNING_SORTED: always the sort. Both give the same
  * lists. Waits for the frame in flight first. */
 #define SK_BINNING_AUTO 0u
@@ -353,8 +353,8 @@ typedef struct {
                                  each warp's tile instances evenly over its lanes */
   uint32_t sort_tile_keys;    /* keys per radix-sort scatter tile: 2048, 4096 or 6144 */
   uint32_t lanes;             /* submissions in flight (<= the batch's lanes) */
-  uint32_t sorted_lists;      /* cell lists: 0 written in place per view where every view has at
-                                 most 4096 binning cells, 1 always by the batch-wide stable sort
+  uint32_t sorted_lists;      /* cell lists: 0 written in place per view (where every view's
+                                 target is one they fit), 1 always by the batch-wide stable sort
                                  of (cell, splat) pairs */
   double gpu_ms;              /* autotune: device time of the chosen kernels for the sample */
   double views_per_s;         /* autotune: throughput with `lanes` in flight, images read back */

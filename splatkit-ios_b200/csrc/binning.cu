@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kThreads) binEmitKernel(const __grid_constant_
           pending &= pending - 1;
           const uint4 sp = stage.span[j];
           const uint32_t val = stage.value[j], first = tileBase + stage.offset[j];
-          const uint32_t w = sp.y & 0xffffu, area = sp.y >> 16;
+          const uint32_t w = sp.y & 0xffffu, area = spanArea(sp);
           const TileGrid g = gridOf<kBatch>(a, stage, j, sp);
           auto emit = [&](uint32_t k, uint32_t slot) {
             if (slot < a.instanceCapacity) {
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kThreads) binEmitKernel(const __grid_constant_
         }
         const uint32_t j = lo, k = p - stage.offset[j];
         const uint4 sp = stage.span[j];
-        const uint32_t w = sp.y & 0xffffu, area = sp.y >> 16;
+        const uint32_t w = sp.y & 0xffffu, area = spanArea(sp);
         uint32_t bit = k;  // box position of the k-th listed tile
         if (area <= 64) {
           const uint32_t nlo = __popc(sp.z);

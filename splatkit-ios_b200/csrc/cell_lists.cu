@@ -1,23 +1,34 @@
-// Direct cell-major lists: each binning cell's front-to-back list of survivors, written in place.
+// Direct lists: each patch's front-to-back list of survivors, written in place.
 //
-// Binning + a stable sort of (cell, projected index) pairs by cell + a ranges pass build the
-// same lists (binning.cu, radix_sort.cu). On a target of at most kDirectMaxCells cells this file
-// builds them without the sort:
-//   1. count: every block of 512 depth ranks (1024 in a batch) histograms its instances by cell;
-//   2. scan: per cell, the running sum of the block histograms (32 cells per block of this pass,
-//      the rows held in registers) gives each block's first slot in the cell's list; the lists'
-//      starts come from a decoupled look-back across the groups of 32 cells, in cell order; the
-//      ranges and the instance count follow;
-//   3. emit: every block histograms its 8 warps' ranks (128 each) by cell again, so that warp w
-//      starts each cell after warps 0..w-1, then each warp walks its output 32 entries at a time
-//      in depth order and writes each entry at its cell's next slot (lanes of one round that
-//      share a cell take consecutive slots).
-// A batch of views runs each pass once for all of them (launchCellListsBatch): every block finds
-// its view in a table (its first count/emit block and first cell group), works on that view's
-// ranks, cells and workspace rows, and the look-back of pass 2 runs over the groups of all views
+// A patch is a square of 1, 2 or 4 binning cells a side (patchGrid). Its list holds, in depth order,
+// one entry per survivor whose box of cells touches it: the survivor's projected index and a bit
+// for each of the patch's cells it touches. A composite tile reads its patch's list and keeps the
+// entries with its cell's bit, which are the cell's front-to-back list that binning + a stable
+// sort of (cell, projected index) pairs by cell give (binning.cu, radix_sort.cu). On a target of at
+// most kDirectMaxPatches patches this file builds the lists without a sort:
+//   1. count: every block of depth ranks histograms its (survivor, patch) pairs by patch;
+//   2. scan: per patch, the running sum of the block histograms gives each block's first slot in
+//      the patch's list; the lists' starts come from a decoupled look-back across groups of 8
+//      patches, in patch order; the ranges and the entry count follow;
+//   3. emit: every block histograms its 8 warps' ranks by patch again, so that warp w starts each
+//      patch after warps 0..w-1, then each warp walks its output 32 entries at a time in depth order
+//      and writes each entry at its patch's next slot (lanes of one round that share a patch take
+//      consecutive slots).
+// A batch of views runs each pass once for all of them (launchPatchListsBatch): every block finds
+// its view in a table (its first count/emit block and first patch group), works on that view's
+// ranks, patches and workspace rows, and the look-back of pass 2 runs over the groups of all views
 // in order, so each view's entries start where the previous view's end.
-// Entries of a cell therefore appear in depth order, which is exactly what the stable sort
-// gives.
+//
+// Why patches and not cells on larger targets: a splat of 3 cells touches about 1.4 patches, and a grid of
+// 4 x 4 patches is 16 times coarser than the cell grid, so the block histograms of the three passes
+// (block x patch words) no longer dominate them, and a splat near the camera, whose box holds hundreds of
+// cells, is 16 times fewer entries for the one warp that writes them. The price is the composite's
+// filter. 1M splats at 1080p (2040 cells, 135 patches): the passes 105 -> 52 us against lists per cell,
+// the composite 193 -> 203. 3M at 3840 x 2160 (8160 cells, 510 patches): 164 us against 668 for the
+// stable sort of (cell, splat) pairs that lists per cell needed there. Small targets keep patches of one
+// cell: their cell grid is small, and many entries of a patch would miss a tile's cell (24 views of up
+// to 640 x 480: composite 1342 us, 1620 with 4 x 4 patches). The line at 320 patches: 1080p at 2 x 2
+// (510 patches) emits in 56 us and composites in 206, at 4 x 4 in 32 and 203.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -33,54 +44,56 @@ namespace {
 
 constexpr uint32_t kThreads = 256;
 constexpr uint32_t kWarps = kThreads / 32;
-// Ranks per lane: a frame's blocks take 512 depth ranks (100.8 -> 81.8 us for the three passes
-// against 1024-rank blocks), a batch's 1024 (it holds every view's block rows at once, and twice
-// the rows cost the 64-view batch more than the smaller blocks save).
-constexpr uint32_t kFrameItems = 2;
-constexpr uint32_t kBatchItems = 4;
-constexpr uint32_t kScanThreads = 1024;
-constexpr uint32_t kScanWarps = kScanThreads / 32;
-constexpr uint32_t kRowsInRegisters = 32;         // block rows one scan warp keeps
+// Depth ranks per lane: count and emission blocks take 512 depth ranks (1024: a frame's emission 32 ->
+// 50 us, the 24-view batch's 228 -> 262; 256: twice the rows to scan).
+constexpr uint32_t kItems = 2;
+constexpr uint32_t kBlockRanks = kThreads * kItems;
+constexpr uint32_t kScanThreads = 512;
+constexpr uint32_t kGroup = 8;                              // patches per scan block
+constexpr uint32_t kScanLanes = kScanThreads / kGroup;      // row lanes per patch
+constexpr uint32_t kRowsInRegisters = 16;                   // block rows one row lane keeps
+// Boxes of more patches than this are walked by the whole warp, smaller ones by their own lane.
+constexpr uint32_t kLanePatches = 8;
 
 struct Work {
-  uint32_t* blockRows;  // blocks x cells: each block's count per cell, then (after pass 2) its
-                        // first slot in each cell's list
-  uint64_t* status;     // one look-back word per group of 32 cells
+  uint32_t* blockRows;  // blocks x patches: each block's count per patch, then (after pass 2) its
+                        // first slot in each patch's list
+  uint64_t* status;     // one look-back word per group of patches
   // a whole batch in one launch (views non-null): the view table, each view's ranks
   // [viewFirst[v], viewFirst[v + 1]) of args.order, and the workspace its rows are in
-  const CellListView* views;
+  const PatchListView* views;
   uint32_t viewCount;
   const uint32_t* viewFirst;
   uint8_t* base;
 };
 
-// What one block of a pass works on: its block (or cell group) within its view, the view's ranks
-// [first, first + n) of the depth order, cells, workspace rows and cell ranges.
+// What one block of a pass works on: its block (or patch group) within its view, the view's ranks
+// [first, first + n) of the depth order, patches, workspace rows and patch ranges.
 struct Job {
-  uint32_t block, first, n, cells, tilesX;
+  uint32_t block, first, n, patches, patchesX, shift;
   uint32_t* blockRows;
   uint2* ranges;
 };
 
-__host__ __device__ inline uint32_t cellWords(uint32_t cells) { return (cells + 1) / 2; }
+__host__ __device__ inline uint32_t counterWords(uint32_t patches) { return (patches + 1) / 2; }
 __host__ __device__ inline size_t align16(size_t n) { return (n + 15) & ~size_t{15}; }
-__host__ __device__ inline uint32_t cellGroups(uint32_t cells) { return (cells + 31) / 32; }
-template <uint32_t kItems>
-__host__ __device__ inline uint32_t blocksFor(uint32_t capacity) {
-  constexpr uint32_t kBlockRanks = kThreads * kItems;
+__host__ __device__ inline uint32_t groupsOf(uint32_t patches) { return (patches + kGroup - 1) / kGroup; }
+__host__ __device__ inline uint32_t blocksOf(uint32_t capacity) {
   return (capacity + kBlockRanks - 1) / kBlockRanks;
 }
 
-// The job of block (or cell group, byGroup) `index` of a pass.
-__device__ __forceinline__ Job jobOf(const BinArgs& a, const Work& w, uint32_t cells,
+// The job of block (or patch group, byGroup) `index` of a pass.
+__device__ __forceinline__ Job jobOf(const BinArgs& a, const Work& w, uint32_t patches,
                                      uint32_t index, bool byGroup, uint2* ranges) {
   Job j;
   if (!w.views) {  // a frame: the ranks [0, count) of the depth order
     j.block = index;
     j.first = 0;
     j.n = min(*a.count, a.capacity);
-    j.cells = cells;
-    j.tilesX = a.tilesX;
+    const PatchGrid g = patchGrid(a.tilesX, a.tilesY);
+    j.patches = patches;
+    j.patchesX = g.x;
+    j.shift = g.shift;
     j.blockRows = w.blockRows;
     j.ranges = ranges;
     return j;
@@ -91,101 +104,173 @@ __device__ __forceinline__ Job jobOf(const BinArgs& a, const Work& w, uint32_t c
     const uint32_t start = byGroup ? w.views[mid].groupBase : w.views[mid].blockBase;
     if (start <= index) lo = mid; else hi = mid;
   }
-  const CellListView v = w.views[lo];
+  const PatchListView v = w.views[lo];
   j.block = index - (byGroup ? v.groupBase : v.blockBase);
   j.first = w.viewFirst[lo];
   j.n = min(w.viewFirst[lo + 1] - j.first, v.capacity);
-  j.cells = v.cells;
-  j.tilesX = v.tilesX;
+  j.patches = v.patches;
+  j.patchesX = v.patchesX;
+  j.shift = v.shift;
   j.blockRows = reinterpret_cast<uint32_t*>(w.base + v.work);
-  j.ranges = ranges + v.binBase;
+  j.ranges = ranges + v.patchBase;
   return j;
 }
 
-__host__ __device__ inline Work workOf(void* workspace, uint32_t blocks, uint32_t cells) {
-  uint8_t* p = static_cast<uint8_t*>(workspace);
+// A frame's workspace: the look-back words at a fixed place (whatever the target, so that they hold
+// nothing but look-back words), then the block rows.
+constexpr size_t kStatusBytes = size_t{kDirectMaxPatches / kGroup} * 8;
+
+Work workOf(void* workspace) {
   Work w{};
-  w.blockRows = reinterpret_cast<uint32_t*>(p);
-  p += align16(size_t{blocks} * cells * 4);
-  w.status = reinterpret_cast<uint64_t*>(p);
+  w.status = static_cast<uint64_t*>(workspace);
+  w.blockRows = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(workspace) + kStatusBytes);
   return w;
 }
 
-size_t workBytes(uint32_t blocks, uint32_t cells) {
-  return align16(size_t{blocks} * cells * 4) + size_t{cellGroups(cells)} * 8;
+// Entries of a span: its listed cells where a patch is one cell, else the patches of its box.
+__device__ __forceinline__ uint32_t entryCount(const uint4 s, uint32_t shift) {
+  if (shift == 0) return spanCount(s);
+  const PatchBox b = patchBox(s, shift);
+  return b.w * b.h;
 }
 
-// Pass 1: each block's instances per cell.
-template <uint32_t kItems>
+// visit(cell) for every listed cell of a masked box whose first cell is `first` (flat over the mask's
+// bits: rows walked one by one diverge more than the division per cell costs).
+template <typename Visit>
+__device__ __forceinline__ void visitListed(const uint4 s, uint32_t first, uint32_t tilesX, Visit visit) {
+  const uint32_t w = s.y & 0xffffu;
+  for (uint32_t m = s.z; m != 0u; m &= m - 1) visit(boxCell(first, __ffs(m) - 1, w, tilesX));
+  for (uint32_t m = s.w; m != 0u; m &= m - 1) visit(boxCell(first, 31 + __ffs(m), w, tilesX));
+}
+
+// visit(patch) for every entry of the warp's spans: a masked box of single-cell patches is walked bit
+// by bit and a box of at most kLanePatches patches patch by patch, by its own lane; a larger one by
+// the whole warp. Every lane of the warp calls this.
+template <typename Visit>
+__device__ __forceinline__ void visitPatches(const uint4 s, uint32_t shift, uint32_t patchesX, Visit visit) {
+  const PatchBox b = patchBox(s, shift);
+  const uint32_t lane = laneId(), first = b.y0 * patchesX + b.x0;
+  uint32_t area = b.w * b.h;
+  if (shift == 0 && area <= 64) {
+    visitListed(s, first, patchesX, visit);
+    area = 0;
+  }
+  if (area <= kLanePatches && area != 0) {
+    for (uint32_t y = 0; y < b.h; ++y)
+      for (uint32_t x = 0; x < b.w; ++x) visit(first + y * patchesX + x);
+  }
+  uint32_t big = __ballot_sync(0xffffffffu, area > kLanePatches);
+  while (big != 0u) {
+    const uint32_t src = __ffs(big) - 1;
+    big &= big - 1;
+    const uint32_t w = __shfl_sync(0xffffffffu, b.w, src), n = __shfl_sync(0xffffffffu, area, src);
+    const uint32_t at = __shfl_sync(0xffffffffu, first, src);
+    for (uint32_t k = lane; k < n; k += 32) visit(boxCell(at, k, w, patchesX));
+  }
+}
+
+// Pass 1: each block's entries per patch; the (survivor, cell) pairs are added up beside them.
 __global__ void __launch_bounds__(kThreads)
-    cellCountKernel(const __grid_constant__ BinArgs a, Work work, uint32_t cells) {
-  constexpr uint32_t kBlockRanks = kThreads * kItems;
+    patchCountKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches) {
   chainedKernelStart();
-  __shared__ uint32_t hist[kDirectMaxCells];
-  const Job job = jobOf(a, work, cells, blockIdx.x, false, nullptr);
+  extern __shared__ uint32_t hist[];
+  __shared__ uint32_t warpPairs[kWarps];
+  const Job job = jobOf(a, work, patches, blockIdx.x, false, nullptr);
   const uint32_t n = job.n;
-  cells = job.cells;
+  patches = job.patches;
   const uint32_t* order = a.order + job.first;
   const uint32_t begin = job.block * kBlockRanks;
   if (begin >= n) return;  // rows of idle blocks are never read
-  for (uint32_t c = threadIdx.x; c < cells; c += kThreads) hist[c] = 0;
-  __syncthreads();
   uint32_t value[kItems];
-  uint4 span[kItems];
 #pragma unroll
   for (uint32_t r = 0; r < kItems; ++r) {
     const uint32_t i = begin + r * kThreads + threadIdx.x;
     value[r] = i < n ? order[i] : 0xffffffffu;
   }
+  for (uint32_t c = threadIdx.x; c < patches; c += kThreads) hist[c] = 0;
+  __syncthreads();
+  uint4 span[kItems];
 #pragma unroll
   for (uint32_t r = 0; r < kItems; ++r)
     span[r] = value[r] != 0xffffffffu ? __ldg(a.spans + value[r]) : make_uint4(0, 0, 0, 0);
+  uint32_t pairs = 0;
 #pragma unroll
-  for (uint32_t r = 0; r < kItems; ++r)
-    visitCells(span[r], job.tilesX, [](uint32_t c) { atomicAdd(&hist[c], 1u); });
+  for (uint32_t r = 0; r < kItems; ++r) {
+    pairs += spanCount(span[r]);
+    visitPatches(span[r], job.shift, job.patchesX, [](uint32_t p) { atomicAdd(&hist[p], 1u); });
+  }
+  pairs = __reduce_add_sync(0xffffffffu, pairs);
+  if (laneId() == 0) warpPairs[threadIdx.x >> 5] = pairs;
   __syncthreads();
-  uint32_t* row = job.blockRows + size_t{job.block} * cells;
-  for (uint32_t c = threadIdx.x; c < cells; c += kThreads) row[c] = hist[c];
+  uint32_t* row = job.blockRows + size_t{job.block} * patches;
+  for (uint32_t c = threadIdx.x; c < patches; c += kThreads) row[c] = hist[c];
+  if (threadIdx.x == 0) {
+    uint32_t sum = 0;
+    for (uint32_t w = 0; w < kWarps; ++w) sum += warpPairs[w];
+    atomicAdd(a.instanceCount, sum);
+  }
 }
 
-// Pass 2: one block per group of 32 cells (groups handed out in start order, so a group only
-// waits on groups already running). Lane = cell of the group; warp w scans a contiguous share
-// of the block rows, the first 32 of them kept in registers between the two sweeps.
-template <uint32_t kItems>
-__global__ void __launch_bounds__(kScanThreads, 1)
-    cellScanKernel(const __grid_constant__ BinArgs a, Work work, uint32_t cells, uint2* ranges,
-                   uint32_t* counters, uint32_t epoch, uint32_t* error) {
+// Pass 2: one block per group of 8 patches (groups handed out in start order, so a group only
+// waits on groups already running). Thread t is row lane t / 8 of the group's patch t % 8: it sums
+// a contiguous share of the block rows, the first 16 of them kept in registers between the two
+// sweeps (a warp reads four rows' 32-byte sectors at a time).
+__global__ void __launch_bounds__(kScanThreads)
+    patchScanKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches, uint2* ranges,
+                    uint32_t* entryCount, uint32_t* counters, uint32_t epoch, uint32_t* error) {
   chainedKernelStart();
-  __shared__ uint32_t part[kScanWarps][33];
-  __shared__ uint32_t cellStart[32];
+  __shared__ uint32_t part[kScanLanes * kGroup];
+  __shared__ uint32_t totals[kGroup], starts[kGroup];
   const uint32_t group = takeTile(counters);  // over all views of a batch
-  const Job job = jobOf(a, work, cells, group, true, ranges);
-  cells = job.cells;
-  const uint32_t active = blocksFor<kItems>(job.n);
+  const Job job = jobOf(a, work, patches, group, true, ranges);
+  patches = job.patches;
+  const uint32_t active = blocksOf(job.n);
   const uint32_t warp = threadIdx.x >> 5, lane = laneId();
-  const uint32_t cell = job.block * 32 + lane;
-  const bool valid = cell < cells;
-  const uint32_t share = (active + kScanWarps - 1) / kScanWarps;
-  const uint32_t r0 = min(warp * share, active), r1 = min(r0 + share, active);
-  uint32_t* rows = job.blockRows + cell;
+  const uint32_t c = threadIdx.x % kGroup, rowLane = threadIdx.x / kGroup;
+  const uint32_t patch = job.block * kGroup + c;
+  const bool valid = patch < patches;
+  const uint32_t share = (active + kScanLanes - 1) / kScanLanes;
+  const uint32_t r0 = min(rowLane * share, active), r1 = min(r0 + share, active);
+  uint32_t* rows = job.blockRows + patch;
   uint32_t v[kRowsInRegisters];
   uint32_t sum = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kRowsInRegisters; ++k) {
     const uint32_t row = r0 + k;
-    v[k] = valid && row < r1 ? __ldcg(rows + size_t{row} * cells) : 0u;
+    v[k] = valid && row < r1 ? __ldcg(rows + size_t{row} * patches) : 0u;
     sum += v[k];
   }
-  if (valid)
-    for (uint32_t row = r0 + kRowsInRegisters; row < r1; ++row)
-      sum += __ldcg(rows + size_t{row} * cells);
-  part[warp][lane] = sum;
+  for (uint32_t at = r0 + kRowsInRegisters; at < r1; at += kRowsInRegisters) {
+#pragma unroll
+    for (uint32_t k = 0; k < kRowsInRegisters; ++k)
+      if (valid && at + k < r1) sum += __ldcg(rows + size_t{at + k} * patches);
+  }
+  part[threadIdx.x] = sum;
   __syncthreads();
-  uint32_t run = 0;
-  for (uint32_t w = 0; w < warp; ++w) run += part[w][lane];
+  if (warp < kGroup) {  // warp w: the running sum of patch w's 64 row lanes, two per lane
+    uint32_t own[kScanLanes / 32], total = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kScanLanes / 32; ++k) {
+      own[k] = part[(lane * (kScanLanes / 32) + k) * kGroup + warp];
+      total += own[k];
+    }
+    uint32_t inc = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t up = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= static_cast<uint32_t>(o)) inc += up;
+    }
+    uint32_t run = inc - total;
+#pragma unroll
+    for (uint32_t k = 0; k < kScanLanes / 32; ++k) {
+      part[(lane * (kScanLanes / 32) + k) * kGroup + warp] = run;
+      run += own[k];
+    }
+    if (lane == 31) totals[warp] = inc;
+  }
+  __syncthreads();
   if (warp == 0) {
-    uint32_t total = 0;
-    for (uint32_t w = 0; w < kScanWarps; ++w) total += part[w][lane];
+    const uint32_t total = lane < kGroup ? totals[lane] : 0u;
     uint32_t inc = total;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -203,138 +288,177 @@ __global__ void __launch_bounds__(kScanThreads, 1)
         storeStatus(work.status + group, makeStatus(epoch, kFlagPrefix, before + aggregate));
     }
     const uint32_t start = before + inc - total;
-    cellStart[lane] = start;
-    if (valid)
-      job.ranges[cell] = make_uint2(min(start, a.instanceCapacity),
-                                    min(start + total, a.instanceCapacity));
+    if (lane < kGroup) {
+      starts[lane] = start;
+      if (job.block * kGroup + lane < patches)
+        job.ranges[job.block * kGroup + lane] = make_uint2(min(start, a.instanceCapacity),
+                                                           min(start + total, a.instanceCapacity));
+    }
     if (group == gridDim.x - 1 && lane == 31) {
       const uint32_t entries = before + aggregate;
-      *a.instanceCount = entries;
+      *entryCount = entries;
       *a.overflow = entries > a.instanceCapacity ? 1u : 0u;
     }
   }
   __syncthreads();
-  if (valid) {  // each count becomes the block's first slot in the cell, in place
-    run += cellStart[lane];
+  if (valid) {  // each count becomes the block's first slot in the patch's list, in place
+    uint32_t run = part[threadIdx.x] + starts[c];
 #pragma unroll
     for (uint32_t k = 0; k < kRowsInRegisters; ++k) {
       const uint32_t row = r0 + k;
-      if (row < r1) rows[size_t{row} * cells] = run;
+      if (row < r1) rows[size_t{row} * patches] = run;
       run += v[k];
     }
-    for (uint32_t row = r0 + kRowsInRegisters; row < r1; ++row) {
-      const uint32_t count = __ldcg(rows + size_t{row} * cells);
-      rows[size_t{row} * cells] = run;
-      run += count;
+    // the rows past the registers, read again: a batch of loads, then their stores
+    for (uint32_t at = r0 + kRowsInRegisters; at < r1; at += kRowsInRegisters) {
+#pragma unroll
+      for (uint32_t k = 0; k < kRowsInRegisters; ++k)
+        v[k] = at + k < r1 ? __ldcg(rows + size_t{at + k} * patches) : 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < kRowsInRegisters; ++k) {
+        if (at + k < r1) rows[size_t{at + k} * patches] = run;
+        run += v[k];
+      }
     }
   }
   finishTile(counters);
 }
 
-// visit(cell, position, item) for every cell of the warp's items whose position offset + k lies
-// in [lo, hi); k numbers a span's cells as spanCell does (mask bits upward, or box order), item
-// is itemBase + the owning lane. A masked span is walked by its own lane, a box of more than 64
-// cells by the whole warp. Every lane calls this.
-template <typename Visit>
-__device__ __forceinline__ void visitPositions(const uint4 s, uint32_t tilesX, uint32_t offset,
-                                               uint32_t lo, uint32_t hi, uint32_t itemBase,
-                                               Visit visit) {
-  const uint32_t w = s.y & 0xffffu, area = s.y >> 16;
-  const uint32_t first = spanFirstCell(s, tilesX);
-  const uint32_t lane = laneId();
-  if (area <= 64 && offset < hi && offset + __popc(s.z) + __popc(s.w) > lo) {
-    uint32_t pos = offset;
-    for (uint32_t m = s.z; m != 0u; m &= m - 1, ++pos)
-      if (pos >= lo && pos < hi) visit(boxCell(first, __ffs(m) - 1, w, tilesX), pos, itemBase + lane);
-    for (uint32_t m = s.w; m != 0u; m &= m - 1, ++pos)
-      if (pos >= lo && pos < hi) visit(boxCell(first, 31 + __ffs(m), w, tilesX), pos, itemBase + lane);
-  }
-  uint32_t big = __ballot_sync(0xffffffffu, area > 64 && offset < hi && offset + area > lo);
-  while (big != 0u) {
-    const uint32_t src = __ffs(big) - 1;
-    big &= big - 1;
-    const uint32_t bw = __shfl_sync(0xffffffffu, w, src);
-    const uint32_t barea = __shfl_sync(0xffffffffu, area, src);
-    const uint32_t bfirst = __shfl_sync(0xffffffffu, first, src);
-    const uint32_t boff = __shfl_sync(0xffffffffu, offset, src);
-    const uint32_t k0 = lo > boff ? lo - boff : 0u, k1 = min(barea, hi - boff);
-    for (uint32_t k = k0 + lane; k < k1; k += 32) visit(boxCell(bfirst, k, bw, tilesX), boff + k, itemBase + src);
-  }
-}
-
 // Pass 3. Dynamic shared memory: kWarps x words per-warp slot counters (16-bit halves: a warp's
-// slots count from the block's first slot in the cell, at most 1024 on), then each cell's first
-// slot for the block. A warp's entries, in depth order, are staged as (cell, item) pairs kWindow
-// positions at a time: the counting walk stages the first window, and a warp with more entries
-// walks its items again for each further one.
-constexpr uint32_t kWindow = 1024;
+// slots count from the block's first slot in the patch, at most kBlockRanks on), then each patch's
+// first slot for the block. A warp's entries, in depth order, are worked out kWindow positions at a
+// time, one position per lane and step (however many patches the items have), and staged as
+// (patch, item, cell mask); a warp of more entries works each further window out when it writes it.
 
-template <uint32_t kItems>
 __global__ void __launch_bounds__(kThreads)
-    cellEmitKernel(const __grid_constant__ BinArgs a, Work work, uint32_t cells) {
+    patchEmitKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches) {
   constexpr uint32_t kChunk = 32 * kItems;  // ranks per warp
-  constexpr uint32_t kBlockRanks = kThreads * kItems;
+  constexpr uint32_t kWindow = 4 * kChunk;  // positions staged at a time
+  static_assert(kChunk < 256, "an item and a marker are bytes");
   chainedKernelStart();
-  extern __shared__ uint32_t cellSmem[];
-  __shared__ uint32_t stageValue[kWarps][kChunk];
-  __shared__ uint16_t stageCell[kWarps][kWindow];
-  __shared__ uint8_t stageItem[kWarps][kWindow];
-  const Job job = jobOf(a, work, cells, blockIdx.x, false, nullptr);
-  const uint32_t n = job.n, tilesX = job.tilesX;
-  cells = job.cells;
+  extern __shared__ uint32_t patchSmem[];
+  __shared__ uint4 itemSpan[kWarps][kChunk];
+  __shared__ uint32_t itemValue[kWarps][kChunk], itemOffset[kWarps][kChunk];
+  __shared__ uint16_t stagePatch[kWarps][kWindow], stageMask[kWarps][kWindow];
+  __shared__ alignas(4) uint8_t stageItem[kWarps][kWindow];
+  const Job job = jobOf(a, work, patches, blockIdx.x, false, nullptr);
+  const uint32_t n = job.n;
+  patches = job.patches;
   const uint32_t* order = a.order + job.first;
   const uint32_t begin = job.block * kBlockRanks;
   if (begin >= n) return;
-  const uint32_t words = cellWords(cells);
-  uint32_t* slots = cellSmem;
-  uint32_t* where = cellSmem + kWarps * words;
-  for (uint32_t i = threadIdx.x; i < kWarps * words; i += kThreads) slots[i] = 0;
-  const uint32_t* starts = job.blockRows + size_t{job.block} * cells;
-  for (uint32_t c = threadIdx.x; c < cells; c += kThreads) where[c] = __ldcg(starts + c);
-  __syncthreads();
-
   const uint32_t warp = threadIdx.x >> 5, lane = laneId();
-  uint32_t* mine = slots + warp * words;
-  uint32_t* sValue = stageValue[warp];
-  uint16_t* sCell = stageCell[warp];
-  uint8_t* sItem = stageItem[warp];
   uint32_t value[kItems];
-  uint4 span[kItems];
 #pragma unroll
   for (uint32_t r = 0; r < kItems; ++r) {
     const uint32_t i = begin + warp * kChunk + r * 32 + lane;
     value[r] = i < n ? order[i] : 0xffffffffu;
   }
+  const uint32_t words = counterWords(patches);
+  uint32_t* slots = patchSmem;
+  uint32_t* where = patchSmem + kWarps * words;
+  for (uint32_t i = threadIdx.x; i < kWarps * words; i += kThreads) slots[i] = 0;
+  const uint32_t* starts = job.blockRows + size_t{job.block} * patches;
+  for (uint32_t c = threadIdx.x; c < patches; c += kThreads) where[c] = __ldcg(starts + c);
+
+  uint32_t* mine = slots + warp * words;
+  uint16_t* sPatch = stagePatch[warp];
+  uint16_t* sMask = stageMask[warp];
+  uint8_t* sItem = stageItem[warp];
+  uint32_t* sOffset = itemOffset[warp];
   // the warp's items in (row, lane) order = depth order, with their first output position
-  uint32_t offset[kItems];
-  uint32_t total = 0;
+  uint32_t total = 0, listed = 0;  // listed: bit r when item r * 32 + lane has a patch
 #pragma unroll
   for (uint32_t r = 0; r < kItems; ++r) {
-    span[r] = value[r] != 0xffffffffu ? __ldg(a.spans + value[r]) : make_uint4(0, 0, 0, 0);
-    sValue[r * 32 + lane] = value[r];
-    const uint32_t cnt = spanCount(span[r]);
+    const uint4 span = value[r] != 0xffffffffu ? __ldg(a.spans + value[r]) : make_uint4(0, 0, 0, 0);
+    const uint32_t cnt = entryCount(span, job.shift);
     uint32_t inc = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t up = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= static_cast<uint32_t>(o)) inc += up;
     }
-    offset[r] = total + inc - cnt;
+    itemSpan[warp][r * 32 + lane] = span;
+    itemValue[warp][r * 32 + lane] = value[r];
+    sOffset[r * 32 + lane] = total + inc - cnt;
+    if (cnt) listed |= 1u << r;
     total += __shfl_sync(0xffffffffu, inc, 31);
   }
-  // count every entry by cell; stage the first window
+  __syncthreads();  // the counters are zero, the starts there
+
+  // Stages the entries at positions [w0, w1). Single-cell patches: every lane walks its items' listed
+  // cells (most items have one or two; a box of more than 64 cells is walked by the whole warp).
+  // Larger patches: one position per lane and step; every item marks its first position, and an
+  // entry's item is the last mark at or before its position (a running maximum).
+  auto stageWindow = [&](uint32_t w0, uint32_t w1, uint32_t& carry, bool count) {
+    if (job.shift == 0) {
+      auto put = [&](uint32_t patch, uint32_t pos, uint32_t item) {
+        if (pos < w0 || pos >= w1) return;
+        if (count) atomicAdd(mine + (patch >> 1), 1u << ((patch & 1u) * 16));
+        sPatch[pos - w0] = static_cast<uint16_t>(patch);
+        sMask[pos - w0] = 1u;
+        sItem[pos - w0] = static_cast<uint8_t>(item);
+      };
+#pragma unroll 1
+      for (uint32_t r = 0; r < kItems; ++r) {
+        const uint32_t item = r * 32 + lane;
+        const uint4 span = itemSpan[warp][item];
+        const uint32_t w = span.y & 0xffffu, area = spanArea(span);
+        const uint32_t first = (span.x >> 16) * job.patchesX + (span.x & 0xffffu);
+        uint32_t pos = sOffset[item];
+        if (area <= 64 && pos < w1) {
+          visitListed(span, first, job.patchesX, [&](uint32_t cell) { put(cell, pos++, item); });
+        }
+        uint32_t big = __ballot_sync(0xffffffffu, area > 64);
+        while (big != 0u) {
+          const uint32_t src = __ffs(big) - 1;
+          big &= big - 1;
+          const uint32_t bw = __shfl_sync(0xffffffffu, w, src), n = __shfl_sync(0xffffffffu, area, src);
+          const uint32_t at = __shfl_sync(0xffffffffu, first, src), from = __shfl_sync(0xffffffffu, pos, src);
+          for (uint32_t k = lane; k < n; k += 32) put(boxCell(at, k, bw, job.patchesX), from + k, r * 32 + src);
+        }
+      }
+      return;
+    }
+    for (uint32_t i = lane; i < kWindow / 4; i += 32) reinterpret_cast<uint32_t*>(sItem)[i] = 0u;
+    __syncwarp();
 #pragma unroll
-  for (uint32_t r = 0; r < kItems; ++r)
-    visitPositions(span[r], tilesX, offset[r], 0u, 0xffffffffu, r * 32,
-                   [mine, sCell, sItem](uint32_t c, uint32_t pos, uint32_t item) {
-                     atomicAdd(mine + (c >> 1), 1u << ((c & 1u) * 16));
-                     if (pos < kWindow) {
-                       sCell[pos] = static_cast<uint16_t>(c);
-                       sItem[pos] = static_cast<uint8_t>(item);
-                     }
-                   });
+    for (uint32_t r = 0; r < kItems; ++r) {
+      const uint32_t at = sOffset[r * 32 + lane];
+      if (((listed >> r) & 1u) && at >= w0 && at < w1) sItem[at - w0] = static_cast<uint8_t>(r * 32 + lane + 1);
+    }
+    __syncwarp();
+    for (uint32_t p0 = w0; p0 < w1; p0 += 32) {
+      const uint32_t p = p0 + lane;
+      uint32_t mark = p < w1 ? sItem[p - w0] : 0u;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, mark, o);
+        if (lane >= static_cast<uint32_t>(o)) mark = max(mark, up);
+      }
+      mark = max(mark, carry);
+      carry = __shfl_sync(0xffffffffu, mark, 31);
+      if (p < w1) {
+        const uint32_t item = mark - 1;
+        const uint4 span = itemSpan[warp][item];
+        const PatchBox box = patchBox(span, job.shift);
+        const uint32_t k = p - sOffset[item];
+        const uint32_t y = static_cast<uint32_t>(__fdividef(static_cast<float>(k) + 0.5f, static_cast<float>(box.w)));
+        const uint32_t px = box.x0 + (k - y * box.w), py = box.y0 + y;
+        const uint32_t patch = py * job.patchesX + px;
+        if (count) atomicAdd(mine + (patch >> 1), 1u << ((patch & 1u) * 16));
+        sPatch[p - w0] = static_cast<uint16_t>(patch);
+        sMask[p - w0] = static_cast<uint16_t>(patchMask(span, px, py, job.shift));
+        sItem[p - w0] = static_cast<uint8_t>(item);
+      }
+      __syncwarp();
+    }
+  };
+  // every entry counted by patch; a single window stays staged
+  for (uint32_t w0 = 0, carry = 0; w0 < total; w0 += kWindow)
+    stageWindow(w0, min(total, w0 + kWindow), carry, true);
   __syncthreads();
-  // warp w's first slot per cell: the counts of warps 0..w-1 (both halves of a word at once)
+  // warp w's first slot per patch: the counts of warps 0..w-1 (both halves of a word at once)
   for (uint32_t q = threadIdx.x; q < words; q += kThreads) {
     uint32_t run = 0;
 #pragma unroll
@@ -347,119 +471,117 @@ __global__ void __launch_bounds__(kThreads)
   __syncthreads();
 
   const uint32_t below = lanemaskLt();
-  for (uint32_t w0 = 0; w0 < total; w0 += kWindow) {
+  const uint32_t bits = 32 - __clz(max(patches, 2u) - 1);  // of a patch index: at most 12
+  for (uint32_t w0 = 0, carry = 0; w0 < total; w0 += kWindow) {
     const uint32_t w1 = min(total, w0 + kWindow);
-    if (w0 > 0) {  // stage the next window (its spans re-read from L2)
+    if (total > kWindow) {
       __syncwarp();
-#pragma unroll
-      for (uint32_t r = 0; r < kItems; ++r) {
-        const uint4 sp = value[r] != 0xffffffffu ? __ldg(a.spans + value[r]) : make_uint4(0, 0, 0, 0);
-        visitPositions(sp, tilesX, offset[r], w0, w1, r * 32,
-                       [sCell, sItem, w0](uint32_t c, uint32_t pos, uint32_t item) {
-                         sCell[pos - w0] = static_cast<uint16_t>(c);
-                         sItem[pos - w0] = static_cast<uint8_t>(item);
-                       });
-      }
+      stageWindow(w0, w1, carry, false);
     }
     __syncwarp();
     for (uint32_t p0 = w0; p0 < w1; p0 += 32) {
       const uint32_t p = p0 + lane;
       const bool valid = p < w1;
-      uint32_t cell = 0xffffffffu, val = 0;
+      uint32_t patch = 0, val = 0, mask = 0;
       if (valid) {
-        cell = sCell[p - w0];
-        val = sValue[sItem[p - w0]];
+        patch = sPatch[p - w0];
+        mask = sMask[p - w0];
+        val = itemValue[warp][sItem[p - w0]];
       }
-      // lanes of this round with the same cell: 13 ballots (cells are below 4096; an idle lane's
-      // 0xffffffff differs from every cell in bit 12)
-      uint32_t peers = 0xffffffffu;
+      // lanes of this round with the same patch: one ballot per bit of a patch index
+      uint32_t peers = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
-      for (uint32_t b = 0; b < 13; ++b) {
-        const bool bit = (cell >> b) & 1u;
-        const uint32_t vote = __ballot_sync(0xffffffffu, bit);
-        peers &= bit ? vote : ~vote;
+      for (uint32_t b = 0; b < 12; ++b) {
+        if (b < bits) {
+          const bool bit = (patch >> b) & 1u;
+          const uint32_t vote = __ballot_sync(0xffffffffu, bit);
+          peers &= bit ? vote : ~vote;
+        }
       }
-      const uint32_t half = (cell & 1u) * 16;
+      const uint32_t half = (patch & 1u) * 16;
       uint32_t slot = 0;
-      if (valid) slot = where[cell] + ((mine[cell >> 1] >> half) & 0xffffu) + __popc(peers & below);
+      if (valid) slot = where[patch] + ((mine[patch >> 1] >> half) & 0xffffu) + __popc(peers & below);
       __syncwarp();
-      if (valid && lane == 31 - __clz(peers)) atomicAdd(mine + (cell >> 1), __popc(peers) << half);
+      if (valid && lane == 31 - __clz(peers)) atomicAdd(mine + (patch >> 1), __popc(peers) << half);
       __syncwarp();
-      if (valid && slot < a.instanceCapacity) a.instanceValues[slot] = val;
+      if (valid && slot < a.instanceCapacity) {
+        a.instanceValues[slot] = val;
+        if (a.instanceMasks) a.instanceMasks[slot] = static_cast<uint16_t>(mask);
+      }
     }
   }
 }
 
-size_t emitDynamicBytes(uint32_t cells) {
-  return (size_t{kWarps} * cellWords(cells) + cells) * sizeof(uint32_t);
+size_t emitDynamicBytes(uint32_t patches) {
+  return (size_t{kWarps} * counterWords(patches) + patches) * sizeof(uint32_t);
 }
+
+size_t countDynamicBytes(uint32_t patches) { return size_t{patches} * sizeof(uint32_t); }
 
 }  // namespace
 
-bool cellListsFit(uint32_t capacity, uint32_t cells) {
-  return cells > 0 && cells <= kDirectMaxCells && capacity > 0;
+bool patchListsFit(uint32_t patches) { return patches > 0 && patches <= kDirectMaxPatches; }
+
+uint32_t patchListBlocks(uint32_t capacity) { return blocksOf(std::max(capacity, 1u)); }
+
+uint32_t patchListGroups(uint32_t patches) { return groupsOf(patches); }
+
+size_t patchListRowBytes(uint32_t capacity, uint32_t patches) {
+  return align16(size_t{patchListBlocks(capacity)} * patches * 4);
 }
 
-size_t cellListBytes(uint32_t capacity, uint32_t cells) {
-  return workBytes(blocksFor<kFrameItems>(std::max(capacity, 1u)), std::max(cells, 1u));
+size_t patchListBytes(uint32_t capacity, uint32_t patches) {
+  return kStatusBytes + patchListRowBytes(capacity, std::max(patches, 1u));
 }
 
-cudaError_t cellListsConfigure() {
+size_t patchListStatusBytes() { return kStatusBytes; }
+
+cudaError_t patchListsConfigure() {
   static bool configured = false;
   if (configured) return cudaSuccess;
-  cudaError_t e =
-      cudaFuncSetAttribute(cellEmitKernel<kFrameItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(emitDynamicBytes(kDirectMaxCells)));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(cellEmitKernel<kBatchItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(emitDynamicBytes(kDirectMaxCells)));
+  const int most = static_cast<int>(emitDynamicBytes(kDirectMaxPatches));
+  const cudaError_t e =
+      cudaFuncSetAttribute(patchEmitKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e == cudaSuccess) configured = true;
   return e;
 }
 
-cudaError_t launchCellLists(const BinArgs& a, const CellLists& lists, cudaStream_t stream) {
-  const uint32_t cells = lists.cells;
-  if (!cellListsFit(a.capacity, cells) || cells != a.tilesX * a.tilesY)
-    return cudaErrorInvalidValue;
-  cudaError_t e = cellListsConfigure();
-  if (e != cudaSuccess) return e;
-  const uint32_t blocks = blocksFor<kFrameItems>(a.capacity);
-  const Work work = workOf(lists.workspace, blocks, cells);
-  e = launchChained(cellCountKernel<kFrameItems>, blocks, kThreads, stream, a, work, cells);
-  if (e != cudaSuccess) return e;
-  e = launchChained(cellScanKernel<kFrameItems>, cellGroups(cells), kScanThreads, stream, a, work, cells,
-                    lists.ranges, lists.counters, lists.epoch, lists.error);
-  if (e != cudaSuccess) return e;
-  return launchChainedShared(cellEmitKernel<kFrameItems>, blocks, kThreads, emitDynamicBytes(cells), stream, a,
-                             work, cells);
+static cudaError_t launchPasses(const BinArgs& a, const Work& work, uint32_t patches, uint32_t blocks,
+                                uint32_t groups, uint2* ranges, uint32_t* entryCount, uint32_t* counters,
+                                uint32_t epoch, uint32_t* error, cudaStream_t stream) {
+  cudaError_t e = patchListsConfigure();
+  if (e == cudaSuccess)
+    e = launchChainedShared(patchCountKernel, blocks, kThreads, countDynamicBytes(patches), stream, a,
+                            work, patches);
+  if (e == cudaSuccess)
+    e = launchChained(patchScanKernel, groups, kScanThreads, stream, a, work, patches, ranges,
+                      entryCount, counters, epoch, error);
+  if (e == cudaSuccess)
+    e = launchChainedShared(patchEmitKernel, blocks, kThreads, emitDynamicBytes(patches), stream, a,
+                            work, patches);
+  return e;
 }
 
-uint32_t cellListBlocks(uint32_t capacity) { return blocksFor<kBatchItems>(std::max(capacity, 1u)); }
-
-size_t cellListRowBytes(uint32_t capacity, uint32_t cells) {
-  return align16(size_t{cellListBlocks(capacity)} * cells * 4);
+cudaError_t launchPatchLists(const BinArgs& a, const PatchLists& lists, cudaStream_t stream) {
+  const PatchGrid g = patchGrid(a.tilesX, a.tilesY);
+  const uint32_t patches = g.x * g.y;
+  if (!patchListsFit(patches) || a.capacity == 0) return cudaErrorInvalidValue;
+  return launchPasses(a, workOf(lists.workspace), patches, blocksOf(a.capacity),
+                                   groupsOf(patches), lists.ranges, lists.entryCount, lists.counters, lists.epoch, lists.error, stream);
 }
 
-cudaError_t launchCellListsBatch(const BinArgs& a, const CellListBatch& lists, cudaStream_t stream) {
-  if (lists.viewCount == 0 || lists.blocks == 0 || lists.groups == 0 || lists.mostCells == 0 ||
-      lists.mostCells > kDirectMaxCells)
+cudaError_t launchPatchListsBatch(const BinArgs& a, const PatchListBatch& lists, cudaStream_t stream) {
+  if (lists.viewCount == 0 || lists.blocks == 0 || lists.groups == 0 || !patchListsFit(lists.mostPatches))
     return cudaErrorInvalidValue;
-  cudaError_t e = cellListsConfigure();
-  if (e != cudaSuccess) return e;
   Work work{};
   work.status = lists.status;
   work.views = lists.views;
   work.viewCount = lists.viewCount;
   work.viewFirst = lists.viewFirst;
   work.base = static_cast<uint8_t*>(lists.workspace);
-  const uint32_t cells = lists.mostCells;  // each block reads its own view's from the table
-  e = launchChained(cellCountKernel<kBatchItems>, lists.blocks, kThreads, stream, a, work, cells);
-  if (e != cudaSuccess) return e;
-  e = launchChained(cellScanKernel<kBatchItems>, lists.groups, kScanThreads, stream, a, work, cells,
-                    lists.ranges, lists.counters, lists.epoch, lists.error);
-  if (e != cudaSuccess) return e;
-  return launchChainedShared(cellEmitKernel<kBatchItems>, lists.blocks, kThreads, emitDynamicBytes(cells),
-                             stream, a, work, cells);
+  // each block reads its own view's patches from the table
+  return launchPasses(a, work, lists.mostPatches, lists.blocks, lists.groups, lists.ranges, lists.entryCount,
+                      lists.counters, lists.epoch, lists.error, stream);
 }
 
 }  // namespace sk

@@ -122,8 +122,10 @@ struct BinArgs {
   uint32_t width, height, tilesX, tilesY;  // tilesX/Y: binning cells per row and column
   uint32_t* instanceKeys;    // binning cell per instance
   uint32_t* instanceValues;  // projected index per instance
+  uint16_t* instanceMasks;   // direct lists: the cells of its patch each entry touches (null: not
+                             // written, where every patch is one cell)
   uint32_t instanceCapacity;
-  uint32_t* instanceCount;  // FrameCounters.instances
+  uint32_t* instanceCount;  // FrameCounters.instances (the direct lists add to it: zero beforehand)
   uint32_t* overflow;       // FrameCounters.overflow
   uint32_t* blockSums;      // binBlocks(capacity) words of scratch
   // a batch (viewCount > 0): tile ids are batch-wide, each view's from its table entry
@@ -145,62 +147,67 @@ cudaError_t launchTileRanges(const uint32_t* sortedKeys, const uint32_t* instanc
                              uint32_t instanceCapacity, uint2* ranges, uint32_t tiles,
                              cudaStream_t stream);
 
-// Direct cell-major lists (cell_lists.cu): the per-cell lists that binning + stable tile sort +
-// ranges produce, written in place on targets of at most kDirectMaxCells binning cells. A count
-// pass histograms every block of 512 depth ranks (1024 in a batch) by cell, a scan pass turns the histograms
-// into each block's first position in every cell's list (and the lists' ranges, by look-back
-// across groups of cells), and the emission pass writes each instance there in depth order.
-// args.instanceValues receives the lists; instanceKeys and blockSums are unused.
-constexpr uint32_t kDirectMaxCells = 4096;
-struct CellLists {
-  uint32_t cells;       // binning cells of the target (args.tilesX * args.tilesY)
-  void* workspace;      // cellListBytes(capacity, cells), no clearing needed
-  uint2* ranges;        // per cell [start, end), clamped to the instance capacity
-  uint32_t* counters;   // two words, zero before the first launch (each launch restores them)
-  uint32_t epoch;       // look-back epoch, fresh per launch
-  uint32_t* error;      // SK_DEVERR_* bits
+// Direct lists (cell_lists.cu) on targets of at most kDirectMaxPatches patches (patchGrid): per patch, the front-to-back projected indices of the survivors whose cell box touches it, each
+// with the bits of the cells it touches there. A cell's entries are those of its patch with its
+// bit, the same list that binning + stable tile sort + ranges produce. args.instanceValues and
+// args.instanceMasks receive the entries, args.instanceCount the number of (survivor, cell) pairs;
+// instanceKeys and blockSums are unused.
+constexpr uint32_t kDirectMaxPatches = 4096;
+struct PatchLists {
+  void* workspace;       // patchListBytes(capacity, patches), the first patchListStatusBytes() zero
+                         // before the first launch
+  uint2* ranges;         // per patch [start, end), clamped to the instance capacity
+  uint32_t* entryCount;  // FrameCounters.entries
+  uint32_t* counters;    // two words, zero before the first launch (each launch restores them)
+  uint32_t epoch;        // look-back epoch, fresh per launch
+  uint32_t* error;       // SK_DEVERR_* bits
 };
-// Whether a target of `cells` cells takes the direct path.
-bool cellListsFit(uint32_t capacity, uint32_t cells);
-size_t cellListBytes(uint32_t capacity, uint32_t cells);
-cudaError_t launchCellLists(const BinArgs& args, const CellLists& lists, cudaStream_t stream);
+// Whether a target of `patches` patches takes the direct path.
+bool patchListsFit(uint32_t patches);
+size_t patchListBytes(uint32_t capacity, uint32_t patches);
+size_t patchListStatusBytes();
+cudaError_t launchPatchLists(const BinArgs& args, const PatchLists& lists, cudaStream_t stream);
 
 // Every view of a batch in one launch per pass. View v's ranks are [viewFirst[v], viewFirst[v+1])
-// of args.order (at most `capacity` of them), its cells binBase .. binBase + cells of the batch's
-// ranges; its count/emit blocks are blockBase .. blockBase + blocks (cellListBlocks(capacity)),
-// its cell groups groupBase .. groupBase + (cells + 31) / 32, and its block rows the
-// cellListRowBytes(capacity, cells) bytes at workspace + work. The look-back runs over the groups
-// of all views in view order, so view v's entries follow those of views 0..v-1; args.instanceCount
-// receives the total and args.overflow whether it exceeds args.instanceCapacity.
-struct CellListView {
-  uint32_t blockBase, groupBase, cells, tilesX;
-  uint32_t binBase, capacity, blocks, pad;
+// of args.order (at most `capacity` of them), its patches patchBase .. patchBase + patches of the
+// batch's ranges; its count/emit blocks are blockBase .. blockBase + patchListBlocks(capacity), its
+// patch groups groupBase .. groupBase + patchListGroups(patches), and its block rows the
+// patchListRowBytes(capacity, patches) bytes at workspace + work. The look-back runs over the
+// groups of all views in view order, so view v's entries follow those of views 0..v-1;
+// *entryCount receives the total and args.overflow whether it exceeds args.instanceCapacity.
+struct PatchListView {
+  uint32_t blockBase, groupBase, patches, patchesX;
+  uint32_t patchBase, capacity, shift, pad;
   uint64_t work;
 };
-struct CellListBatch {
-  const CellListView* views;  // device table, views in order
+struct PatchListBatch {
+  const PatchListView* views;  // device table, views in order
   uint32_t viewCount;
   const uint32_t* viewFirst;  // viewCount + 1 rank offsets (device)
   void* workspace;            // the views' block rows, no clearing needed
-  uint64_t* status;           // one look-back word per cell group of the batch, zero beforehand
-  uint2* ranges;              // the batch's cells
+  uint64_t* status;           // one look-back word per patch group of the batch, zero beforehand
+  uint2* ranges;              // the batch's patches
+  uint32_t* entryCount;
   uint32_t* counters;         // two words, zero before the first launch (each launch restores them)
   uint32_t epoch;
   uint32_t* error;
-  uint32_t blocks, groups, mostCells;  // totals over the views; the largest view's cells
+  uint32_t blocks, groups, mostPatches;  // totals over the views; the largest view's patches
 };
-uint32_t cellListBlocks(uint32_t capacity);
-size_t cellListRowBytes(uint32_t capacity, uint32_t cells);
-cudaError_t launchCellListsBatch(const BinArgs& args, const CellListBatch& lists, cudaStream_t stream);
+uint32_t patchListBlocks(uint32_t capacity);
+uint32_t patchListGroups(uint32_t patches);
+size_t patchListRowBytes(uint32_t capacity, uint32_t patches);
+cudaError_t launchPatchListsBatch(const BinArgs& args, const PatchListBatch& lists, cudaStream_t stream);
 // Sets the emission kernel's shared-memory limit (once; before any stream capture).
-cudaError_t cellListsConfigure();
+cudaError_t patchListsConfigure();
 
 // ---- composite (composite.cu) ----------------------------------------------------------
 enum PixelFormat : int { kRgba8 = 0, kRgba32f = 1 };
 struct CompositeArgs {
   const Projected* projected;
-  const uint32_t* values;  // tile-sorted projected indices
-  const uint2* ranges;  // per binning cell
+  const uint32_t* values;  // list entries' projected indices, front to back
+  const uint16_t* masks;   // direct lists: each entry's cells of its patch; null: lists per cell
+  uint32_t patches;        // a batch: 1 when the views' lists start at their patchBase (else binBase)
+  const uint2* ranges;     // per patch (direct lists) or per binning cell
   uint32_t width, height, tilesX, tilesY;  // composite tiles (kTileSize pixels)
   uint32_t binsX;                          // binning cells per row
   float background[3];

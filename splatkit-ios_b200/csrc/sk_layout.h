@@ -101,14 +101,15 @@ struct LodState {
 // Per-frame device counters the host reads back after a frame completes.
 struct FrameCounters {
   uint32_t visible;       // survivors of the cull
-  uint32_t instances;     // tile instances the binning needed
-  uint32_t overflow;      // 1 when instances exceeded the reserved capacity
+  uint32_t instances;     // (splat, cell) pairs of the frame
+  uint32_t overflow;      // 1 when the list entries exceeded the reserved capacity
   uint32_t error;         // SK_DEVERR_* bits
   uint32_t lod[6];        // LOD counters of this frame
   uint32_t fragments_lo;  // blended fragments (pixel x splat), when counted
   uint32_t fragments_hi;
   uint32_t loaded;  // tile-list records the composite read before its tiles terminated
-  uint32_t pad[3];
+  uint32_t entries;  // list entries written: (splat, patch) or (splat, cell) pairs
+  uint32_t pad[2];
 };
 static_assert(sizeof(FrameCounters) == 64, "FrameCounters is 64 bytes");
 
@@ -132,6 +133,27 @@ constexpr uint32_t kTileSize = 16;  // composite tile edge in pixels
 // (about 2.6x fewer list entries than per tile at 1080p); each composite tile reads its cell's
 // list and keeps, per warp quadrant, only the splats that reach it.
 constexpr uint32_t kBinSize = 2 * kTileSize;
+// Patch: a square of 1, 2 or 4 binning cells a side (a shift of 0, 1 or 2), the unit of the direct
+// lists: one entry per splat and patch it touches, with a bit for each of the patch's cells it
+// touches (bit (y % edge) * edge + x % edge of cell (x, y)).
+constexpr uint32_t kPatchShiftMost = 2;
+constexpr uint32_t kPatchGoal = 320;
+struct PatchGrid {
+  uint32_t shift, x, y;  // log2 of the edge; patches per row and column
+};
+// The patches of a target of binsX x binsY cells: the smallest edge with at most kPatchGoal patches.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline PatchGrid patchGrid(uint32_t binsX, uint32_t binsY) {
+  PatchGrid g{0, binsX, binsY};
+  while (g.shift < kPatchShiftMost && g.x * g.y > kPatchGoal) {
+    ++g.shift;
+    g.x = (binsX + (1u << g.shift) - 1) >> g.shift;
+    g.y = (binsY + (1u << g.shift) - 1) >> g.shift;
+  }
+  return g;
+}
 
 // One view of a batch (device table, 96 bytes): the world range it draws (or, for a LOD world,
 // the cut its selection wrote), where its work items, tiles and pixels start in the batch-wide
@@ -154,7 +176,7 @@ struct alignas(16) BatchView {
                                // order (null: the range offset .. offset + count)
   const uint32_t* indexCount;  // a LOD view: the cut's length (device word); count bounds it
   uint32_t worldCount;         // records of the world (every cut index is below it)
-  uint32_t pad;
+  uint32_t patchBase;          // first batch-wide patch of this view
 };
 static_assert(sizeof(BatchView) == 96, "BatchView is 96 bytes");
 

@@ -6,9 +6,9 @@
 // square is the pixel area, half a pixel beyond every pixel centre, so the test can only keep
 // too many cells, never drop one the compositor would cover. ("Tile" below means a cell.)
 //
-// A span packs the result in 16 bytes: (x0 | y0 << 16, width | area << 16, mask lo, mask hi),
+// A span packs the result in 16 bytes: (x0 | y0 << 16, width | height << 16, mask lo, mask hi),
 // bit k of the mask standing for box tile (x0 + k % width, y0 + k / width). A box of more than
-// 64 tiles keeps all of them (its mask is unused); area 0 means no tile.
+// 64 tiles keeps all of them (its mask is unused); a width of 0 means no tile.
 #pragma once
 #include "sk_device.cuh"
 
@@ -74,13 +74,16 @@ __device__ __forceinline__ uint4 tileSpan(const uint4 lo, const uint4 hi, float 
     }
     if (mask == 0) return make_uint4(0, 0, 0, 0);
   }
-  return make_uint4(x0 | (y0 << 16), w | (area << 16), static_cast<uint32_t>(mask),
+  return make_uint4(x0 | (y0 << 16), w | ((y1 - y0 + 1) << 16), static_cast<uint32_t>(mask),
                     static_cast<uint32_t>(mask >> 32));
 }
 
+// Tiles of a span's box.
+__device__ __forceinline__ uint32_t spanArea(const uint4 s) { return (s.y & 0xffffu) * (s.y >> 16); }
+
 // Tiles a span lists.
 __device__ __forceinline__ uint32_t spanCount(const uint4 s) {
-  const uint32_t area = s.y >> 16;
+  const uint32_t area = spanArea(s);
   if (area > 64) return area;
   return static_cast<uint32_t>(__popc(s.z) + __popc(s.w));
 }
@@ -111,41 +114,39 @@ __device__ __forceinline__ uint32_t boxCell(uint32_t first, uint32_t b, uint32_t
   return first + q * tilesX + (b - q * w);
 }
 
-// First cell of a span's box on a grid tilesX cells wide.
-__device__ __forceinline__ uint32_t spanFirstCell(const uint4 s, uint32_t tilesX) {
-  return (s.x >> 16) * tilesX + (s.x & 0xffffu);
+// ---- patches (sk_layout.h) --------------------------------------------------------------
+struct PatchBox {
+  uint32_t x0, y0, w, h;  // first patch, patches per row and column; w 0: none
+};
+
+// The patches of 2^shift cells a side that a span's box touches.
+__device__ __forceinline__ PatchBox patchBox(const uint4 s, uint32_t shift) {
+  const uint32_t x0 = s.x & 0xffffu, y0 = s.x >> 16, w = s.y & 0xffffu, h = s.y >> 16;
+  PatchBox b;
+  b.x0 = x0 >> shift;
+  b.y0 = y0 >> shift;
+  b.w = w ? ((x0 + w - 1) >> shift) - b.x0 + 1 : 0u;
+  b.h = w ? ((y0 + h - 1) >> shift) - b.y0 + 1 : 0u;
+  return b;
 }
 
-// The k-th (from 0) cell a span lists, k < spanCount(s).
-__device__ __forceinline__ uint32_t spanCell(const uint4 s, uint32_t k, uint32_t tilesX) {
-  const uint32_t w = s.y & 0xffffu, area = s.y >> 16;
-  uint32_t bit = k;
-  if (area <= 64) {
-    const uint32_t nlo = __popc(s.z);
-    bit = k < nlo ? kthSetBit(s.z, k) : 32u + kthSetBit(s.w, k - nlo);
+// The cells of patch (px, py) a span lists (0 when its box only touches the patch).
+__device__ __forceinline__ uint32_t patchMask(const uint4 s, uint32_t px, uint32_t py, uint32_t shift) {
+  const uint32_t x0 = s.x & 0xffffu, y0 = s.x >> 16, w = s.y & 0xffffu, h = s.y >> 16;
+  const uint32_t cx = px << shift, cy = py << shift, edge = 1u << shift;
+  const uint32_t xa = max(x0, cx), xb = min(x0 + w, cx + edge);
+  const uint32_t ya = max(y0, cy), yb = min(y0 + h, cy + edge);
+  const uint32_t row = (1u << (xb - xa)) - 1u;
+  const bool masked = w * h <= 64;
+  uint32_t out = 0;
+  uint32_t at = (ya - y0) * w + (xa - x0);  // the row's first bit of the box mask
+  uint32_t to = ((ya - cy) << shift) + (xa - cx);
+  for (uint32_t y = ya; y < yb; ++y, at += w, to += edge) {
+    uint32_t bits = row;
+    if (masked) bits &= at < 32 ? __funnelshift_r(s.z, s.w, at) : s.w >> (at - 32);
+    out |= bits << to;
   }
-  return boxCell(spanFirstCell(s, tilesX), bit, w, tilesX);
-}
-
-// visit(cell) for every cell a span lists. A masked span is walked by its own lane; a box of
-// more than 64 cells by the whole warp. Every lane of the warp calls this.
-template <typename Visit>
-__device__ __forceinline__ void visitCells(const uint4 s, uint32_t tilesX, Visit visit) {
-  const uint32_t w = s.y & 0xffffu, area = s.y >> 16;
-  const uint32_t first = spanFirstCell(s, tilesX);
-  if (area <= 64) {
-    for (uint32_t m = s.z; m != 0u; m &= m - 1) visit(boxCell(first, __ffs(m) - 1, w, tilesX));
-    for (uint32_t m = s.w; m != 0u; m &= m - 1) visit(boxCell(first, 31 + __ffs(m), w, tilesX));
-  }
-  uint32_t big = __ballot_sync(0xffffffffu, area > 64);
-  while (big != 0u) {
-    const uint32_t src = __ffs(big) - 1;
-    big &= big - 1;
-    const uint32_t bw = __shfl_sync(0xffffffffu, w, src);
-    const uint32_t barea = __shfl_sync(0xffffffffu, area, src);
-    const uint32_t bfirst = __shfl_sync(0xffffffffu, first, src);
-    for (uint32_t k = threadIdx.x & 31u; k < barea; k += 32) visit(boxCell(bfirst, k, bw, tilesX));
-  }
+  return out;
 }
 
 }  // namespace sk

@@ -5,9 +5,9 @@
 // pipeline's, each launched once over the whole batch:
 //   visibility (all views, one look-back chain: survivors contiguous in (view, source) order,
 //   key = view << 16 | 16-bit depth key) -> one stable radix sort of those keys (every view's
-//   depth order, views back to back) -> binning with batch-wide tile ids -> stable tile sort ->
-//   tile ranges -> composite of every tile of every view -> images, survivor counts and
-//   counters copied to pinned memory.
+//   depth order, views back to back) -> every view's patch lists (or binning with batch-wide tile
+//   ids, stable tile sort and ranges) -> composite of every tile of every view -> images, survivor
+//   counts and counters copied to pinned memory.
 // A view of a LOD world selects its cut first (on the lane's stream, with its context's current
 // threshold) and its visibility items draw the cut instead of a range.
 // The arithmetic per view is the plain frame's, so the images and counts equal sk_draw's.
@@ -277,44 +277,52 @@ sk_status Batch::prepare(BatchLane& l, const sk_batch_view* views, uint32_t coun
       t.indexCount = static_cast<const uint32_t*>(l.lodReports.ptr) + k * 8;  // report word 0
     }
   }
-  // Every view's lists written in place when each has at most kDirectMaxCells cells.
-  uint32_t mostCells = 1;
-  for (const BatchView& t : l.table) mostCells = std::max(mostCells, t.binsX * t.binsY);
-  l.directLists = !tuning.sortedLists && mostCells <= kDirectMaxCells &&
-                  cellListsConfigure() == cudaSuccess;
+  // Every view's lists written in place when each has at most kDirectMaxPatches patches.
+  uint32_t mostPatches = 1;
+  l.patchMasks = false;
+  for (const BatchView& t : l.table) {
+    const PatchGrid g = patchGrid(t.binsX, t.binsY);
+    mostPatches = std::max(mostPatches, g.x * g.y);
+    if (g.shift) l.patchMasks = true;  // patches of one cell need no masks
+  }
+  l.directLists = !tuning.sortedLists && patchListsFit(mostPatches) &&
+                  patchListsConfigure() == cudaSuccess;
   if (l.directLists) {
-    // view v's count/emit blocks, cell groups and block rows follow those of views 0..v-1
-    CellListBatch& cb = l.cellBatch;
-    cb = CellListBatch{};
-    cb.viewCount = count;
-    cb.mostCells = mostCells;
-    std::vector<CellListView> cellViews(count);
+    // view v's count/emit blocks, patches, patch groups and block rows follow those of views 0..v-1
+    PatchListBatch& pb = l.patchBatch;
+    pb = PatchListBatch{};
+    pb.viewCount = count;
+    pb.mostPatches = mostPatches;
+    std::vector<PatchListView> patchViews(count);
     uint64_t rowBytes = 0;
+    uint32_t patches = 0;
     for (uint32_t v = 0; v < count; ++v) {
-      const BatchView& t = l.table[v];
-      CellListView& c = cellViews[v];
+      BatchView& t = l.table[v];
+      PatchListView& c = patchViews[v];
       c.capacity = std::max(t.count, 1u);
-      c.cells = t.binsX * t.binsY;
-      c.tilesX = t.binsX;
-      c.binBase = t.binBase;
-      c.blocks = cellListBlocks(c.capacity);
-      c.blockBase = cb.blocks;
-      c.groupBase = cb.groups;
+      const PatchGrid g = patchGrid(t.binsX, t.binsY);
+      c.patches = g.x * g.y;
+      c.patchesX = g.x;
+      c.shift = g.shift;
+      c.patchBase = t.patchBase = patches;
+      c.blockBase = pb.blocks;
+      c.groupBase = pb.groups;
       c.work = rowBytes;
-      cb.blocks += c.blocks;
-      cb.groups += (c.cells + 31) / 32;
-      rowBytes += cellListRowBytes(c.capacity, c.cells);
+      patches += c.patches;
+      pb.blocks += patchListBlocks(c.capacity);
+      pb.groups += patchListGroups(c.patches);
+      rowBytes += patchListRowBytes(c.capacity, c.patches);
     }
-    void* before[3] = {l.cellLists.ptr, l.cellStatus.ptr, l.cellViews.ptr};
-    cudaError_t e = l.cellLists.allocateOn(
-        rowBytes > l.cellLists.bytes ? std::max<uint64_t>(rowBytes, l.cellLists.bytes + l.cellLists.bytes / 2)
-                                     : rowBytes, l.stream);
-    if (e == cudaSuccess) e = l.cellStatus.allocateOn(size_t{cb.groups} * 8, l.stream);
-    if (e == cudaSuccess) e = l.cellViews.allocateOn(size_t{count} * sizeof(CellListView), l.stream);
-    if (e == cudaSuccess) e = l.hostCellViews.allocate(size_t{count} * sizeof(CellListView));
-    if (e != cudaSuccess) return check(e, "batch cell lists");
-    std::memcpy(l.hostCellViews.ptr, cellViews.data(), size_t{count} * sizeof(CellListView));
-    if (before[0] != l.cellLists.ptr || before[1] != l.cellStatus.ptr || before[2] != l.cellViews.ptr) {
+    void* before[3] = {l.patchLists.ptr, l.patchStatus.ptr, l.patchViews.ptr};
+    cudaError_t e = l.patchLists.allocateOn(
+        rowBytes > l.patchLists.bytes ? std::max<uint64_t>(rowBytes, l.patchLists.bytes + l.patchLists.bytes / 2)
+                                      : rowBytes, l.stream);
+    if (e == cudaSuccess) e = l.patchStatus.allocateOn(size_t{pb.groups} * 8, l.stream);
+    if (e == cudaSuccess) e = l.patchViews.allocateOn(size_t{count} * sizeof(PatchListView), l.stream);
+    if (e == cudaSuccess) e = l.hostPatchViews.allocate(size_t{count} * sizeof(PatchListView));
+    if (e != cudaSuccess) return check(e, "batch lists");
+    std::memcpy(l.hostPatchViews.ptr, patchViews.data(), size_t{count} * sizeof(PatchListView));
+    if (before[0] != l.patchLists.ptr || before[1] != l.patchStatus.ptr || before[2] != l.patchViews.ptr) {
       if (l.graph) cudaGraphExecDestroy(l.graph);  // a captured graph points at the old buffers
       l.graph = nullptr;
       l.graphShape.clear();
@@ -338,12 +346,12 @@ sk_status Batch::enqueueStages(BatchLane& l, bool clearStatus) {
   if (e == cudaSuccess && !l.directLists)
     e = clearTileRanges(static_cast<uint2*>(l.ranges.ptr), l.totalBins, s);
   if (e == cudaSuccess && l.directLists) {
-    // the look-back words of the batch's cell groups must read "not ready" (a replayed graph
+    // the look-back words of the batch's patch groups must read "not ready" (a replayed graph
     // reuses its epochs); the view table goes up with the other tables
-    e = cudaMemsetAsync(l.cellStatus.ptr, 0, size_t{l.cellBatch.groups} * 8, s);
+    e = cudaMemsetAsync(l.patchStatus.ptr, 0, size_t{l.patchBatch.groups} * 8, s);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(l.cellViews.ptr, l.hostCellViews.ptr,
-                          size_t{l.viewCount} * sizeof(CellListView), cudaMemcpyHostToDevice, s);
+      e = cudaMemcpyAsync(l.patchViews.ptr, l.hostPatchViews.ptr,
+                          size_t{l.viewCount} * sizeof(PatchListView), cudaMemcpyHostToDevice, s);
   }
   if (e == cudaSuccess && clearStatus) {
     e = cudaMemsetAsync(l.visStatus.ptr, 0, size_t{l.totalItems} * 8, s);
@@ -419,27 +427,28 @@ sk_status Batch::enqueueStages(BatchLane& l, bool clearStatus) {
   }
   if (e == cudaSuccess && l.directLists) {
     // every view's lists in one launch per pass: view v's ranks are order[viewFirst[v] ..
-    // viewFirst[v + 1]) (views in order by the key's high bits), its cells binBase .. binBase +
-    // binsX * binsY of the batch
+    // viewFirst[v + 1]) (views in order by the key's high bits), its patches from its patchBase on
     BinArgs b{};
     b.spans = static_cast<const uint4*>(l.spans.ptr);
     b.order = static_cast<const uint32_t*>(l.order.ptr);
     b.count = &fc->visible;
     b.capacity = l.sources;
     b.instanceValues = static_cast<uint32_t*>(l.instValuesSorted.ptr);
+    b.instanceMasks = l.patchMasks ? static_cast<uint16_t*>(l.instKeysSorted.ptr) : nullptr;
     b.instanceCapacity = l.instances;
     b.instanceCount = &fc->instances;
     b.overflow = &fc->overflow;
-    CellListBatch cl = l.cellBatch;
-    cl.views = static_cast<const CellListView*>(l.cellViews.ptr);
-    cl.viewFirst = viewFirst;
-    cl.workspace = l.cellLists.ptr;
-    cl.status = static_cast<uint64_t*>(l.cellStatus.ptr);
-    cl.ranges = static_cast<uint2*>(l.ranges.ptr);
-    cl.counters = counters + 8;
-    cl.epoch = nextEpoch(1);
-    cl.error = error;
-    e = launchCellListsBatch(b, cl, s);
+    PatchListBatch pl = l.patchBatch;
+    pl.views = static_cast<const PatchListView*>(l.patchViews.ptr);
+    pl.viewFirst = viewFirst;
+    pl.workspace = l.patchLists.ptr;
+    pl.status = static_cast<uint64_t*>(l.patchStatus.ptr);
+    pl.ranges = static_cast<uint2*>(l.ranges.ptr);
+    pl.entryCount = &fc->entries;
+    pl.counters = counters + 8;
+    pl.epoch = nextEpoch(1);
+    pl.error = error;
+    e = launchPatchListsBatch(b, pl, s);
   }
   if (e == cudaSuccess && !l.directLists) {
     BinArgs b{};
@@ -481,6 +490,7 @@ sk_status Batch::enqueueStages(BatchLane& l, bool clearStatus) {
     CompositeArgs c{};
     c.projected = static_cast<const Projected*>(l.projected.ptr);
     c.values = static_cast<const uint32_t*>(l.instValuesSorted.ptr);
+    c.masks = l.directLists && l.patchMasks ? static_cast<const uint16_t*>(l.instKeysSorted.ptr) : nullptr;
     c.ranges = static_cast<const uint2*>(l.ranges.ptr);
     for (int j = 0; j < 3; ++j) c.background[j] = static_cast<float>(policy.background[j]);
     c.opaque = 1;
@@ -491,6 +501,7 @@ sk_status Batch::enqueueStages(BatchLane& l, bool clearStatus) {
     c.countFragments = 1;
     c.loaded = &fc->loaded;
     c.views = views;
+    c.patches = l.directLists ? 1u : 0u;
     c.viewCount = l.viewCount;
     c.batchTiles = l.totalTiles;
     e = launchComposite(c, s);
@@ -597,8 +608,9 @@ sk_status Batch::finish(BatchLane& l, bool wait) {
   FrameCounters c = *static_cast<const FrameCounters*>(l.hostCounters.ptr);
   if (c.overflow) {
     // Grow the instance buffers to what the batch needed and draw it again.
+    const uint32_t most = std::max(c.instances, c.entries);
     const uint32_t need = static_cast<uint32_t>(std::min<uint64_t>(
-        uint64_t{c.instances} + c.instances / 4 + 1024, 0x7fffffffu));
+        uint64_t{most} + most / 4 + 1024, 0x7fffffffu));
     sk_status st = reserve(l, l.sources, need, l.items, l.tiles, l.views, l.pixels);
     if (st == SK_OK) st = enqueue(l);
     if (st != SK_OK) {

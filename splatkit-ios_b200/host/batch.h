@@ -35,7 +35,7 @@ struct BatchTuning {
   bool graphs = false;          // replay captured stage sequences
   bool balancedEmit = true;     // binning emission strategy (BinArgs::balanced)
   uint32_t sortTileKeys = 4096; // keys per radix scatter tile: 2048, 4096 or 6144
-  bool sortedLists = false;     // cell lists by the batch-wide sort even where in place fits
+  bool sortedLists = false;     // lists by the batch-wide sort even where direct ones fit
 };
 
 // The selection one LOD view of a submission runs (LodArgs less the lane's scratch).
@@ -58,12 +58,13 @@ struct BatchLane {
   DeviceBuffer keys, projected, spans, order, sortWorkspace, visStatus, binSums;
   DeviceBuffer instKeys, instValues, instKeysSorted, instValuesSorted, tileSortWorkspace;
   DeviceBuffer ranges, viewFirst, counters, frameCounters, viewTable, cameras, image;
-  // direct cell lists (every view at most kDirectMaxCells cells), all views in one launch per
-  // pass: every view's block rows, the look-back words of the batch's cell groups, the view
-  // table (host copy in hostCellViews) and its totals
-  DeviceBuffer cellLists, cellStatus, cellViews;
+  // direct lists (every view at most kDirectMaxPatches patches), all views in one launch per
+  // pass: every view's block rows, the look-back words of the batch's patch groups, the view
+  // table (host copy in hostPatchViews) and its totals
+  DeviceBuffer patchLists, patchStatus, patchViews;
   bool directLists = false;
-  CellListBatch cellBatch{};
+  bool patchMasks = false;  // some view's patches hold more than one cell
+  PatchListBatch patchBatch{};
   // LOD views: every view's cut, each view's six report words (LodState's first six), and the
   // selection scratch the views share in turn (sized for the largest)
   DeviceBuffer lodIndices, lodReports, lodFrontier[2], lodCosts, lodOffsets, lodPackets, lodState,
@@ -72,7 +73,7 @@ struct BatchLane {
   std::vector<LodPlan> lodPlans;
   // pinned host
   PinnedBuffer hostViews, hostCameras, hostCounters, hostViewFirst, hostImage, hostLodReports,
-      hostCellViews;
+      hostPatchViews;
   // the submission it holds
   uint64_t ticket = 0;
   bool busy = false, harvested = true;

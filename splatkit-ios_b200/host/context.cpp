@@ -4,8 +4,9 @@
 //
 // A frame is enqueued on the context's stream without a host round trip:
 //   [LOD cut] -> visibility (cull, project, SH, depth key, tile span, source-order compaction)
-//   -> depth sort (onesweep radix, 16- or 32-bit keys) -> tile binning -> stable tile sort
-//   -> tile ranges -> composite, then a 64-byte counter block is copied back asynchronously.
+//   -> depth sort (onesweep radix, 16- or 32-bit keys) -> each patch's front-to-back list (very
+//   large targets: binning, stable tile sort and ranges) -> composite, then a 64-byte counter
+//   block is copied back asynchronously.
 // Every grid is sized by a host-known capacity; live counts stay on the device.
 #include "context.h"
 
@@ -161,7 +162,9 @@ sk_status Context::reserveScratch(FrameScratch& f, uint32_t sources, uint32_t in
   grab(f.instValuesSorted, size_t{instances} * 4);
   grab(f.tileSortWorkspace, sortWorkspaceBytesFor(instances, kTileSortTileKeys));
   grab(f.ranges, size_t{maxTiles} * sizeof(uint2));
-  grab(f.cellLists, cellListBytes(sources, std::min(std::max(maxTiles, f.maxTiles), kDirectMaxCells)));
+  // a target of t composite tiles has at most kPatchGoal patches, or t / 8 + 1 of the largest
+  grab(f.patchLists, patchListBytes(sources, std::min(std::max(std::max(maxTiles, f.maxTiles) / 8 + 1, kPatchGoal),
+                                                      kDirectMaxPatches)));
   grab(f.rangeBuffer, size_t{kMaxRanges} * sizeof(Range));
   grab(f.rangeStarts, size_t{kMaxRanges + 1} * 4);
   const bool fresh = f.counters.ptr == nullptr;
@@ -171,6 +174,7 @@ sk_status Context::reserveScratch(FrameScratch& f, uint32_t sources, uint32_t in
   if (e == cudaSuccess) e = cudaMemsetAsync(f.sortWorkspace.ptr, 0, f.sortWorkspace.bytes, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(f.tileSortWorkspace.ptr, 0, f.tileSortWorkspace.bytes, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(f.visStatus.ptr, 0, f.visStatus.bytes, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(f.patchLists.ptr, 0, patchListStatusBytes(), s);
   if (e != cudaSuccess) return check(e, "frame buffers");
   f.sources = sources;
   f.instanceCapacity = instances;
@@ -274,12 +278,12 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
   uint32_t* counters = static_cast<uint32_t*>(f.counters.ptr);
   FrameCounters* fc = view.counters;
   uint32_t* error = &fc->error;
-  // Direct cell lists write every range; the sorted path only those of non-empty cells.
-  const uint32_t cells = binsX * binsY;
-  const bool direct = binningMode == SK_BINNING_AUTO && cellListsFit(f.sources, cells) &&
-                      f.cellLists.bytes >= cellListBytes(f.sources, cells);
+  const bool direct = view.direct;
+  // patches of one cell are cell lists: their entries need no masks
+  uint16_t* masks = direct && view.patches().shift ? static_cast<uint16_t*>(f.instKeysSorted.ptr) : nullptr;
   cudaError_t e = cudaMemsetAsync(fc, 0, sizeof(FrameCounters), s);
-  if (e == cudaSuccess && !direct) e = clearTileRanges(static_cast<uint2*>(f.ranges.ptr), cells, s);
+  // Direct lists write every range; the sorted path only those of non-empty cells.
+  if (e == cudaSuccess && !direct) e = clearTileRanges(static_cast<uint2*>(f.ranges.ptr), binsX * binsY, s);
   if (timing != 0) cudaEventRecord(events[0], s);
 
   const bool lod = world.lod;
@@ -377,7 +381,7 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
   }
   if (timed) cudaEventRecord(events[3], s);
   if (e == cudaSuccess && direct) {
-    // each cell's list written in place, front to back, with its range
+    // each patch's list written in place, front to back, with its range
     BinArgs b{};
     b.spans = static_cast<const uint4*>(f.spans.ptr);
     b.order = static_cast<const uint32_t*>(f.order.ptr);
@@ -385,57 +389,26 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
     b.capacity = f.sources;
     b.width = view.width, b.height = view.height, b.tilesX = binsX, b.tilesY = binsY;
     b.instanceValues = static_cast<uint32_t*>(f.instValuesSorted.ptr);
+    b.instanceMasks = masks;
     b.instanceCapacity = f.instanceCapacity;
     b.instanceCount = &fc->instances;
     b.overflow = &fc->overflow;
-    CellLists cl{};
-    cl.cells = cells;
-    cl.workspace = f.cellLists.ptr;
-    cl.ranges = static_cast<uint2*>(f.ranges.ptr);
-    cl.counters = counters + 8;
-    cl.epoch = nextEpoch(1);
-    cl.error = error;
-    e = launchCellLists(b, cl, s);
+    PatchLists pl{};
+    pl.workspace = f.patchLists.ptr;
+    pl.ranges = static_cast<uint2*>(f.ranges.ptr);
+    pl.entryCount = &fc->entries;
+    pl.counters = counters + 8;
+    pl.epoch = nextEpoch(1);
+    pl.error = error;
+    e = launchPatchLists(b, pl, s);
   }
-  if (e == cudaSuccess && !direct) {
-    BinArgs b{};
-    b.spans = static_cast<const uint4*>(f.spans.ptr);
-    b.order = static_cast<const uint32_t*>(f.order.ptr);
-    b.count = &fc->visible;
-    b.capacity = f.sources;
-    b.width = view.width, b.height = view.height, b.tilesX = binsX, b.tilesY = binsY;
-    b.instanceKeys = static_cast<uint32_t*>(f.instKeys.ptr);
-    b.instanceValues = static_cast<uint32_t*>(f.instValues.ptr);
-    b.instanceCapacity = f.instanceCapacity;
-    b.instanceCount = &fc->instances;
-    b.overflow = &fc->overflow;
-    b.blockSums = static_cast<uint32_t*>(f.binSums.ptr);
-    b.balanced = 1;
-    e = launchBinning(b, s);
-  }
-  if (e == cudaSuccess && !direct) {
-    SortArgs a{};
-    a.keysIn = static_cast<const uint32_t*>(f.instKeys.ptr);
-    a.valuesIn = static_cast<const uint32_t*>(f.instValues.ptr);
-    a.keysOut = static_cast<uint32_t*>(f.instKeysSorted.ptr);
-    a.valuesOut = static_cast<uint32_t*>(f.instValuesSorted.ptr);
-    a.count = &fc->instances;
-    a.capacity = f.instanceCapacity;
-    a.bits = 16;
-    sortBindWorkspaceFor(a, f.tileSortWorkspace.ptr, f.instanceCapacity, kTileSortTileKeys);
-    a.tileKeys = kTileSortTileKeys;
-    a.epoch = nextEpoch(4);
-    a.error = error;
-    e = launchSort(a, s);
-  }
-  if (e == cudaSuccess && !direct)
-    e = launchTileRanges(static_cast<const uint32_t*>(f.instKeysSorted.ptr), &fc->instances,
-                         f.instanceCapacity, static_cast<uint2*>(f.ranges.ptr), binsX * binsY, s);
+  if (e == cudaSuccess && !direct) e = enqueueSortedLists(f, view, s);
   if (timed) cudaEventRecord(events[4], s);
   if (e == cudaSuccess) {
     CompositeArgs c{};
     c.projected = static_cast<const Projected*>(f.projected.ptr);
     c.values = static_cast<const uint32_t*>(f.instValuesSorted.ptr);
+    c.masks = masks;
     c.ranges = static_cast<const uint2*>(f.ranges.ptr);
     c.width = view.width, c.height = view.height, c.tilesX = tilesX, c.tilesY = tilesY;
     c.binsX = binsX;
@@ -455,11 +428,69 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
   return check(e, "frame");
 }
 
+cudaError_t Context::enqueueSortedLists(FrameScratch& f, const ViewTarget& view, cudaStream_t s) {
+  FrameCounters* fc = view.counters;
+  BinArgs b{};
+  b.spans = static_cast<const uint4*>(f.spans.ptr);
+  b.order = static_cast<const uint32_t*>(f.order.ptr);
+  b.count = &fc->visible;
+  b.capacity = f.sources;
+  b.width = view.width, b.height = view.height, b.tilesX = view.binsX(), b.tilesY = view.binsY();
+  b.instanceKeys = static_cast<uint32_t*>(f.instKeys.ptr);
+  b.instanceValues = static_cast<uint32_t*>(f.instValues.ptr);
+  b.instanceCapacity = f.instanceCapacity;
+  b.instanceCount = &fc->instances;
+  b.overflow = &fc->overflow;
+  b.blockSums = static_cast<uint32_t*>(f.binSums.ptr);
+  b.balanced = 1;
+  cudaError_t e = launchBinning(b, s);
+  if (e == cudaSuccess) {
+    SortArgs a{};
+    a.keysIn = static_cast<const uint32_t*>(f.instKeys.ptr);
+    a.valuesIn = static_cast<const uint32_t*>(f.instValues.ptr);
+    a.keysOut = static_cast<uint32_t*>(f.instKeysSorted.ptr);
+    a.valuesOut = static_cast<uint32_t*>(f.instValuesSorted.ptr);
+    a.count = &fc->instances;
+    a.capacity = f.instanceCapacity;
+    a.bits = 16;
+    sortBindWorkspaceFor(a, f.tileSortWorkspace.ptr, f.instanceCapacity, kTileSortTileKeys);
+    a.tileKeys = kTileSortTileKeys;
+    a.epoch = nextEpoch(4);
+    a.error = &fc->error;
+    e = launchSort(a, s);
+  }
+  if (e == cudaSuccess)
+    e = launchTileRanges(static_cast<const uint32_t*>(f.instKeysSorted.ptr), &fc->instances,
+                         f.instanceCapacity, static_cast<uint2*>(f.ranges.ptr),
+                         view.binsX() * view.binsY(), s);
+  return e;
+}
+
+sk_status Context::expandLists() {
+  const Slot& slot = slots[lastSlot];
+  if (!slot.direct || listsExpanded) return SK_OK;
+  FrameScratch& f = scratchOf(lastSlot);
+  const cudaStream_t s = streamOf(lastSlot);
+  if (lastCounters.instances > f.instanceCapacity) {  // a pair per cell where the frame needed one per patch
+    const sk_status st = reserveScratch(f, f.sources, lastCounters.instances, f.maxTiles, s);
+    if (st != SK_OK) return st;
+  }
+  ViewTarget view = plainView(slot);
+  view.width = slot.width;
+  view.height = slot.height;
+  cudaError_t e = clearTileRanges(static_cast<uint2*>(f.ranges.ptr), view.binsX() * view.binsY(), s);
+  if (e == cudaSuccess) e = enqueueSortedLists(f, view, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  listsExpanded = e == cudaSuccess;
+  return check(e, "tile lists");
+}
+
 ViewTarget Context::plainView(const Slot& slot) {
   const bool second = &slot == &slots[1];
   ViewTarget v;
   v.width = width;
   v.height = height;
+  v.direct = slot.direct;
   v.image = imageOf(slot.image);
   v.counters = static_cast<FrameCounters*>(second ? frameCounters2.ptr : frameCounters.ptr);
   v.hostCounters = static_cast<FrameCounters*>(slot.hostCounters.ptr);
@@ -502,7 +533,14 @@ sk_status Context::enqueueSlot(uint32_t index) {
   Slot& slot = slots[index];
   const cudaStream_t s = streamOf(index);
   *static_cast<Camera*>(slot.hostCamera.ptr) = cameraFor(slot.frame, width, height);
-  const ViewTarget view = plainView(slot);
+  FrameScratch& f = scratchOf(index);
+  ViewTarget view = plainView(slot);
+  const uint32_t patches = view.patches().x * view.patches().y;
+  view.direct = binningMode == SK_BINNING_AUTO && patchListsFit(patches) &&
+                f.patchLists.bytes >= patchListBytes(f.sources, patches);
+  slot.direct = view.direct;
+  slot.width = width;
+  slot.height = height;
   cudaError_t e = cudaMemcpyAsync(const_cast<Camera*>(view.camera), slot.hostCamera.ptr,
                                   sizeof(Camera), cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return check(e, "camera upload");
@@ -511,7 +549,7 @@ sk_status Context::enqueueSlot(uint32_t index) {
     e = cudaStreamWaitEvent(s, imageFree[slot.image], 0);
     if (e != cudaSuccess) return check(e, "capture wait");
   }
-  sk_status st = enqueuePipeline(scratchOf(index), view, slot.frame, slot.total, s, timeStages,
+  sk_status st = enqueuePipeline(f, view, slot.frame, slot.total, s, timeStages,
                                  slot.events);
   if (st != SK_OK) return st;
   st = check(cudaEventRecord(slot.done, s), "frame");
@@ -553,10 +591,10 @@ sk_status Context::finishOldest() {
     // image): wait for all of them, grow the buffers and draw them all again, in order.
     e = syncStreams();
     if (e != cudaSuccess) return check(e, "frame wait");
-    uint32_t most = c.instances;
+    uint32_t most = 0;  // per-cell pairs (the sorted lists), or entries per patch
     for (const uint32_t k : inFlight) {
       const auto* fc = static_cast<const FrameCounters*>(slots[k].hostCounters.ptr);
-      most = std::max(most, fc->instances);
+      most = std::max({most, fc->instances, fc->entries});
     }
     const uint32_t need = static_cast<uint32_t>(
         std::min<uint64_t>(uint64_t{most} + most / 4 + 1024, 0x7fffffffu));
@@ -570,6 +608,7 @@ sk_status Context::finishOldest() {
     return finishOldest();
   }
   lastSlot = inFlight.front();
+  listsExpanded = false;
   inFlight.pop_front();
   ++completed;
   lastCounters = c;
@@ -1135,12 +1174,19 @@ sk_status sk_read_tile_lists(sk_context* handle, uint32_t* ranges, uint32_t* val
   SK_CTX(handle);
   sk_status st = ctx->finishFrame(true);
   if (st != SK_OK) return st;
+  const bool direct = ctx->slots[ctx->lastSlot].direct;
+  if (direct && (st = ctx->expandLists()) != SK_OK) return st;
   const uint32_t n = std::min(ctx->lastCounters.instances, ctx->scratchOf(ctx->lastSlot).instanceCapacity);
   if (count) *count = n;
   cudaError_t e = cudaSuccess;
   const size_t bins = size_t{(ctx->width + sk::kBinSize - 1) / sk::kBinSize} *
                       ((ctx->height + sk::kBinSize - 1) / sk::kBinSize);
   if (ranges) e = cudaMemcpy(ranges, ctx->scratchOf(ctx->lastSlot).ranges.ptr, bins * 8, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess && ranges && direct)  // an empty cell's range sits after the cells before it
+    for (size_t c = 0, run = 0; c < bins; ++c) {
+      if (ranges[2 * c + 1] == 0) ranges[2 * c] = ranges[2 * c + 1] = static_cast<uint32_t>(run);
+      run = ranges[2 * c + 1];
+    }
   const uint32_t copy = std::min(n, capacity);
   if (e == cudaSuccess && values && copy)
     e = cudaMemcpy(values, ctx->scratchOf(ctx->lastSlot).instValuesSorted.ptr, size_t{copy} * 4, cudaMemcpyDeviceToHost);

@@ -91,7 +91,7 @@ struct FrameScratch {
   DeviceBuffer keys, projected, spans, order, sortWorkspace, visStatus, binSums;
   DeviceBuffer instKeys, instValues, instKeysSorted, instValuesSorted, tileSortWorkspace;
   DeviceBuffer ranges, rangeBuffer, rangeStarts, counters;
-  DeviceBuffer cellLists;  // direct cell-major lists: block x cell counts and starts
+  DeviceBuffer patchLists;  // direct lists: block x patch counts and starts
   DeviceBuffer lodIndices, lodFrontier[2], lodCosts, lodOffsets, lodPackets, lodState, lodStatus,
       lodCounters;
   uint32_t lodFrontierCapacity = 0;
@@ -107,10 +107,12 @@ struct ViewTarget {
   FrameCounters* counters = nullptr;       // device
   FrameCounters* hostCounters = nullptr;   // pinned; null: no readback
   const Camera* camera = nullptr;          // device, written before the pipeline runs
+  bool direct = false;                     // lists per patch, written in place
   uint32_t tilesX() const { return (width + kTileSize - 1) / kTileSize; }
   uint32_t tilesY() const { return (height + kTileSize - 1) / kTileSize; }
   uint32_t binsX() const { return (width + kBinSize - 1) / kBinSize; }
   uint32_t binsY() const { return (height + kBinSize - 1) / kBinSize; }
+  PatchGrid patches() const { return patchGrid(binsX(), binsY()); }
 };
 
 // The per-view camera block of a frame on a width x height target.
@@ -157,6 +159,8 @@ struct Context {
     sk_frame frame{};
     std::vector<sk_range> ranges;
     uint32_t total = 0, image = 0;
+    uint32_t width = 0, height = 0;  // target it was drawn on
+    bool direct = false;             // its lists are per patch (csrc/cell_lists.cu)
     uint64_t number = 0;  // the submitted-frame count it was drawn as
   };
   Slot slots[kFrameSlots];
@@ -209,6 +213,12 @@ struct Context {
   // The whole frame pipeline for one view on stream s; nothing waits on the host.
   sk_status enqueuePipeline(FrameScratch& f, const ViewTarget& v, const sk_frame& frame,
                             uint32_t total, cudaStream_t s, uint32_t timing, cudaEvent_t* events);
+  // The lists by a stable sort of (cell, splat) pairs: binning, sort, ranges.
+  cudaError_t enqueueSortedLists(FrameScratch& f, const ViewTarget& v, cudaStream_t s);
+  // The last finished frame's per-cell lists from its spans and order, where it drew from direct
+  // lists (the read-back is per cell); its patch lists are overwritten.
+  sk_status expandLists();
+  bool listsExpanded = false;  // of the last finished frame
   ViewTarget plainView(const Slot& slot);
   sk_status enqueueSlot(uint32_t slot);
   // Finishes the oldest frame in flight (waiting for it); grows the list buffers and draws

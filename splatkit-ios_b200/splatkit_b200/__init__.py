@@ -486,7 +486,7 @@ class Renderer:
         self._check(self._lib.sk_apply_render_policy(self._h, ctypes.byref(p)), "policy")
 
     def set_binning(self, mode: str):
-        """"auto": cell lists written in place on targets of up to 4096 cells, else sorted;
+        """"auto": lists written in place (very large targets: sorted);
         "sorted": always the stable (cell, splat) sort. Both give the same lists."""
         code = {"auto": 0, "sorted": 1}[mode]
         self._check(self._lib.sk_set_binning(self._h, code), "binning")

@@ -1,0 +1,48 @@
+"""Frames drawn from the direct lists (cell_lists.cu: one entry per splat and patch of 1, 2 or 4 cells
+a side, filtered by the composite) against the same frames drawn from the stable (cell, splat) sort:
+the image bit for bit, the (splat, cell) pairs and the list records the composite read. Targets at
+the edges of the patch sizes (320 patches, odd cells and tiles), beyond the direct lists' 4096
+patches, and splats of many patches (several staging windows, whole-warp walks)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import splatkit_b200 as sk
+from splatkit_b200 import synthetic
+
+from test_gpu_cell_lists import frames_for
+
+
+def draw(cloud, frames, w, h, mode):
+    r = sk.Renderer(w, h, image_format=sk.FORMAT_RGBA32F)
+    r.set_binning(mode)
+    r.upload_world(cloud, cloud.sh_degree)
+    out = []
+    for frame in frames:
+        r.draw(frame)
+        image = r.read_image(sk.FORMAT_RGBA32F)
+        s = r.stats()
+        out.append((image, s["draw_count"], s["instances"], s["instances_read"]))
+    r.close()
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,w,h,log_scale", [
+    (60_000, 640, 512, -3.0),     # 20 x 16 = 320 cells: the most for single-cell patches
+    (60_000, 641, 512, -2.5),     # one column more: patches of 2 x 2 cells
+    (80_000, 1279, 1021, -2.0),   # odd cells and tiles, 2 x 2
+    (40_000, 1281, 1025, -1.0),   # just above: 4 x 4 patches that hang over the target
+    (150_000, 3840, 2160, -2.5),  # 4 x 4, 510 patches
+    (300, 8224, 8096, 0.0),       # 65 x 64 patches: both modes sort
+    (2_500, 1280, 720, 0.5),      # boxes of hundreds of cells, several windows per warp
+    (1, 33, 17, -1.0),
+])
+def test_direct_frames_equal_the_sorted_frames(cuda_device, n, w, h, log_scale):
+    cloud = synthetic.random_cloud(n, seed=17, sh_degree=0, log_scale_mean=log_scale)
+    frames = frames_for(cloud, w, h, (11, 52))
+    for (ia, va, pa, ra), (ib, vb, pb, rb) in zip(draw(cloud, frames, w, h, "auto"),
+                                                  draw(cloud, frames, w, h, "sorted")):
+        assert (va, pa, ra) == (vb, pb, rb)
+        assert np.array_equal(ia, ib)
