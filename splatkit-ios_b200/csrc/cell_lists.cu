@@ -98,12 +98,9 @@ __device__ __forceinline__ Job jobOf(const BinArgs& a, const Work& w, uint32_t p
     j.ranges = ranges;
     return j;
   }
-  uint32_t lo = 0, hi = w.viewCount;  // the last view whose first block (group) is <= index
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) / 2;
-    const uint32_t start = byGroup ? w.views[mid].groupBase : w.views[mid].blockBase;
-    if (start <= index) lo = mid; else hi = mid;
-  }
+  const uint32_t lo = lastAtOrBelow(w.viewCount, index, [&](uint32_t v) {
+    return byGroup ? __ldg(&w.views[v].groupBase) : __ldg(&w.views[v].blockBase);
+  });
   const PatchListView v = w.views[lo];
   j.block = index - (byGroup ? v.groupBase : v.blockBase);
   j.first = w.viewFirst[lo];

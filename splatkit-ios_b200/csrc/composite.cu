@@ -260,11 +260,7 @@ __global__ void __launch_bounds__(kThreads) compositeKernel(const __grid_constan
     t.patchesX = g.x, t.patchShift = g.shift;
   }
   if constexpr (kBatch) {
-    uint32_t lo = 0, hi = a.viewCount;
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) / 2;
-      if (__ldg(&a.views[mid].tileBase) <= blockIdx.x) lo = mid; else hi = mid;
-    }
+    const uint32_t lo = lastAtOrBelow(a.viewCount, blockIdx.x, [&](uint32_t v) { return __ldg(&a.views[v].tileBase); });
     const BatchView* v = a.views + lo;
     t.width = __ldg(&v->width);
     t.height = __ldg(&v->height);

@@ -47,8 +47,12 @@ __device__ __forceinline__ float halfToFloat(uint32_t h) {
 
 __device__ __forceinline__ float lowHalf(uint32_t w) { return halfToFloat(w & 0xffffu); }
 __device__ __forceinline__ float highHalf(uint32_t w) { return halfToFloat(w >> 16); }
+// Both halves by one saturating conversion; the rare NaN (whose payload it would not keep) one by one.
 __device__ __forceinline__ uint32_t packHalf2(float lo, float hi) {
-  return floatToHalf(lo) | (floatToHalf(hi) << 16);
+  if (lo != lo || hi != hi) return floatToHalf(lo) | (floatToHalf(hi) << 16);
+  uint32_t packed;
+  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(packed) : "f"(hi), "f"(lo));
+  return packed;
 }
 __device__ __forceinline__ float halfRound(float v) { return halfToFloat(floatToHalf(v)); }
 
@@ -101,6 +105,22 @@ __device__ __forceinline__ float lnF32(float x) {
 __device__ __forceinline__ void chainedKernelStart() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The last of `count` ascending starts (startOf(0) <= index) at or below `index`, searched by a warp:
+// every lane looks at a start of its own, so up to 32 take one step. All lanes call this and get it.
+template <typename StartOf>
+__device__ __forceinline__ uint32_t lastAtOrBelow(uint32_t count, uint32_t index, StartOf startOf) {
+  uint32_t lo = 0;
+  while (count > 1) {
+    const uint32_t step = (count + 31) / 32;
+    const uint32_t at = laneId() * step;
+    const bool below = at < count && startOf(lo + at) <= index;
+    const uint32_t top = 31 - __clz(__ballot_sync(0xffffffffu, below) | 1u);
+    lo += top * step;
+    count = min(step, count - top * step);
+  }
+  return lo;
 }
 
 // Copies the 208-byte camera from device memory into shared memory (the caller syncs).

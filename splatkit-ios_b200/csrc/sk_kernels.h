@@ -32,7 +32,7 @@ struct VisibilityArgs {
   uint4* spans;  // per survivor: the binning cells its quad touches (sk_tiles.cuh)
   uint32_t tilesX, tilesY;  // binning cells (kBinSize pixels) per row and column
   uint32_t* visibleCount;
-  uint64_t* status;    // one word per 1024-splat tile
+  uint64_t* status;    // one word per tile: visibilityTiles(total)
   uint32_t* counters;  // two words
   uint32_t epoch;
   uint32_t* error;
@@ -43,7 +43,8 @@ struct VisibilityArgs {
   uint32_t* sortBases;
   uint32_t sortPasses;
 };
-uint32_t visibilityTileSplats();
+uint32_t visibilityTileSplats();               // records of a batch's work item
+uint32_t visibilityTiles(uint32_t total);      // most tiles a frame of up to `total` records has
 // `cam` is a device pointer: the kernels stage it in shared memory, so a captured graph can be
 // replayed with new cameras written into the same buffer.
 cudaError_t launchVisibility(const Camera* cam, const VisibilityArgs& args, int shDegree,

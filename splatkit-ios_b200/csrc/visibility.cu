@@ -30,20 +30,34 @@ constexpr uint32_t kDepthKeyShift = 11;
 constexpr uint32_t kDepthKeyMax = 65535;
 
 constexpr uint32_t kThreads = 256;
+constexpr uint32_t kWarps = kThreads / 32;
+// Splats per thread: tiles of 1024 splats, or of 256 where that many blocks fit the chip at once
+// (launchVisibility).
 constexpr uint32_t kItems = 4;
 constexpr uint32_t kTileSplats = kThreads * kItems;
 
-// Per block: i / 255 for the 8-bit colour and opacity channels (the same IEEE quotients the
-// division gives, computed once per block instead of four times per splat) and the camera's
-// near distance proj[14] / proj[10].
+// Per block, by 8-bit opacity: i / 255 (also the 8-bit colour channels: the same IEEE quotients the
+// division gives, computed once per block instead of four times per splat) and the quad radius that
+// opacity allows; and the camera's near distance proj[14] / proj[10].
 __shared__ float blockUnorm8[256];
+__shared__ float blockReach[256];
 __shared__ float blockZNear;
 
-// Fills the block constants; the camera must be in shared memory. Ends with a barrier.
-__device__ __forceinline__ void loadBlockConstants(const Camera& cam) {
-  blockUnorm8[threadIdx.x] = static_cast<float>(threadIdx.x) / 255.0f;
-  if (threadIdx.x == 0) blockZNear = cam.proj[14] / cam.proj[10];
-  __syncthreads();
+__device__ __forceinline__ float quadReach(float alpha, float bound) {
+  return fminf(bound, sqrtf(2.0f * lnF32(fmaxf(alpha / kQuadMinAlpha, 1.0f))));
+}
+
+// The block's tables (the caller syncs). They depend on nothing that a kernel before wrote.
+__device__ __forceinline__ void fillBlockTables() {
+  const float unorm = static_cast<float>(threadIdx.x) / 255.0f;
+  blockUnorm8[threadIdx.x] = unorm;
+  blockReach[threadIdx.x] = quadReach(unorm, kBoundsRadius);
+}
+
+// Copies the view's camera and its near distance into shared memory (the caller syncs).
+__device__ __forceinline__ void loadView(const Camera* __restrict__ camera, Camera* cam) {
+  loadCamera(camera, cam);
+  if (threadIdx.x == kThreads - 1) blockZNear = __ldg(&camera->proj[14]) / __ldg(&camera->proj[10]);
 }
 
 __device__ __forceinline__ void mulPoint(const float* m, float x, float y, float z, float w,
@@ -193,8 +207,7 @@ __device__ __forceinline__ bool projectSplat(const Camera& cam, const uint4 lo, 
   const float a1x = e1x * s1, a1y = e1y * s1;
   const float a2x = e1y * s2, a2y = (-e1x) * s2;
 
-  float radius = fminf(lodAlpha != 0u ? kLodBoundsRadius : kBoundsRadius,
-                       sqrtf(2.0f * lnF32(fmaxf(alpha / kQuadMinAlpha, 1.0f))));
+  float radius = lodAlpha != 0u ? quadReach(alpha, kLodBoundsRadius) : blockReach[rgba8 >> 24];
   const float sigmaPixels = sqrtf(fmaxf(a1x * a1x + a1y * a1y, a2x * a2x + a2y * a2y));
   radius = fminf(radius, kMaxPixelRadius / fmaxf(sigmaPixels, 1e-6f));
 
@@ -296,23 +309,25 @@ __device__ __forceinline__ uint32_t sourceIndex(const VisibilityArgs& a, uint32_
 }
 
 // Shared memory of one tile: survivors staged at their source slot, then compacted.
+template <uint32_t kRows>
 struct VisibilitySmem {
-  uint4 rec[kTileSplats * 2];     // projected records by source slot
-  uint32_t key[kTileSplats];      // depth keys by source slot
-  uint16_t slotOf[kTileSplats];   // survivor k of the tile -> its source slot
-  uint32_t rowMask[kThreads / 32][kItems];
-  uint32_t warpBase[kThreads / 32];
-  uint32_t tileBase, tileCount;
+  static constexpr uint32_t kSlots = kThreads * kRows;
+  uint4 rec[kSlots * 2];     // projected records by source slot
+  uint32_t key[kSlots];      // depth keys by source slot
+  uint16_t slotOf[kSlots];   // survivor k of the tile -> its source slot
+  uint32_t rowMask[kWarps][kRows];
+  uint32_t warpTotal[kWarps];
+  uint32_t tileBase;
 };
 
-// Projects one 1024-record tile into shared memory: survivors' keys and records at their
+// Projects one tile (kRows records per thread) into shared memory: survivors' keys and records at their
 // source slot, and per warp row the mask of survivors. Part styles (when labels are given) and
 // the reveal glow are applied to each survivor's record after its projection. indexOf(t) gives the record index of
 // tile position t, or 0xffffffff past the end. keyHigh is or-ed into every key (the view id of a
 // batch, above a 16-bit key). One record per row of the warp, not unrolled (the projection is
 // large); the next row's record is fetched while this one is projected.
-template <int D, bool kKey16, typename IndexOf>
-__device__ __forceinline__ void projectTile(VisibilitySmem& s, const Camera& cam,
+template <int D, bool kKey16, uint32_t kRows, typename IndexOf>
+__device__ __forceinline__ void projectTile(VisibilitySmem<kRows>& s, const Camera& cam,
                                             const GpuSplat* __restrict__ splats,
                                             const uint32_t* __restrict__ sh, uint32_t shStride,
                                             const PartLabels& parts, uint32_t first,
@@ -325,10 +340,10 @@ __device__ __forceinline__ void projectTile(VisibilitySmem& s, const Camera& cam
     lo = __ldg(p), hi = __ldg(p + 1);
   }
 #pragma unroll 1
-  for (uint32_t r = 0; r < kItems; ++r) {
+  for (uint32_t r = 0; r < kRows; ++r) {
     uint32_t nextIndex = 0xffffffffu;
     uint4 nextLo = make_uint4(0, 0, 0, 0), nextHi = nextLo;
-    if (r + 1 < kItems) {
+    if (r + 1 < kRows) {
       nextIndex = indexOf(first + (r + 1) * 32);
       if (nextIndex != 0xffffffffu) {
         const uint4* p = reinterpret_cast<const uint4*>(splats + nextIndex);
@@ -336,7 +351,7 @@ __device__ __forceinline__ void projectTile(VisibilitySmem& s, const Camera& cam
       }
     }
     bool visible = false;
-    const uint32_t slot = warp * (32 * kItems) + r * 32 + lane;
+    const uint32_t slot = warp * (32 * kRows) + r * 32 + lane;
     if (index != 0xffffffffu) {
       uint32_t key, rec[8];
       visible = projectSplat<D, kKey16>(cam, lo, hi, index, sh, shStride, key, rec);
@@ -355,90 +370,94 @@ __device__ __forceinline__ void projectTile(VisibilitySmem& s, const Camera& cam
   __syncwarp();
 }
 
-// Order-preserving compaction of the tile's survivors: warp totals, the tile's offset by
-// decoupled look-back over status[0 .. tile], then survivor k of the tile -> its source slot.
-// Leaves the offset and count in s.tileBase / s.tileCount.
-__device__ __forceinline__ void compactTile(VisibilitySmem& s, uint64_t* status, uint32_t tile,
-                                            uint32_t epoch, uint32_t* error) {
+// Order-preserving compaction of the tile's survivors and their copy-out: the tile's count is published,
+// survivor k -> its source slot, then one warp takes the tile's offset by decoupled look-back over
+// status[0 .. tile] while the others work out the cells each survivor's quad touches (on a width x height
+// target), and consecutive threads write consecutive survivors. With digitPasses > 0 each key's 8-bit
+// digits are counted into digits[pass][digit]. Returns the survivors before and in the tile.
+template <uint32_t kRows>
+__device__ __forceinline__ uint2 compactTile(VisibilitySmem<kRows>& s, uint64_t* status, uint32_t tile,
+                                             uint32_t epoch, uint32_t* error, uint32_t* keys,
+                                             Projected* projected, uint4* spans, float width, float height,
+                                             uint32_t tilesX, uint32_t tilesY,
+                                             uint32_t (*digits)[256] = nullptr, uint32_t digitPasses = 0) {
   const uint32_t warp = threadIdx.x >> 5, lane = laneId();
-  uint32_t warpTotal = 0;
+  uint32_t mine = 0;
 #pragma unroll
-  for (uint32_t r = 0; r < kItems; ++r) warpTotal += __popc(s.rowMask[warp][r]);
-  if (lane == 0) s.warpBase[warp] = warpTotal;
+  for (uint32_t r = 0; r < kRows; ++r) mine += __popc(s.rowMask[warp][r]);
+  if (lane == 0) s.warpTotal[warp] = mine;
   __syncthreads();
-  if (warp == 0) {
-    const uint32_t mine = lane < kThreads / 32 ? s.warpBase[lane] : 0u;
-    uint32_t inclusive = mine;
+  uint32_t count = 0, pos = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t up = __shfl_up_sync(0xffffffffu, inclusive, o);
-      if (lane >= static_cast<uint32_t>(o)) inclusive += up;
-    }
-    const uint32_t aggregate = __shfl_sync(0xffffffffu, inclusive, 31);
-    if (lane < kThreads / 32) s.warpBase[lane] = inclusive - mine;
-    uint32_t exclusive = 0;
-    if (tile == 0) {
-      if (lane == 0) storeStatus(status, makeStatus(epoch, kFlagPrefix, aggregate));
-    } else {
-      if (lane == 0) storeStatus(status + tile, makeStatus(epoch, kFlagAggregate, aggregate));
-      exclusive = warpLookback(status, tile, epoch, error);
-      if (lane == 0) storeStatus(status + tile, makeStatus(epoch, kFlagPrefix, exclusive + aggregate));
-    }
-    if (lane == 0) {
-      s.tileBase = exclusive;
-      s.tileCount = aggregate;
-    }
+  for (uint32_t w = 0; w < kWarps; ++w) {
+    if (w == warp) pos = count;
+    count += s.warpTotal[w];
   }
-  __syncthreads();
-  uint32_t pos = s.warpBase[warp];
+  if (threadIdx.x == 0) storeStatus(status + tile, makeStatus(epoch, tile == 0 ? kFlagPrefix : kFlagAggregate, count));
   const uint32_t below = lanemaskLt();
 #pragma unroll
-  for (uint32_t r = 0; r < kItems; ++r) {
+  for (uint32_t r = 0; r < kRows; ++r) {
     const uint32_t mask = s.rowMask[warp][r];
-    if (mask & (1u << lane)) s.slotOf[pos + __popc(mask & below)] = warp * (32 * kItems) + r * 32 + lane;
+    if (mask & (1u << lane)) s.slotOf[pos + __popc(mask & below)] = warp * (32 * kRows) + r * 32 + lane;
     pos += __popc(mask);
   }
   __syncthreads();
-}
-
-// Coalesced copy-out: consecutive threads write consecutive survivors, with the tiles each
-// survivor's quad touches on a width x height target.
-// With digitPasses > 0 each key's 8-bit digits are counted into digits[pass][digit].
-__device__ __forceinline__ void copyOutTile(const VisibilitySmem& s, uint32_t* keys,
-                                            Projected* projected, uint4* spans, float width,
-                                            float height, uint32_t tilesX, uint32_t tilesY,
-                                            uint32_t (*digits)[256] = nullptr,
-                                            uint32_t digitPasses = 0) {
-  const uint32_t count = s.tileCount, base = s.tileBase;
-  for (uint32_t k = threadIdx.x; k < count; k += kThreads) {
-    const uint32_t slot = s.slotOf[k];
-    const uint32_t key = s.key[slot];
-    keys[base + k] = key;
-    for (uint32_t p = 0; p < digitPasses; ++p) atomicAdd(&digits[p][(key >> (8 * p)) & 0xffu], 1u);
-    const uint4 lo = s.rec[2 * slot], hi = s.rec[2 * slot + 1];
-    uint4* o = reinterpret_cast<uint4*>(projected + base + k);
-    o[0] = lo;
-    o[1] = hi;
-    spans[base + k] = tileSpan(lo, hi, width, height, tilesX, tilesY);
+  if (warp == 0) {
+    uint32_t before = 0;
+    if (tile != 0) {
+      before = warpLookback(status, tile, epoch, error);
+      if (lane == 0) storeStatus(status + tile, makeStatus(epoch, kFlagPrefix, before + count));
+    }
+    if (lane == 0) s.tileBase = before;
   }
+  uint4 span[kRows];
+#pragma unroll
+  for (uint32_t r = 0; r < kRows; ++r) {
+    const uint32_t k = threadIdx.x + r * kThreads;
+    if (k < count) {
+      const uint32_t slot = s.slotOf[k];
+      span[r] = tileSpan(s.rec[2 * slot], s.rec[2 * slot + 1], width, height, tilesX, tilesY);
+      const uint32_t key = s.key[slot];
+      for (uint32_t p = 0; p < digitPasses; ++p) atomicAdd(&digits[p][(key >> (8 * p)) & 0xffu], 1u);
+    }
+  }
+  __syncthreads();
+  const uint32_t base = s.tileBase;
+#pragma unroll
+  for (uint32_t r = 0; r < kRows; ++r) {
+    const uint32_t k = threadIdx.x + r * kThreads;
+    if (k < count) {
+      const uint32_t slot = s.slotOf[k];
+      keys[base + k] = s.key[slot];
+      uint4* o = reinterpret_cast<uint4*>(projected + base + k);
+      o[0] = s.rec[2 * slot];
+      o[1] = s.rec[2 * slot + 1];
+      spans[base + k] = span[r];
+    }
+  }
+  return make_uint2(base, count);
 }
 
-template <int D, bool kKey16, bool kIndexed>
+template <int D, bool kKey16, bool kIndexed, uint32_t kRows>
 __global__ void __launch_bounds__(kThreads, 4)
     visibilityKernel(const Camera* __restrict__ camera, const __grid_constant__ VisibilityArgs a) {
-  chainedKernelStart();
-  __shared__ VisibilitySmem s;
+  constexpr uint32_t kTile = kThreads * kRows;
+  __shared__ VisibilitySmem<kRows> s;
   __shared__ Camera cam;
   __shared__ uint32_t digits[4][256];
-  loadCamera(camera, &cam);
+  // Before the wait for the kernel before this one: what depends on nothing it writes (the tile counter
+  // is this launch's alone; its last block left it at zero in an earlier, finished launch).
+  fillBlockTables();
   for (uint32_t p = 0; p < a.sortPasses; ++p) digits[p][threadIdx.x] = 0;
-  const uint32_t tile = takeTile(a.counters);  // its barrier also publishes the camera
-  loadBlockConstants(cam);
+  const uint32_t tile = takeTile(a.counters);
+  chainedKernelStart();
+  loadView(camera, &cam);
+  __syncthreads();
   const uint32_t total = kIndexed ? min(*a.indexCount, a.total) : a.total;
-  const uint32_t tiles = (total + kTileSplats - 1) / kTileSplats;
+  const uint32_t tiles = (total + kTile - 1) / kTile;
   if (tile < tiles) {
     const uint32_t warp = threadIdx.x >> 5, lane = laneId();
-    const uint32_t first = tile * kTileSplats + warp * (32 * kItems) + lane;
+    const uint32_t first = tile * kTile + warp * (32 * kRows) + lane;
     auto indexOf = [&](uint32_t t) -> uint32_t {
       if (t >= total) return 0xffffffffu;
       const uint32_t index = kIndexed ? a.indices[t] : sourceIndex(a, t);
@@ -449,10 +468,9 @@ __global__ void __launch_bounds__(kThreads, 4)
       return index;
     };
     projectTile<D, kKey16>(s, cam, a.splats, a.sh, a.shStride, a.parts, first, 0u, indexOf);
-    compactTile(s, a.status, tile, a.epoch, a.error);
-    if (tile == tiles - 1 && threadIdx.x == 0) *a.visibleCount = s.tileBase + s.tileCount;
-    copyOutTile(s, a.keys, a.projected, a.spans, cam.screenSize[0], cam.screenSize[1], a.tilesX,
-                a.tilesY, digits, a.sortPasses);
+    const uint2 at = compactTile(s, a.status, tile, a.epoch, a.error, a.keys, a.projected, a.spans,
+                                 cam.screenSize[0], cam.screenSize[1], a.tilesX, a.tilesY, digits, a.sortPasses);
+    if (tile == tiles - 1 && threadIdx.x == 0) *a.visibleCount = at.x + at.y;
   }
   if (tiles == 0 && tile == 0 && threadIdx.x == 0) *a.visibleCount = 0;
   if (a.sortPasses) {
@@ -476,30 +494,20 @@ __global__ void __launch_bounds__(kThreads, 4)
 template <int D>
 __global__ void __launch_bounds__(kThreads, 4)
     visibilityBatchKernel(const __grid_constant__ BatchVisibilityArgs a) {
-  chainedKernelStart();
-  __shared__ VisibilitySmem s;
+  __shared__ VisibilitySmem<kItems> s;
   __shared__ Camera cam;
-  __shared__ uint32_t viewOf;
   __shared__ BatchView view;
+  fillBlockTables();
   const uint32_t item = takeTile(a.counters);
+  chainedKernelStart();
   if (item < a.items) {
-    if (threadIdx.x == 0) {
-      // the last view whose first item is <= item
-      uint32_t lo = 0, hi = a.viewCount;
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (__ldg(&a.views[mid].itemStart) <= item) lo = mid; else hi = mid;
-      }
-      viewOf = lo;
-    }
-    __syncthreads();
-    const uint32_t v = viewOf;
-    loadCamera(a.cameras + v, &cam);
+    // the last view whose first item is <= item
+    const uint32_t v = lastAtOrBelow(a.viewCount, item, [&](uint32_t i) { return __ldg(&a.views[i].itemStart); });
+    loadView(a.cameras + v, &cam);
     if (threadIdx.x < sizeof(BatchView) / 4)
       reinterpret_cast<uint32_t*>(&view)[threadIdx.x] =
           __ldg(reinterpret_cast<const uint32_t*>(a.views + v) + threadIdx.x);
     __syncthreads();
-    loadBlockConstants(cam);
     const uint32_t chunk = item - view.itemStart;
     const uint32_t warp = threadIdx.x >> 5, lane = laneId();
     const uint32_t first = chunk * kTileSplats + warp * (32 * kItems) + lane;
@@ -517,41 +525,61 @@ __global__ void __launch_bounds__(kThreads, 4)
     };
     projectTile<D, true>(s, cam, view.splats, view.sh, view.shStride, PartLabels{}, first, v << 16,
                          indexOf);
-    compactTile(s, a.status, item, a.epoch, a.error);
+    const uint2 at = compactTile(s, a.status, item, a.epoch, a.error, a.keys, a.projected, a.spans,
+                                 static_cast<float>(view.width), static_cast<float>(view.height), view.binsX,
+                                 view.binsY);
     if (threadIdx.x == 0) {
-      if (chunk == 0) a.viewFirst[v] = s.tileBase;
+      if (chunk == 0) a.viewFirst[v] = at.x;
       if (item == a.items - 1) {
-        a.viewFirst[a.viewCount] = s.tileBase + s.tileCount;
-        *a.visibleCount = s.tileBase + s.tileCount;
+        a.viewFirst[a.viewCount] = at.x + at.y;
+        *a.visibleCount = at.x + at.y;
       }
     }
-    copyOutTile(s, a.keys, a.projected, a.spans, static_cast<float>(view.width),
-                static_cast<float>(view.height), view.binsX, view.binsY);
   }
   finishTile(a.counters);
 }
 
 
+// 1M splats at 1080p take 80 us whatever the arithmetic costs (78 without the harmonics' evaluation, 82
+// with approximate divisions): a third of the warps' time is the compaction's barriers, where a tile waits
+// for the counts of the tiles before it, all projected at the same time. A batch of many waves is bound by
+// instructions (569 us for 12M splats, 476 without the harmonics): the opacity's quad radius from a table,
+// saturating half conversions and the cells worked out during the look-back took it from 604 us.
+//
+// 256-splat tiles while the chip holds all their blocks at once (four per SM): the pass then lasts as
+// long as one tile, and a quarter of the rows end it sooner (4k splats 15.5 -> 9.0 us, 30k 21.4 -> 12.9, 100k
+// 21.2 -> 18.3); 1024-splat tiles beyond, where the tables, the look-back and the copy-out per block count
+// for more (1M splats 80 us, 86 with 512-splat tiles).
+constexpr uint32_t kSmallTotal = 4 * 148 * kThreads;
+
 template <int D, bool kKey16, bool kIndexed>
-void launchOne(const Camera* cam, const VisibilityArgs& a, uint32_t grid, cudaStream_t stream) {
-  launchChained(visibilityKernel<D, kKey16, kIndexed>, grid, kThreads, stream, cam, a);
+void launchOne(const Camera* cam, const VisibilityArgs& a, cudaStream_t stream) {
+  auto blocks = [&](uint32_t tile) { return max(1u, (a.total + tile - 1) / tile); };
+  if (a.total <= kSmallTotal) {
+    launchChained(visibilityKernel<D, kKey16, kIndexed, 1>, blocks(kThreads), kThreads, stream, cam, a);
+  } else {
+    launchChained(visibilityKernel<D, kKey16, kIndexed, kItems>, blocks(kTileSplats), kThreads, stream, cam, a);
+  }
 }
 
 template <int D>
-void launchDegree(const Camera* cam, const VisibilityArgs& a, bool key16, bool indexed,
-                  uint32_t grid, cudaStream_t stream) {
+void launchDegree(const Camera* cam, const VisibilityArgs& a, bool key16, bool indexed, cudaStream_t stream) {
   if (key16) {
-    if (indexed) launchOne<D, true, true>(cam, a, grid, stream);
-    else launchOne<D, true, false>(cam, a, grid, stream);
+    if (indexed) launchOne<D, true, true>(cam, a, stream);
+    else launchOne<D, true, false>(cam, a, stream);
   } else {
-    if (indexed) launchOne<D, false, true>(cam, a, grid, stream);
-    else launchOne<D, false, false>(cam, a, grid, stream);
+    if (indexed) launchOne<D, false, true>(cam, a, stream);
+    else launchOne<D, false, false>(cam, a, stream);
   }
 }
 
 }  // namespace
 
 uint32_t visibilityTileSplats() { return kTileSplats; }
+
+uint32_t visibilityTiles(uint32_t total) {
+  return (total + kTileSplats - 1) / kTileSplats + kSmallTotal / kThreads;
+}
 
 cudaError_t launchVisibilityBatch(const BatchVisibilityArgs& args, int shDegree,
                                   cudaStream_t stream) {
@@ -567,12 +595,11 @@ cudaError_t launchVisibilityBatch(const BatchVisibilityArgs& args, int shDegree,
 
 cudaError_t launchVisibility(const Camera* cam, const VisibilityArgs& args, int shDegree,
                              bool key16, bool indexed, cudaStream_t stream) {
-  const uint32_t grid = max(1u, (args.total + kTileSplats - 1) / kTileSplats);
   switch (shDegree) {
-    case 0: launchDegree<0>(cam, args, key16, indexed, grid, stream); break;
-    case 1: launchDegree<1>(cam, args, key16, indexed, grid, stream); break;
-    case 2: launchDegree<2>(cam, args, key16, indexed, grid, stream); break;
-    default: launchDegree<3>(cam, args, key16, indexed, grid, stream); break;
+    case 0: launchDegree<0>(cam, args, key16, indexed, stream); break;
+    case 1: launchDegree<1>(cam, args, key16, indexed, stream); break;
+    case 2: launchDegree<2>(cam, args, key16, indexed, stream); break;
+    default: launchDegree<3>(cam, args, key16, indexed, stream); break;
   }
   return cudaGetLastError();
 }
