@@ -534,13 +534,11 @@ size_t patchListBytes(uint32_t capacity, uint32_t patches) {
 size_t patchListStatusBytes() { return kStatusBytes; }
 
 cudaError_t patchListsConfigure() {
-  static bool configured = false;
-  if (configured) return cudaSuccess;
-  const int most = static_cast<int>(emitDynamicBytes(kDirectMaxPatches));
-  const cudaError_t e =
-      cudaFuncSetAttribute(patchEmitKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e == cudaSuccess) configured = true;
-  return e;
+  static std::atomic<uint64_t> done{0};
+  return oncePerDevice(done, [] {
+    return cudaFuncSetAttribute(patchEmitKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(emitDynamicBytes(kDirectMaxPatches)));
+  });
 }
 
 static cudaError_t launchPasses(const BinArgs& a, const Work& work, uint32_t patches, uint32_t blocks,

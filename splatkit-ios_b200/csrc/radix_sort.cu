@@ -273,9 +273,11 @@ template <bool kImplicitValues, bool kWriteKeys, uint32_t kGroups, uint32_t kPer
 cudaError_t launchScatter(const ScatterArgs& a, uint32_t tiles, cudaStream_t stream) {
   constexpr size_t kBytes = size_t{2} * kThreads * kGroups * kPer * 4;  // staged keys and values
   constexpr auto kernel = scatterKernel<kImplicitValues, kWriteKeys, kGroups, kPer>;
-  if (kBytes + sizeof(ScatterSmem<kGroups>) > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kBytes));
+  if constexpr (kBytes + sizeof(ScatterSmem<kGroups>) > 48 * 1024) {
+    static std::atomic<uint64_t> done{0};
+    const cudaError_t e = oncePerDevice(done, [&] {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kBytes));
+    });
     if (e != cudaSuccess) return e;
   }
   return launchChainedShared(kernel, tiles, kThreads * kGroups, kBytes, stream, a);
@@ -331,6 +333,7 @@ cudaError_t sortResetWorkspace(const SortArgs& a, cudaStream_t stream) {
 
 cudaError_t launchSort(const SortArgs& a, cudaStream_t stream) {
   const uint32_t passes = static_cast<uint32_t>(min(max(a.bits, 8), 32) + 7) / 8u;
+  if (sortInOneLaunch(a.capacity) && a.withheldTilePlusOne == 0) return launchClusterSort(a, passes, stream);
   const uint32_t tileKeys = tileKeysOf(a);
   if (tileKeys != 2048 && tileKeys != 4096 && tileKeys != 6144) return cudaErrorInvalidValue;
   const uint32_t tiles = sortTiles(a.capacity, tileKeys);

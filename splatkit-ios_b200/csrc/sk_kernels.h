@@ -111,6 +111,10 @@ void sortBindWorkspace(SortArgs& args, void* workspace, uint32_t capacity);
 size_t sortWorkspaceBytesFor(uint32_t capacity, uint32_t minTileKeys);
 void sortBindWorkspaceFor(SortArgs& args, void* workspace, uint32_t capacity, uint32_t minTileKeys);
 cudaError_t launchSort(const SortArgs& args, cudaStream_t stream);
+// Whether launchSort sorts up to `capacity` keys in one launch (cluster_sort.cu, unless the test hook asks
+// for the look-back): it then uses neither the histogram, the counters nor the status words.
+bool sortInOneLaunch(uint32_t capacity);
+cudaError_t launchClusterSort(const SortArgs& args, uint32_t passes, cudaStream_t stream);
 // Clears the counters and histogram accumulators of a bound workspace.
 cudaError_t sortResetWorkspace(const SortArgs& args, cudaStream_t stream);
 

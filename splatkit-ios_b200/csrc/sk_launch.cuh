@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <cstdint>
 #include <utility>
 
 namespace sk {
@@ -22,6 +24,19 @@ cudaError_t launchChainedShared(void (*kernel)(Params...), dim3 grid, dim3 block
   config.attrs = attribute;
   config.numAttrs = 1;
   return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
+
+// Runs `configure` once for each device (a kernel's attributes are the device's); `done` is the caller's
+// static. A thread that loses a race repeats it, which is harmless.
+template <typename Configure>
+cudaError_t oncePerDevice(std::atomic<uint64_t>& done, Configure configure) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  const uint64_t bit = device < 64 ? uint64_t{1} << device : 0;
+  if (e != cudaSuccess || (done.load(std::memory_order_acquire) & bit)) return e;
+  e = configure();
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
 
 template <typename... Params, typename... Args>

@@ -90,7 +90,7 @@ extern "C" sk_status sk_radix_argsort_noalloc(const uint32_t* d_keys, const uint
   cudaError_t e = cudaSuccess;
   if (a.epoch == 1 && raw != 1)  // the counter wrapped: the old status words could match again
     e = cudaMemsetAsync(a.status, 0, static_cast<size_t>(a.statusTiles) * 256 * 8, s);
-  if (e == cudaSuccess) e = sk::sortResetWorkspace(a, s);
+  if (e == cudaSuccess && !sk::sortInOneLaunch(capacity)) e = sk::sortResetWorkspace(a, s);
   if (e == cudaSuccess) e = sk::launchSort(a, s);
   return e == cudaSuccess ? SK_OK : SK_E_DEVICE;
 }

@@ -359,7 +359,7 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
                            static_cast<const uint32_t*>(styleStateTable.ptr), styleStateCount};
     v.sortAccum = sortDigitAccumulators(depthSort);
     v.sortBases = sortDigitBases(depthSort);
-    v.sortPasses = key16 ? 2u : 4u;
+    v.sortPasses = sortInOneLaunch(f.sources) && testWithheldTile == 0 ? 0u : (key16 ? 2u : 4u);
     e = launchVisibility(view.camera, v, degree, key16, lod, s);
   }
   if (timed) cudaEventRecord(events[2], s);
@@ -1216,7 +1216,7 @@ sk_status sk_radix_argsort_device(const uint32_t* d_keys, const uint32_t* d_coun
   a.error = d_error;
   const auto s = static_cast<cudaStream_t>(stream);
   // Counters and histogram accumulators start at zero; status words carry the epoch.
-  cudaError_t e = sk::sortResetWorkspace(a, s);
+  cudaError_t e = sk::sortInOneLaunch(capacity) ? cudaSuccess : sk::sortResetWorkspace(a, s);
   if (e == cudaSuccess) e = sk::launchSort(a, s);
   return e == cudaSuccess ? SK_OK : SK_E_DEVICE;
 }

@@ -52,3 +52,15 @@ def test_a_count_below_the_capacity(cuda_device, n, capacity):
 def test_keys_that_are_all_equal_keep_their_order(cuda_device, value):
     keys = np.full(70_001, value, np.uint32)
     assert np.array_equal(argsort(keys, 32), np.arange(70_001))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 1023, 1024, 1025, 2049, 8192, 8193, 16_385, 20_011, 32_767, 32_768, 32_769])
+@pytest.mark.parametrize("bits", [16, 32])
+def test_sizes_around_the_one_launch_sort(cuda_device, n, bits):
+    """One cluster of 1, 2, 4 or 8 blocks of 1 to 4 rows (cluster_sort.cu) up to 32,768 keys."""
+    rng = np.random.default_rng(n * 3 + bits)
+    keys = rng.integers(0, 1 << bits, n, dtype=np.uint64).astype(np.uint32)
+    keys[rng.random(n) < 0.2] = keys[0]
+    assert np.array_equal(argsort(keys, bits), np.argsort(keys, kind="stable"))
+    assert np.array_equal(argsort(keys[: n // 2], bits, n), np.argsort(keys[: n // 2], kind="stable"))
