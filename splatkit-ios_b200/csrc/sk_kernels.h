@@ -42,13 +42,13 @@ struct VisibilityArgs {
   uint32_t* sortAccum;
   uint32_t* sortBases;
   uint32_t sortPasses;
+  const Camera* cameraInMemory;  // device; null: `camera`, passed with the launch
+  Camera camera;
 };
 uint32_t visibilityTileSplats();               // records of a batch's work item
 uint32_t visibilityTiles(uint32_t total);      // most tiles a frame of up to `total` records has
-// `cam` is a device pointer: the kernels stage it in shared memory, so a captured graph can be
-// replayed with new cameras written into the same buffer.
-cudaError_t launchVisibility(const Camera* cam, const VisibilityArgs& args, int shDegree,
-                             bool key16, bool indexed, cudaStream_t stream);
+cudaError_t launchVisibility(const VisibilityArgs& args, int shDegree, bool key16, bool indexed,
+                             cudaStream_t stream);
 
 // A batch of views (visibility.cu): one launch over every view's records, 16-bit depth keys with
 // the view id above them, survivors of all views contiguous in (view, source) order.

@@ -54,10 +54,16 @@ __device__ __forceinline__ void fillBlockTables() {
   blockReach[threadIdx.x] = quadReach(unorm, kBoundsRadius);
 }
 
-// Copies the view's camera and its near distance into shared memory (the caller syncs).
+// Copies the view's camera and its near distance into shared memory (the caller syncs); the camera is
+// in device memory, or (a plain load) in the kernel's parameters.
 __device__ __forceinline__ void loadView(const Camera* __restrict__ camera, Camera* cam) {
   loadCamera(camera, cam);
   if (threadIdx.x == kThreads - 1) blockZNear = __ldg(&camera->proj[14]) / __ldg(&camera->proj[10]);
+}
+__device__ __forceinline__ void copyView(const Camera& camera, Camera* cam) {
+  if (threadIdx.x < sizeof(Camera) / 4)
+    reinterpret_cast<uint32_t*>(cam)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&camera)[threadIdx.x];
+  if (threadIdx.x == kThreads - 1) blockZNear = camera.proj[14] / camera.proj[10];
 }
 
 __device__ __forceinline__ void mulPoint(const float* m, float x, float y, float z, float w,
@@ -440,7 +446,7 @@ __device__ __forceinline__ uint2 compactTile(VisibilitySmem<kRows>& s, uint64_t*
 
 template <int D, bool kKey16, bool kIndexed, uint32_t kRows>
 __global__ void __launch_bounds__(kThreads, 4)
-    visibilityKernel(const Camera* __restrict__ camera, const __grid_constant__ VisibilityArgs a) {
+    visibilityKernel(const __grid_constant__ VisibilityArgs a) {
   constexpr uint32_t kTile = kThreads * kRows;
   __shared__ VisibilitySmem<kRows> s;
   __shared__ Camera cam;
@@ -450,8 +456,9 @@ __global__ void __launch_bounds__(kThreads, 4)
   fillBlockTables();
   for (uint32_t p = 0; p < a.sortPasses; ++p) digits[p][threadIdx.x] = 0;
   const uint32_t tile = takeTile(a.counters);
+  if (!kIndexed) copyView(a.camera, &cam);
   chainedKernelStart();
-  loadView(camera, &cam);
+  if (kIndexed) loadView(a.cameraInMemory, &cam);
   __syncthreads();
   const uint32_t total = kIndexed ? min(*a.indexCount, a.total) : a.total;
   const uint32_t tiles = (total + kTile - 1) / kTile;
@@ -553,23 +560,23 @@ __global__ void __launch_bounds__(kThreads, 4)
 constexpr uint32_t kSmallTotal = 4 * 148 * kThreads;
 
 template <int D, bool kKey16, bool kIndexed>
-void launchOne(const Camera* cam, const VisibilityArgs& a, cudaStream_t stream) {
+void launchOne(const VisibilityArgs& a, cudaStream_t stream) {
   auto blocks = [&](uint32_t tile) { return max(1u, (a.total + tile - 1) / tile); };
   if (a.total <= kSmallTotal) {
-    launchChained(visibilityKernel<D, kKey16, kIndexed, 1>, blocks(kThreads), kThreads, stream, cam, a);
+    launchChained(visibilityKernel<D, kKey16, kIndexed, 1>, blocks(kThreads), kThreads, stream, a);
   } else {
-    launchChained(visibilityKernel<D, kKey16, kIndexed, kItems>, blocks(kTileSplats), kThreads, stream, cam, a);
+    launchChained(visibilityKernel<D, kKey16, kIndexed, kItems>, blocks(kTileSplats), kThreads, stream, a);
   }
 }
 
 template <int D>
-void launchDegree(const Camera* cam, const VisibilityArgs& a, bool key16, bool indexed, cudaStream_t stream) {
+void launchDegree(const VisibilityArgs& a, bool key16, bool indexed, cudaStream_t stream) {
   if (key16) {
-    if (indexed) launchOne<D, true, true>(cam, a, stream);
-    else launchOne<D, true, false>(cam, a, stream);
+    if (indexed) launchOne<D, true, true>(a, stream);
+    else launchOne<D, true, false>(a, stream);
   } else {
-    if (indexed) launchOne<D, false, true>(cam, a, stream);
-    else launchOne<D, false, false>(cam, a, stream);
+    if (indexed) launchOne<D, false, true>(a, stream);
+    else launchOne<D, false, false>(a, stream);
   }
 }
 
@@ -593,13 +600,13 @@ cudaError_t launchVisibilityBatch(const BatchVisibilityArgs& args, int shDegree,
   return cudaGetLastError();
 }
 
-cudaError_t launchVisibility(const Camera* cam, const VisibilityArgs& args, int shDegree,
+cudaError_t launchVisibility(const VisibilityArgs& args, int shDegree,
                              bool key16, bool indexed, cudaStream_t stream) {
   switch (shDegree) {
-    case 0: launchDegree<0>(cam, args, key16, indexed, stream); break;
-    case 1: launchDegree<1>(cam, args, key16, indexed, stream); break;
-    case 2: launchDegree<2>(cam, args, key16, indexed, stream); break;
-    default: launchDegree<3>(cam, args, key16, indexed, stream); break;
+    case 0: launchDegree<0>(args, key16, indexed, stream); break;
+    case 1: launchDegree<1>(args, key16, indexed, stream); break;
+    case 2: launchDegree<2>(args, key16, indexed, stream); break;
+    default: launchDegree<3>(args, key16, indexed, stream); break;
   }
   return cudaGetLastError();
 }

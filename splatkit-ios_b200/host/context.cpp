@@ -360,7 +360,9 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
     v.sortAccum = sortDigitAccumulators(depthSort);
     v.sortBases = sortDigitBases(depthSort);
     v.sortPasses = sortInOneLaunch(f.sources) && testWithheldTile == 0 ? 0u : (key16 ? 2u : 4u);
-    e = launchVisibility(view.camera, v, degree, key16, lod, s);
+    v.cameraInMemory = lod ? view.camera : nullptr;
+    v.camera = *view.hostCamera;
+    e = launchVisibility(v, degree, key16, lod, s);
   }
   if (timed) cudaEventRecord(events[2], s);
   if (e == cudaSuccess) {
@@ -495,6 +497,7 @@ ViewTarget Context::plainView(const Slot& slot) {
   v.counters = static_cast<FrameCounters*>(second ? frameCounters2.ptr : frameCounters.ptr);
   v.hostCounters = static_cast<FrameCounters*>(slot.hostCounters.ptr);
   v.camera = static_cast<const Camera*>(second ? camera2.ptr : camera.ptr);
+  v.hostCamera = static_cast<const Camera*>(slot.hostCamera.ptr);
   return v;
 }
 
@@ -541,8 +544,11 @@ sk_status Context::enqueueSlot(uint32_t index) {
   slot.direct = view.direct;
   slot.width = width;
   slot.height = height;
-  cudaError_t e = cudaMemcpyAsync(const_cast<Camera*>(view.camera), slot.hostCamera.ptr,
-                                  sizeof(Camera), cudaMemcpyHostToDevice, s);
+  // A flat frame's camera travels in the cull's parameters; a LOD world's walk reads it from memory too.
+  cudaError_t e = cudaSuccess;
+  if (world.lod)
+    e = cudaMemcpyAsync(const_cast<Camera*>(view.camera), slot.hostCamera.ptr, sizeof(Camera),
+                        cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return check(e, "camera upload");
   // the image this frame draws into may still be on its way to a capture's host buffer
   if (imageCopied[slot.image]) {
@@ -598,6 +604,7 @@ sk_status Context::finishOldest() {
     }
     const uint32_t need = static_cast<uint32_t>(
         std::min<uint64_t>(uint64_t{most} + most / 4 + 1024, 0x7fffffffu));
+    ++redraws;
     sk_status st = reserveScratch(scratch, scratch.sources, need, scratch.maxTiles, stream);
     if (st == SK_OK && stream2) st = prepareSecondSlot();
     for (size_t k = 0; st == SK_OK && k < inFlight.size(); ++k) st = enqueueSlot(inFlight[k]);
@@ -1001,11 +1008,25 @@ sk_status sk_wait_idle(sk_context* handle) {
 sk_status sk_read_image(sk_context* handle, void* host, size_t bytes, int32_t format) {
   SK_CTX(handle);
   if (!host) return SK_E_INVALID;
-  sk_status st = ctx->finishFrame(true);
-  if (st != SK_OK) return st;
   const size_t pixels = size_t{ctx->width} * ctx->height;
   const bool deviceFloat = ctx->imageFormat == SK_FORMAT_RGBA32F;
   const size_t need = pixels * (format == SK_FORMAT_RGBA32F ? 16 : 4);
+  // The image in the context's own format follows the newest frame on its stream, so one wait covers
+  // both; it is copied again below when finishing the frames drew them again.
+  const bool own = format == (deviceFloat ? SK_FORMAT_RGBA32F : SK_FORMAT_RGBA8);
+  if (own && bytes >= need && !ctx->inFlight.empty()) {
+    const uint32_t newest = ctx->inFlight.back();
+    const uint64_t redraws = ctx->redraws;
+    cudaError_t e = cudaMemcpyAsync(host, ctx->imageOf(ctx->slots[newest].image), need, cudaMemcpyDeviceToHost,
+                                    ctx->streamOf(newest));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->streamOf(newest));
+    const sk_status copied = ctx->check(e, "readback");
+    if (copied != SK_OK) return copied;
+    const sk_status finished = ctx->finishFrame(true);
+    if (finished != SK_OK || redraws == ctx->redraws) return finished;
+  }
+  sk_status st = ctx->finishFrame(true);
+  if (st != SK_OK) return st;
   if (bytes < need) return ctx->fail(SK_E_INVALID, "image buffer too small");
   if (format == SK_FORMAT_RGBA32F && !deviceFloat)
     return ctx->fail(SK_E_INVALID, "the context renders 8-bit images");

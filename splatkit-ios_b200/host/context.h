@@ -106,7 +106,8 @@ struct ViewTarget {
   void* image = nullptr;                   // device, the context's pixel format
   FrameCounters* counters = nullptr;       // device
   FrameCounters* hostCounters = nullptr;   // pinned; null: no readback
-  const Camera* camera = nullptr;          // device, written before the pipeline runs
+  const Camera* camera = nullptr;          // device, written before the pipeline runs (LOD worlds)
+  const Camera* hostCamera = nullptr;      // the same on the host
   bool direct = false;                     // lists per patch, written in place
   uint32_t tilesX() const { return (width + kTileSize - 1) / kTileSize; }
   uint32_t tilesY() const { return (height + kTileSize - 1) / kTileSize; }
@@ -219,6 +220,7 @@ struct Context {
   // lists (the read-back is per cell); its patch lists are overwritten.
   sk_status expandLists();
   bool listsExpanded = false;  // of the last finished frame
+  uint64_t redraws = 0;        // times the frames in flight were drawn again
   ViewTarget plainView(const Slot& slot);
   sk_status enqueueSlot(uint32_t slot);
   // Finishes the oldest frame in flight (waiting for it); grows the list buffers and draws

@@ -409,14 +409,9 @@ class Frame:
 
     def native(self):
         f = _Frame()
-        view = np.asarray(self.view, np.float32).reshape(16)
-        proj = np.asarray(self.proj, np.float32).reshape(16)
-        for i in range(16):
-            f.view[i] = float(view[i])
-            f.proj[i] = float(proj[i])
-        pos = np.asarray(self.camera_position, np.float32).reshape(3)
-        for i in range(3):
-            f.camera_position[i] = float(pos[i])
+        f.view[:] = np.asarray(self.view, np.float32).reshape(16).tolist()
+        f.proj[:] = np.asarray(self.proj, np.float32).reshape(16).tolist()
+        f.camera_position[:] = np.asarray(self.camera_position, np.float32).reshape(3).tolist()
         f.reveal_level = self.reveal_level
         f.reveal_band = self.reveal_band
         f.reveal_tint_amount = self.reveal_tint_amount
