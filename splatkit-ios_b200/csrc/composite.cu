@@ -246,7 +246,8 @@ __device__ __forceinline__ void writePixel(const CompositeArgs& a, const Target&
   }
 }
 
-// kBatch: block b is batch-wide tile b; its view is the last one whose first tile is <= b.
+// kBatch: block b is batch-wide tile firstTile + b; its view is the last one whose first tile is at or
+// below that.
 // kCount: count blended fragments (a statistic; without it the loop saves an add per splat).
 // kPatches: the lists are per patch, each entry with its cells (else per cell).
 template <int kFormat, bool kBatch, bool kCount, bool kPatches>
@@ -260,12 +261,13 @@ __global__ void __launch_bounds__(kThreads) compositeKernel(const __grid_constan
     t.patchesX = g.x, t.patchShift = g.shift;
   }
   if constexpr (kBatch) {
-    const uint32_t lo = lastAtOrBelow(a.viewCount, blockIdx.x, [&](uint32_t v) { return __ldg(&a.views[v].tileBase); });
+    const uint32_t tile = a.firstTile + blockIdx.x;
+    const uint32_t lo = lastAtOrBelow(a.viewCount, tile, [&](uint32_t v) { return __ldg(&a.views[v].tileBase); });
     const BatchView* v = a.views + lo;
     t.width = __ldg(&v->width);
     t.height = __ldg(&v->height);
     t.tilesX = __ldg(&v->tilesX);
-    t.tile = blockIdx.x - __ldg(&v->tileBase);
+    t.tile = tile - __ldg(&v->tileBase);
     t.binsX = __ldg(&v->binsX);
     t.listBase = a.patches ? __ldg(&v->patchBase) : __ldg(&v->binBase);
     if constexpr (kPatches) {

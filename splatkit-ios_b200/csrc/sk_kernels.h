@@ -223,10 +223,11 @@ struct CompositeArgs {
   uint32_t* fragments;  // FrameCounters.fragments_lo/hi (64-bit add), when countFragments
   uint32_t countFragments;
   uint32_t* loaded;     // FrameCounters.loaded
-  // a batch (viewCount > 0): one block per batch-wide tile, image = the batch image
+  // a batch (viewCount > 0): one block per batch-wide tile firstTile .. firstTile + batchTiles, image =
+  // the batch image
   const BatchView* views;
   uint32_t viewCount;
-  uint32_t batchTiles;
+  uint32_t firstTile, batchTiles;
 };
 cudaError_t launchComposite(const CompositeArgs& args, cudaStream_t stream);
 

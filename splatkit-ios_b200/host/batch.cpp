@@ -27,6 +27,12 @@ BatchLane::~BatchLane() {
   if (done) cudaEventDestroy(done);
   if (start) cudaEventDestroy(start);
   if (end) cudaEventDestroy(end);
+  if (copyStream) {
+    cudaStreamSynchronize(copyStream);
+    cudaStreamDestroy(copyStream);
+  }
+  for (cudaEvent_t e : composited) cudaEventDestroy(e);
+  if (copied) cudaEventDestroy(copied);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -486,27 +492,90 @@ sk_status Batch::enqueueStages(BatchLane& l, bool clearStatus) {
   if (e == cudaSuccess && !l.directLists)
     e = launchTileRanges(static_cast<const uint32_t*>(l.instKeysSorted.ptr), &fc->instances,
                          l.instances, static_cast<uint2*>(l.ranges.ptr), l.totalBins, s);
-  if (e == cudaSuccess) {
-    CompositeArgs c{};
-    c.projected = static_cast<const Projected*>(l.projected.ptr);
-    c.values = static_cast<const uint32_t*>(l.instValuesSorted.ptr);
-    c.masks = l.directLists && l.patchMasks ? static_cast<const uint16_t*>(l.instKeysSorted.ptr) : nullptr;
-    c.ranges = static_cast<const uint2*>(l.ranges.ptr);
-    for (int j = 0; j < 3; ++j) c.background[j] = static_cast<float>(policy.background[j]);
-    c.opaque = 1;
-    c.cutoff = policy.enable_early_termination ? kTransmittanceCutoff : 0.0f;
-    c.image = l.image.ptr;
-    c.format = kRgba8;
-    c.fragments = &fc->fragments_lo;
-    c.countFragments = 1;
-    c.loaded = &fc->loaded;
-    c.views = views;
-    c.patches = l.directLists ? 1u : 0u;
-    c.viewCount = l.viewCount;
-    c.batchTiles = l.totalTiles;
-    e = launchComposite(c, s);
-  }
   return check(e, "batch stages");
+}
+
+// A composite launch and its views' copies run side by side with the next launch, so the images of a large
+// submission cross PCIe while it is still drawn (16 served requests of up to 4K: 3.1 ms of copies, which
+// followed 3 ms of compositing). A launch holds at least this many tiles (2 megapixels): each ends in a
+// partly filled wave of about 20 us.
+constexpr uint32_t kChunkTiles = 8192;
+
+std::vector<uint32_t> Batch::compositeChunks(const BatchLane& l) const {
+  std::vector<uint32_t> ends;
+  uint32_t begin = 0;
+  for (uint32_t v = 1; v < l.viewCount; ++v) {
+    const uint32_t at = l.table[v].tileBase;
+    if (at - begin >= kChunkTiles && l.totalTiles - at >= kChunkTiles) {
+      ends.push_back(v);
+      begin = at;
+    }
+  }
+  ends.push_back(l.viewCount);
+  return ends;
+}
+
+sk_status Batch::enqueueImages(BatchLane& l) {
+  const cudaStream_t s = l.stream;
+  FrameCounters* fc = static_cast<FrameCounters*>(l.frameCounters.ptr);
+  CompositeArgs c{};
+  c.projected = static_cast<const Projected*>(l.projected.ptr);
+  c.values = static_cast<const uint32_t*>(l.instValuesSorted.ptr);
+  c.masks = l.directLists && l.patchMasks ? static_cast<const uint16_t*>(l.instKeysSorted.ptr) : nullptr;
+  c.ranges = static_cast<const uint2*>(l.ranges.ptr);
+  for (int j = 0; j < 3; ++j) c.background[j] = static_cast<float>(policy.background[j]);
+  c.opaque = 1;
+  c.cutoff = policy.enable_early_termination ? kTransmittanceCutoff : 0.0f;
+  c.image = l.image.ptr;
+  c.format = kRgba8;
+  c.fragments = &fc->fragments_lo;
+  c.countFragments = 1;
+  c.loaded = &fc->loaded;
+  c.views = static_cast<const BatchView*>(l.viewTable.ptr);
+  c.patches = l.directLists ? 1u : 0u;
+  c.viewCount = l.viewCount;
+  const std::vector<uint32_t> ends = compositeChunks(l);
+  const bool aside = ends.size() > 1;
+  cudaError_t e = cudaSuccess;
+  if (aside && !l.copyStream) e = cudaStreamCreateWithFlags(&l.copyStream, cudaStreamNonBlocking);
+  if (aside && !l.copied && e == cudaSuccess) e = cudaEventCreateWithFlags(&l.copied, cudaEventDisableTiming);
+  while (aside && e == cudaSuccess && l.composited.size() < ends.size()) {
+    cudaEvent_t ev = nullptr;
+    e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) l.composited.push_back(ev);
+  }
+  const cudaStream_t copies = aside ? l.copyStream : s;
+  const auto* image = static_cast<const uint8_t*>(l.image.ptr);
+  auto tileAt = [&](uint32_t v) { return v < l.viewCount ? l.table[v].tileBase : l.totalTiles; };
+  auto pixelAt = [&](uint32_t v) { return v < l.viewCount ? l.table[v].pixelOffset : l.totalPixels; };
+  for (size_t k = 0; k < ends.size() && e == cudaSuccess; ++k) {
+    c.firstTile = tileAt(k ? ends[k - 1] : 0u);
+    c.batchTiles = tileAt(ends[k]) - c.firstTile;
+    e = launchComposite(c, s);
+    if (aside && e == cudaSuccess) e = cudaEventRecord(l.composited[k], s);
+  }
+  // (after every launch: a copy to pageable memory blocks this thread until it is done)
+  for (size_t k = 0; k < ends.size() && e == cudaSuccess; ++k) {
+    const uint32_t first = k ? ends[k - 1] : 0u, last = ends[k];
+    if (aside) e = cudaStreamWaitEvent(copies, l.composited[k], 0);
+    if (l.destinations.empty()) {
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(static_cast<uint8_t*>(l.hostImage.ptr) + pixelAt(first) * 4, image + pixelAt(first) * 4,
+                            (pixelAt(last) - pixelAt(first)) * 4, cudaMemcpyDeviceToHost, copies);
+    } else {
+      for (uint32_t v = first; v < last && e == cudaSuccess; ++v) {
+        const BatchView& t = l.table[v];
+        if (l.destinations[v])
+          e = cudaMemcpyAsync(l.destinations[v], image + t.pixelOffset * 4, size_t{t.width} * t.height * 4,
+                              cudaMemcpyDeviceToHost, copies);
+      }
+    }
+  }
+  if (aside) {  // the lane's stream goes on, and the submission is done, when the images have landed
+    if (e == cudaSuccess) e = cudaEventRecord(l.copied, copies);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, l.copied, 0);
+  }
+  return check(e, "batch images");
 }
 
 sk_status Batch::enqueue(BatchLane& l) {
@@ -539,6 +608,7 @@ sk_status Batch::enqueue(BatchLane& l) {
                           cudaMemcpyHostToDevice, s);
     if (r != cudaSuccess) return check(r, "batch upload");
     sk_status st = enqueueStages(l, clearStatus);
+    if (st == SK_OK) st = enqueueImages(l);
     if (st != SK_OK) return st;
     r = cudaMemcpyAsync(l.hostCounters.ptr, l.frameCounters.ptr, sizeof(FrameCounters),
                         cudaMemcpyDeviceToHost, s);
@@ -548,17 +618,6 @@ sk_status Batch::enqueue(BatchLane& l) {
     if (r == cudaSuccess && !l.lodPlans.empty())
       r = cudaMemcpyAsync(l.hostLodReports.ptr, l.lodReports.ptr, l.lodPlans.size() * 8 * 4,
                           cudaMemcpyDeviceToHost, s);
-    if (l.destinations.empty()) {
-      if (r == cudaSuccess)
-        r = cudaMemcpyAsync(l.hostImage.ptr, l.image.ptr, l.totalPixels * 4, cudaMemcpyDeviceToHost, s);
-    } else {
-      for (uint32_t i = 0; i < l.viewCount && r == cudaSuccess; ++i) {
-        const BatchView& t = l.table[i];
-        if (l.destinations[i])
-          r = cudaMemcpyAsync(l.destinations[i], static_cast<const uint8_t*>(l.image.ptr) + t.pixelOffset * 4,
-                              size_t{t.width} * t.height * 4, cudaMemcpyDeviceToHost, s);
-      }
-    }
     return check(r, "batch readback");
   };
   sk_status st = SK_OK;

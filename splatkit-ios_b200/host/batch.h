@@ -51,6 +51,11 @@ struct LodPlan {
 struct BatchLane {
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr, start = nullptr, end = nullptr;
+  // The images of a submission of several composite launches are copied to the host on their own
+  // stream, each launch's views while the next ones are composited; copied: the last of them.
+  cudaStream_t copyStream = nullptr;
+  std::vector<cudaEvent_t> composited;  // one per launch
+  cudaEvent_t copied = nullptr;
   // capacities
   uint32_t sources = 0, instances = 0, items = 0, tiles = 0, views = 0;
   uint64_t pixels = 0;
@@ -121,6 +126,10 @@ struct Batch {
   // Enqueues the lane's whole batch on its stream (uploads, stages, readbacks, done event).
   sk_status enqueue(BatchLane& lane);
   sk_status enqueueStages(BatchLane& lane, bool clearStatus);
+  // The composite launches and the copies of the images.
+  sk_status enqueueImages(BatchLane& lane);
+  // The views each composite launch ends before (the last: all of them).
+  std::vector<uint32_t> compositeChunks(const BatchLane& lane) const;
   // Waits for (or polls) the lane's submission; grows and redraws on instance overflow.
   sk_status finish(BatchLane& lane, bool wait);
   BatchLane* laneOf(uint64_t ticket);
