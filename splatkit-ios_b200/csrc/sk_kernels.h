@@ -32,7 +32,7 @@ struct VisibilityArgs {
   uint4* spans;  // per survivor: the binning cells its quad touches (sk_tiles.cuh)
   uint32_t tilesX, tilesY;  // binning cells (kBinSize pixels) per row and column
   uint32_t* visibleCount;
-  uint64_t* status;    // one word per tile: visibilityTiles(total)
+  uint64_t* status;    // one word per tile of visibilityTileSplats() records
   uint32_t* counters;  // two words
   uint32_t epoch;
   uint32_t* error;
@@ -45,8 +45,7 @@ struct VisibilityArgs {
   const Camera* cameraInMemory;  // device; null: `camera`, passed with the launch
   Camera camera;
 };
-uint32_t visibilityTileSplats();               // records of a batch's work item
-uint32_t visibilityTiles(uint32_t total);      // most tiles a frame of up to `total` records has
+uint32_t visibilityTileSplats();  // records of a tile, and of a batch's work item
 cudaError_t launchVisibility(const VisibilityArgs& args, int shDegree, bool key16, bool indexed,
                              cudaStream_t stream);
 
@@ -56,7 +55,7 @@ struct BatchVisibilityArgs {
   const BatchView* views;   // viewCount entries
   const Camera* cameras;    // one per view (device)
   uint32_t viewCount;
-  uint32_t items;           // work items: sum over views of max(1, ceil(count / 1024))
+  uint32_t items;           // work items: per view max(1, ceil(count / visibilityTileSplats()))
   uint32_t* keys;
   Projected* projected;
   uint4* spans;

@@ -165,7 +165,7 @@ struct alignas(16) BatchView {
   uint32_t shStride;     // harmonics words per record of this world
   uint32_t offset;       // first record drawn
   uint32_t count;        // records drawn
-  uint32_t itemStart;    // first visibility work item (1024-record chunk) of this view
+  uint32_t itemStart;    // first visibility work item (256-record chunk) of this view
   uint32_t tileBase;     // first batch-wide composite tile of this view
   uint32_t binBase;      // first batch-wide binning cell of this view
   uint32_t tilesX;       // composite tiles per row

@@ -4,10 +4,18 @@
 //
 // Follows splatkit-ios/Sources/SplatKitCore/rendering/metal/layout/SplatProjection.metalh:6-141
 // and .../metal/cull/SplatVisibility.metal:16-106. The reference compacts with one atomic per
-// SIMD group, so its survivor order depends on scheduling; here each 1024-splat tile counts
+// SIMD group, so its survivor order depends on scheduling; here each 256-splat tile counts
 // its survivors, takes its offset by decoupled look-back and writes them in source order, so
 // the sorted order downstream is deterministic and equal to a stable sort of (key, source
 // position).
+//
+// A frame larger than L2 is bound by latency (1M SH3 splats, 128 MB: 65 us, 2 TB/s, 22 us at the measured
+// peak), a batch of many waves by instructions (12M splats in 560 us, 476 without the harmonics' arithmetic).
+// One splat per thread, four blocks per SM that take tiles in turn and look a tile's place up one tile
+// later: 80 -> 65 us (1M), 222 -> 201 (3M), 30 -> 18 (a 0.4M-splat LOD cut), 15.5 -> 8.0 (4k) against 1024-splat
+// tiles that waited at once. With two splats per thread 78 us (1M), with three blocks per SM 71, with five 74.
+// The quad radius by 8-bit opacity from a table, saturating half conversions and 32 views searched at once
+// are the batch's share (604 -> 560 us).
 //
 // Built with -fmad=false: every product and sum rounds on its own, in the order written.
 #include <cuda_runtime.h>
@@ -31,10 +39,8 @@ constexpr uint32_t kDepthKeyMax = 65535;
 
 constexpr uint32_t kThreads = 256;
 constexpr uint32_t kWarps = kThreads / 32;
-// Splats per thread: tiles of 1024 splats, or of 256 where that many blocks fit the chip at once
-// (launchVisibility).
-constexpr uint32_t kItems = 4;
-constexpr uint32_t kTileSplats = kThreads * kItems;
+constexpr uint32_t kTileSplats = kThreads;     // a splat per thread
+constexpr uint32_t kResidentBlocks = 148 * 4;  // of either kernel
 
 // Per block, by 8-bit opacity: i / 255 (also the 8-bit colour channels: the same IEEE quotients the
 // division gives, computed once per block instead of four times per splat) and the quad radius that
@@ -314,141 +320,179 @@ __device__ __forceinline__ uint32_t sourceIndex(const VisibilityArgs& a, uint32_
   return a.ranges[lo].offset + (t - a.rangeStarts[lo]);
 }
 
-// Shared memory of one tile: survivors staged at their source slot, then compacted.
-template <uint32_t kRows>
-struct VisibilitySmem {
-  static constexpr uint32_t kSlots = kThreads * kRows;
-  uint4 rec[kSlots * 2];     // projected records by source slot
-  uint32_t key[kSlots];      // depth keys by source slot
-  uint16_t slotOf[kSlots];   // survivor k of the tile -> its source slot
-  uint32_t rowMask[kWarps][kRows];
-  uint32_t warpTotal[kWarps];
-  uint32_t tileBase;
+// One tile in shared memory: survivors staged at their source slot, then compacted.
+struct TileSmem {
+  uint4 rec[kTileSplats * 2];    // projected records by source slot
+  uint32_t key[kTileSplats];     // depth keys by source slot
+  uint16_t slotOf[kTileSplats];  // survivor k of the tile -> its source slot
+  uint32_t survivors[kWarps];    // per warp: a bit per lane
 };
 
-// Projects one tile (kRows records per thread) into shared memory: survivors' keys and records at their
-// source slot, and per warp row the mask of survivors. Part styles (when labels are given) and
-// the reveal glow are applied to each survivor's record after its projection. indexOf(t) gives the record index of
-// tile position t, or 0xffffffff past the end. keyHigh is or-ed into every key (the view id of a
-// batch, above a 16-bit key). One record per row of the warp, not unrolled (the projection is
-// large); the next row's record is fetched while this one is projected.
-template <int D, bool kKey16, uint32_t kRows, typename IndexOf>
-__device__ __forceinline__ void projectTile(VisibilitySmem<kRows>& s, const Camera& cam,
-                                            const GpuSplat* __restrict__ splats,
+// A block works on two tiles: one whose survivors wait for their place in the output, and the next one,
+// projected meanwhile.
+struct VisibilitySmem {
+  TileSmem tile[2];
+  uint32_t next;      // the tile after the one being projected
+  uint32_t tileBase;  // survivors before the waiting tile
+};
+
+// Projects one tile into shared memory, a record per thread: survivors' keys and records at their source
+// slot, and per warp the mask of survivors. Part styles (when labels are given) and the reveal glow are
+// applied to each survivor's record after its projection. index is this thread's record, 0xffffffff past
+// the end. keyHigh is or-ed into every key (the view id of a batch, above a 16-bit key).
+template <int D, bool kKey16>
+__device__ __forceinline__ void projectTile(TileSmem& s, const Camera& cam, const GpuSplat* __restrict__ splats,
                                             const uint32_t* __restrict__ sh, uint32_t shStride,
-                                            const PartLabels& parts, uint32_t first,
-                                            uint32_t keyHigh, IndexOf indexOf) {
-  const uint32_t warp = threadIdx.x >> 5, lane = laneId();
-  uint32_t index = indexOf(first);
-  uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+                                            const PartLabels& parts, uint32_t index, uint32_t keyHigh) {
+  bool visible = false;
   if (index != 0xffffffffu) {
     const uint4* p = reinterpret_cast<const uint4*>(splats + index);
-    lo = __ldg(p), hi = __ldg(p + 1);
-  }
-#pragma unroll 1
-  for (uint32_t r = 0; r < kRows; ++r) {
-    uint32_t nextIndex = 0xffffffffu;
-    uint4 nextLo = make_uint4(0, 0, 0, 0), nextHi = nextLo;
-    if (r + 1 < kRows) {
-      nextIndex = indexOf(first + (r + 1) * 32);
-      if (nextIndex != 0xffffffffu) {
-        const uint4* p = reinterpret_cast<const uint4*>(splats + nextIndex);
-        nextLo = __ldg(p), nextHi = __ldg(p + 1);
-      }
+    const uint4 lo = __ldg(p), hi = __ldg(p + 1);
+    uint32_t key, rec[8];
+    visible = projectSplat<D, kKey16>(cam, lo, hi, index, sh, shStride, key, rec);
+    if (visible && parts.labels) visible = styleRecord(parts, index, rec);
+    if (visible) revealGlow(cam, asF(lo.y), rec);
+    if (visible) {
+      const uint32_t slot = threadIdx.x;
+      s.key[slot] = key | keyHigh;
+      s.rec[2 * slot] = make_uint4(rec[0], rec[1], rec[2], rec[3]);
+      s.rec[2 * slot + 1] = make_uint4(rec[4], rec[5], rec[6], rec[7]);
     }
-    bool visible = false;
-    const uint32_t slot = warp * (32 * kRows) + r * 32 + lane;
-    if (index != 0xffffffffu) {
-      uint32_t key, rec[8];
-      visible = projectSplat<D, kKey16>(cam, lo, hi, index, sh, shStride, key, rec);
-      if (visible && parts.labels) visible = styleRecord(parts, index, rec);
-      if (visible) revealGlow(cam, asF(lo.y), rec);
-      if (visible) {
-        s.key[slot] = key | keyHigh;
-        s.rec[2 * slot] = make_uint4(rec[0], rec[1], rec[2], rec[3]);
-        s.rec[2 * slot + 1] = make_uint4(rec[4], rec[5], rec[6], rec[7]);
-      }
-    }
-    const uint32_t mask = __ballot_sync(0xffffffffu, visible);
-    if (lane == 0) s.rowMask[warp][r] = mask;
-    index = nextIndex, lo = nextLo, hi = nextHi;
   }
-  __syncwarp();
+  const uint32_t mask = __ballot_sync(0xffffffffu, visible);
+  if (laneId() == 0) s.survivors[threadIdx.x >> 5] = mask;
 }
 
-// Order-preserving compaction of the tile's survivors and their copy-out: the tile's count is published,
-// survivor k -> its source slot, then one warp takes the tile's offset by decoupled look-back over
-// status[0 .. tile] while the others work out the cells each survivor's quad touches (on a width x height
-// target), and consecutive threads write consecutive survivors. With digitPasses > 0 each key's 8-bit
-// digits are counted into digits[pass][digit]. Returns the survivors before and in the tile.
-template <uint32_t kRows>
-__device__ __forceinline__ uint2 compactTile(VisibilitySmem<kRows>& s, uint64_t* status, uint32_t tile,
-                                             uint32_t epoch, uint32_t* error, uint32_t* keys,
-                                             Projected* projected, uint4* spans, float width, float height,
-                                             uint32_t tilesX, uint32_t tilesY,
-                                             uint32_t (*digits)[256] = nullptr, uint32_t digitPasses = 0) {
+// A block's tiles, taken in start order until none is left. Survivors are compacted in source order: a
+// tile's place follows from the counts of the tiles before it by decoupled look-back over
+// out.status[0 .. tile]. A tile's count is published as soon as it is projected, but its place is looked up
+// only after the block has projected its next tile, when the tiles before it have long published theirs
+// (looked up at once, a third of the warps' time went by at the barriers behind it: tiles that start
+// together end together). The source names the tiles: enter (all threads, no barrier) loads tile's view for
+// buffer b, project projects it, width/height/binsX/binsY are b's target, finish takes its place and count.
+// With digitPasses > 0 each survivor key's 8-bit digits are counted into digits[pass][digit].
+struct VisibilityOut {
+  uint32_t* keys;
+  Projected* projected;
+  uint4* spans;
+  uint64_t* status;
+  uint32_t* counters;
+  uint32_t epoch;
+  uint32_t* error;
+};
+
+template <typename Source>
+__device__ __forceinline__ void runTiles(VisibilitySmem& s, Source& source, const VisibilityOut& out,
+                                         uint32_t tile, uint32_t tiles, uint32_t (*digits)[256],
+                                         uint32_t digitPasses) {
   const uint32_t warp = threadIdx.x >> 5, lane = laneId();
-  uint32_t mine = 0;
+  constexpr uint32_t kNone = 0xffffffffu;
+  uint32_t waiting = kNone, waitingCount = 0;
+  for (uint32_t b = 0; tile < tiles || waiting != kNone; b ^= 1u) {
+    const bool have = tile < tiles;
+    TileSmem& t = s.tile[b];
+    const TileSmem& w = s.tile[b ^ 1u];
+    if (have) source.project(t, tile, b);
+    if (threadIdx.x == 0) s.next = have ? atomicAdd(&out.counters[0], 1u) : kNone;
+    __syncthreads();
+    uint32_t count = 0;
+    if (have) {
+      uint32_t pos = 0;
 #pragma unroll
-  for (uint32_t r = 0; r < kRows; ++r) mine += __popc(s.rowMask[warp][r]);
-  if (lane == 0) s.warpTotal[warp] = mine;
-  __syncthreads();
-  uint32_t count = 0, pos = 0;
-#pragma unroll
-  for (uint32_t w = 0; w < kWarps; ++w) {
-    if (w == warp) pos = count;
-    count += s.warpTotal[w];
-  }
-  if (threadIdx.x == 0) storeStatus(status + tile, makeStatus(epoch, tile == 0 ? kFlagPrefix : kFlagAggregate, count));
-  const uint32_t below = lanemaskLt();
-#pragma unroll
-  for (uint32_t r = 0; r < kRows; ++r) {
-    const uint32_t mask = s.rowMask[warp][r];
-    if (mask & (1u << lane)) s.slotOf[pos + __popc(mask & below)] = warp * (32 * kRows) + r * 32 + lane;
-    pos += __popc(mask);
-  }
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t before = 0;
-    if (tile != 0) {
-      before = warpLookback(status, tile, epoch, error);
-      if (lane == 0) storeStatus(status + tile, makeStatus(epoch, kFlagPrefix, before + count));
+      for (uint32_t v = 0; v < kWarps; ++v) {
+        if (v == warp) pos = count;
+        count += __popc(t.survivors[v]);
+      }
+      if (threadIdx.x == 0)
+        storeStatus(out.status + tile, makeStatus(out.epoch, tile == 0 ? kFlagPrefix : kFlagAggregate, count));
+      const uint32_t mask = t.survivors[warp];
+      if (mask & (1u << lane)) t.slotOf[pos + __popc(mask & lanemaskLt())] = static_cast<uint16_t>(threadIdx.x);
     }
-    if (lane == 0) s.tileBase = before;
-  }
-  uint4 span[kRows];
-#pragma unroll
-  for (uint32_t r = 0; r < kRows; ++r) {
-    const uint32_t k = threadIdx.x + r * kThreads;
-    if (k < count) {
-      const uint32_t slot = s.slotOf[k];
-      span[r] = tileSpan(s.rec[2 * slot], s.rec[2 * slot + 1], width, height, tilesX, tilesY);
-      const uint32_t key = s.key[slot];
-      for (uint32_t p = 0; p < digitPasses; ++p) atomicAdd(&digits[p][(key >> (8 * p)) & 0xffu], 1u);
+    uint4 span = make_uint4(0, 0, 0, 0);
+    const uint32_t k = threadIdx.x;
+    if (waiting != kNone) {
+      if (warp == 0) {
+        uint32_t before = 0;
+        if (waiting != 0) {
+          before = warpLookback(out.status, waiting, out.epoch, out.error);
+          if (lane == 0) storeStatus(out.status + waiting, makeStatus(out.epoch, kFlagPrefix, before + waitingCount));
+        }
+        if (lane == 0) s.tileBase = before;
+      }
+      if (k < waitingCount) {
+        const uint32_t slot = w.slotOf[k];
+        span = tileSpan(w.rec[2 * slot], w.rec[2 * slot + 1], source.width(b ^ 1u), source.height(b ^ 1u),
+                        source.binsX(b ^ 1u), source.binsY(b ^ 1u));
+        const uint32_t key = w.key[slot];
+        for (uint32_t p = 0; p < digitPasses; ++p) atomicAdd(&digits[p][(key >> (8 * p)) & 0xffu], 1u);
+      }
+    }
+    __syncthreads();
+    if (waiting != kNone) {
+      const uint32_t base = s.tileBase;
+      if (k < waitingCount) {
+        const uint32_t slot = w.slotOf[k];
+        out.keys[base + k] = w.key[slot];
+        uint4* o = reinterpret_cast<uint4*>(out.projected + base + k);
+        o[0] = w.rec[2 * slot];
+        o[1] = w.rec[2 * slot + 1];
+        out.spans[base + k] = span;
+      }
+      if (threadIdx.x == 0) source.finish(waiting, b ^ 1u, base, waitingCount);
+    }
+    waiting = have ? tile : kNone;
+    waitingCount = count;
+    tile = s.next;
+    __syncthreads();  // the waiting tile's buffer, s.next and s.tileBase are free
+    if (tile < tiles) {
+      source.enter(tile, b ^ 1u);
+      if constexpr (Source::kEnters) __syncthreads();
     }
   }
-  __syncthreads();
-  const uint32_t base = s.tileBase;
-#pragma unroll
-  for (uint32_t r = 0; r < kRows; ++r) {
-    const uint32_t k = threadIdx.x + r * kThreads;
-    if (k < count) {
-      const uint32_t slot = s.slotOf[k];
-      keys[base + k] = s.key[slot];
-      uint4* o = reinterpret_cast<uint4*>(projected + base + k);
-      o[0] = s.rec[2 * slot];
-      o[1] = s.rec[2 * slot + 1];
-      spans[base + k] = span[r];
-    }
-  }
-  return make_uint2(base, count);
 }
 
-template <int D, bool kKey16, bool kIndexed, uint32_t kRows>
+// A frame's tiles: the records of its ranges, or of a LOD cut, on one target.
+template <int D, bool kKey16, bool kIndexed>
+struct FrameSource {
+  static constexpr bool kEnters = false;
+  const VisibilityArgs& a;
+  const Camera& cam;
+  uint32_t total, tiles;
+
+  // Asks for this thread's record of the tile (and its harmonics) ahead of their loads.
+  __device__ __forceinline__ void enter(uint32_t tile, uint32_t) {
+    const uint32_t at = tile * kTileSplats + threadIdx.x;
+    if (at >= total || (!kIndexed && a.rangeCount != 1)) return;
+    const uint32_t index = kIndexed ? a.indices[at] : a.single.offset + at;
+    if (index >= a.worldCount) return;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.splats + index));
+    if (D > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.sh + size_t{index} * a.shStride));
+  }
+  __device__ __forceinline__ void project(TileSmem& t, uint32_t tile, uint32_t) {
+    const uint32_t at = tile * kTileSplats + threadIdx.x;
+    uint32_t index = 0xffffffffu;
+    if (at < total) {
+      index = kIndexed ? a.indices[at] : sourceIndex(a, at);
+      if (index >= a.worldCount) {
+        atomicOr(a.error, SK_DEVERR_BOUNDS);
+        index = 0xffffffffu;
+      }
+    }
+    projectTile<D, kKey16>(t, cam, a.splats, a.sh, a.shStride, a.parts, index, 0u);
+  }
+  __device__ __forceinline__ float width(uint32_t) const { return cam.screenSize[0]; }
+  __device__ __forceinline__ float height(uint32_t) const { return cam.screenSize[1]; }
+  __device__ __forceinline__ uint32_t binsX(uint32_t) const { return a.tilesX; }
+  __device__ __forceinline__ uint32_t binsY(uint32_t) const { return a.tilesY; }
+  __device__ __forceinline__ void finish(uint32_t tile, uint32_t, uint32_t before, uint32_t count) {
+    if (tile == tiles - 1) *a.visibleCount = before + count;
+  }
+};
+
+template <int D, bool kKey16, bool kIndexed>
 __global__ void __launch_bounds__(kThreads, 4)
     visibilityKernel(const __grid_constant__ VisibilityArgs a) {
-  constexpr uint32_t kTile = kThreads * kRows;
-  __shared__ VisibilitySmem<kRows> s;
+  __shared__ VisibilitySmem s;
   __shared__ Camera cam;
   __shared__ uint32_t digits[4][256];
   // Before the wait for the kernel before this one: what depends on nothing it writes (the tile counter
@@ -461,24 +505,10 @@ __global__ void __launch_bounds__(kThreads, 4)
   if (kIndexed) loadView(a.cameraInMemory, &cam);
   __syncthreads();
   const uint32_t total = kIndexed ? min(*a.indexCount, a.total) : a.total;
-  const uint32_t tiles = (total + kTile - 1) / kTile;
-  if (tile < tiles) {
-    const uint32_t warp = threadIdx.x >> 5, lane = laneId();
-    const uint32_t first = tile * kTile + warp * (32 * kRows) + lane;
-    auto indexOf = [&](uint32_t t) -> uint32_t {
-      if (t >= total) return 0xffffffffu;
-      const uint32_t index = kIndexed ? a.indices[t] : sourceIndex(a, t);
-      if (index >= a.worldCount) {
-        atomicOr(a.error, SK_DEVERR_BOUNDS);
-        return 0xffffffffu;
-      }
-      return index;
-    };
-    projectTile<D, kKey16>(s, cam, a.splats, a.sh, a.shStride, a.parts, first, 0u, indexOf);
-    const uint2 at = compactTile(s, a.status, tile, a.epoch, a.error, a.keys, a.projected, a.spans,
-                                 cam.screenSize[0], cam.screenSize[1], a.tilesX, a.tilesY, digits, a.sortPasses);
-    if (tile == tiles - 1 && threadIdx.x == 0) *a.visibleCount = at.x + at.y;
-  }
+  const uint32_t tiles = (total + kTileSplats - 1) / kTileSplats;
+  FrameSource<D, kKey16, kIndexed> source{a, cam, total, tiles};
+  runTiles(s, source, VisibilityOut{a.keys, a.projected, a.spans, a.status, a.counters, a.epoch, a.error}, tile, tiles,
+           digits, a.sortPasses);
   if (tiles == 0 && tile == 0 && threadIdx.x == 0) *a.visibleCount = 0;
   if (a.sortPasses) {
     __syncthreads();
@@ -492,81 +522,79 @@ __global__ void __launch_bounds__(kThreads, 4)
   finishTile(a.counters);
 }
 
-// A batch of views in one launch. Work item i is a 1024-record chunk of one view's range (or of
+// A batch of views in one launch. Work item i is a 256-record chunk of one view's range (or of
 // a LOD view's cut, in emission order: the chunks past the cut's length hold nothing); items
 // are numbered view by view, so one look-back chain over all items places every view's
 // survivors contiguously, in (view, source) order, and the first item of each view records
 // where that view starts. Keys carry the view id above the 16-bit depth key, so one stable
 // sort orders all views at once.
 template <int D>
-__global__ void __launch_bounds__(kThreads, 4)
-    visibilityBatchKernel(const __grid_constant__ BatchVisibilityArgs a) {
-  __shared__ VisibilitySmem<kItems> s;
-  __shared__ Camera cam;
-  __shared__ BatchView view;
-  fillBlockTables();
-  const uint32_t item = takeTile(a.counters);
-  chainedKernelStart();
-  if (item < a.items) {
+struct BatchSource {
+  static constexpr bool kEnters = true;
+  const BatchVisibilityArgs& a;
+  Camera& cam;
+  BatchView* view;     // per buffer
+  uint32_t* viewIndex; // per buffer
+
+  __device__ __forceinline__ void enter(uint32_t item, uint32_t b) {
     // the last view whose first item is <= item
     const uint32_t v = lastAtOrBelow(a.viewCount, item, [&](uint32_t i) { return __ldg(&a.views[i].itemStart); });
     loadView(a.cameras + v, &cam);
     if (threadIdx.x < sizeof(BatchView) / 4)
-      reinterpret_cast<uint32_t*>(&view)[threadIdx.x] =
+      reinterpret_cast<uint32_t*>(view + b)[threadIdx.x] =
           __ldg(reinterpret_cast<const uint32_t*>(a.views + v) + threadIdx.x);
-    __syncthreads();
-    const uint32_t chunk = item - view.itemStart;
-    const uint32_t warp = threadIdx.x >> 5, lane = laneId();
-    const uint32_t first = chunk * kTileSplats + warp * (32 * kItems) + lane;
+    if (threadIdx.x == 0) viewIndex[b] = v;
+  }
+  __device__ __forceinline__ void project(TileSmem& t, uint32_t item, uint32_t b) {
+    const BatchView& w = view[b];
+    const uint32_t at = (item - w.itemStart) * kTileSplats + threadIdx.x;
     // a LOD view draws its cut (written by this stream's selection before this kernel)
-    const uint32_t drawn = view.indices ? min(view.count, *view.indexCount) : view.count;
-    auto indexOf = [&](uint32_t t) -> uint32_t {
-      if (t >= drawn) return 0xffffffffu;
-      if (!view.indices) return view.offset + t;
-      const uint32_t index = view.indices[t];
-      if (index >= view.worldCount) {
+    const uint32_t drawn = w.indices ? min(w.count, *w.indexCount) : w.count;
+    uint32_t index = 0xffffffffu;
+    if (at < drawn) {
+      index = w.indices ? w.indices[at] : w.offset + at;
+      if (w.indices && index >= w.worldCount) {
         atomicOr(a.error, SK_DEVERR_BOUNDS);
-        return 0xffffffffu;
-      }
-      return index;
-    };
-    projectTile<D, true>(s, cam, view.splats, view.sh, view.shStride, PartLabels{}, first, v << 16,
-                         indexOf);
-    const uint2 at = compactTile(s, a.status, item, a.epoch, a.error, a.keys, a.projected, a.spans,
-                                 static_cast<float>(view.width), static_cast<float>(view.height), view.binsX,
-                                 view.binsY);
-    if (threadIdx.x == 0) {
-      if (chunk == 0) a.viewFirst[v] = at.x;
-      if (item == a.items - 1) {
-        a.viewFirst[a.viewCount] = at.x + at.y;
-        *a.visibleCount = at.x + at.y;
+        index = 0xffffffffu;
       }
     }
+    projectTile<D, true>(t, cam, w.splats, w.sh, w.shStride, PartLabels{}, index, viewIndex[b] << 16);
   }
+  __device__ __forceinline__ float width(uint32_t b) const { return static_cast<float>(view[b].width); }
+  __device__ __forceinline__ float height(uint32_t b) const { return static_cast<float>(view[b].height); }
+  __device__ __forceinline__ uint32_t binsX(uint32_t b) const { return view[b].binsX; }
+  __device__ __forceinline__ uint32_t binsY(uint32_t b) const { return view[b].binsY; }
+  __device__ __forceinline__ void finish(uint32_t item, uint32_t b, uint32_t before, uint32_t count) {
+    if (item == view[b].itemStart) a.viewFirst[viewIndex[b]] = before;
+    if (item == a.items - 1) {
+      a.viewFirst[a.viewCount] = before + count;
+      *a.visibleCount = before + count;
+    }
+  }
+};
+
+template <int D>
+__global__ void __launch_bounds__(kThreads, 4)
+    visibilityBatchKernel(const __grid_constant__ BatchVisibilityArgs a) {
+  __shared__ VisibilitySmem s;
+  __shared__ Camera cam;
+  __shared__ BatchView view[2];
+  __shared__ uint32_t viewIndex[2];
+  fillBlockTables();
+  const uint32_t item = takeTile(a.counters);
+  chainedKernelStart();
+  BatchSource<D> source{a, cam, view, viewIndex};
+  if (item < a.items) source.enter(item, 0);
+  __syncthreads();
+  runTiles(s, source, VisibilityOut{a.keys, a.projected, a.spans, a.status, a.counters, a.epoch, a.error}, item, a.items,
+           nullptr, 0u);
   finishTile(a.counters);
 }
 
-
-// 1M splats at 1080p take 80 us whatever the arithmetic costs (78 without the harmonics' evaluation, 82
-// with approximate divisions): a third of the warps' time is the compaction's barriers, where a tile waits
-// for the counts of the tiles before it, all projected at the same time. A batch of many waves is bound by
-// instructions (569 us for 12M splats, 476 without the harmonics): the opacity's quad radius from a table,
-// saturating half conversions and the cells worked out during the look-back took it from 604 us.
-//
-// 256-splat tiles while the chip holds all their blocks at once (four per SM): the pass then lasts as
-// long as one tile, and a quarter of the rows end it sooner (4k splats 15.5 -> 9.0 us, 30k 21.4 -> 12.9, 100k
-// 21.2 -> 18.3); 1024-splat tiles beyond, where the tables, the look-back and the copy-out per block count
-// for more (1M splats 80 us, 86 with 512-splat tiles).
-constexpr uint32_t kSmallTotal = 4 * 148 * kThreads;
-
 template <int D, bool kKey16, bool kIndexed>
 void launchOne(const VisibilityArgs& a, cudaStream_t stream) {
-  auto blocks = [&](uint32_t tile) { return max(1u, (a.total + tile - 1) / tile); };
-  if (a.total <= kSmallTotal) {
-    launchChained(visibilityKernel<D, kKey16, kIndexed, 1>, blocks(kThreads), kThreads, stream, a);
-  } else {
-    launchChained(visibilityKernel<D, kKey16, kIndexed, kItems>, blocks(kTileSplats), kThreads, stream, a);
-  }
+  const uint32_t tiles = max(1u, (a.total + kTileSplats - 1) / kTileSplats);
+  launchChained(visibilityKernel<D, kKey16, kIndexed>, min(tiles, kResidentBlocks), kThreads, stream, a);
 }
 
 template <int D>
@@ -584,18 +612,15 @@ void launchDegree(const VisibilityArgs& a, bool key16, bool indexed, cudaStream_
 
 uint32_t visibilityTileSplats() { return kTileSplats; }
 
-uint32_t visibilityTiles(uint32_t total) {
-  return (total + kTileSplats - 1) / kTileSplats + kSmallTotal / kThreads;
-}
-
 cudaError_t launchVisibilityBatch(const BatchVisibilityArgs& args, int shDegree,
                                   cudaStream_t stream) {
   if (args.items == 0 || args.viewCount == 0) return cudaSuccess;
+  const uint32_t blocks = min(args.items, kResidentBlocks);
   switch (shDegree) {
-    case 0: launchChained(visibilityBatchKernel<0>, args.items, kThreads, stream, args); break;
-    case 1: launchChained(visibilityBatchKernel<1>, args.items, kThreads, stream, args); break;
-    case 2: launchChained(visibilityBatchKernel<2>, args.items, kThreads, stream, args); break;
-    default: launchChained(visibilityBatchKernel<3>, args.items, kThreads, stream, args); break;
+    case 0: launchChained(visibilityBatchKernel<0>, blocks, kThreads, stream, args); break;
+    case 1: launchChained(visibilityBatchKernel<1>, blocks, kThreads, stream, args); break;
+    case 2: launchChained(visibilityBatchKernel<2>, blocks, kThreads, stream, args); break;
+    default: launchChained(visibilityBatchKernel<3>, blocks, kThreads, stream, args); break;
   }
   return cudaGetLastError();
 }

@@ -148,7 +148,7 @@ sk_status Context::reserveScratch(FrameScratch& f, uint32_t sources, uint32_t in
   auto grab = [&](DeviceBuffer& b, size_t n) {
     if (e == cudaSuccess) e = b.allocate(n);
   };
-  const uint32_t visTiles = visibilityTiles(sources);
+  const uint32_t visTiles = (sources + visibilityTileSplats() - 1) / visibilityTileSplats();
   grab(f.keys, size_t{sources} * 4);
   grab(f.projected, size_t{sources} * sizeof(Projected));
   grab(f.spans, size_t{sources} * 16);

@@ -1,6 +1,6 @@
-"""The cull at the edges of its tiles (256 splats up to 151,552 records, 1024 beyond), against the
-oracle: survivors, keys and records bit for bit, for record counts around a tile and around the change
-of tile, opacities over the whole 8-bit range, merged opacities above 1 and colours that saturate binary16."""
+"""The cull at the edges of its tiles (256 splats; beyond 592 tiles a block takes several), against the
+oracle: survivors, keys and records bit for bit, for record counts around a tile and around 592 of
+them, opacities over the whole 8-bit range, merged opacities above 1 and colours that saturate binary16."""
 from __future__ import annotations
 
 import math
