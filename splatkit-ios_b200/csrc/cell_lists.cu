@@ -45,9 +45,13 @@ namespace {
 constexpr uint32_t kThreads = 256;
 constexpr uint32_t kWarps = kThreads / 32;
 // Depth ranks per lane: count and emission blocks take 512 depth ranks (1024: a frame's emission 32 ->
-// 50 us, the 24-view batch's 228 -> 262; 256: twice the rows to scan).
-constexpr uint32_t kItems = 2;
-constexpr uint32_t kBlockRanks = kThreads * kItems;
+// 50 us, the 24-view batch's 228 -> 262). Up to 151,552 ranks, where all blocks of 256 ranks are on the chip
+// at once and a pass lasts as long as one block, they take 256: 100k splats at 720p emit in 11 us against
+// 16, the frame 213.6 against 217.1; a thumbnail's frame 62.7 against 65.0. Above, 512 ranks halve the
+// rows to scan.
+constexpr uint32_t kMostItems = 2;
+constexpr uint32_t kFewRanks = 148 * 4 * kThreads;
+
 constexpr uint32_t kScanThreads = 512;
 constexpr uint32_t kGroup = 8;                              // patches per scan block
 constexpr uint32_t kScanLanes = kScanThreads / kGroup;      // row lanes per patch
@@ -78,9 +82,11 @@ struct Job {
 __host__ __device__ inline uint32_t counterWords(uint32_t patches) { return (patches + 1) / 2; }
 __host__ __device__ inline size_t align16(size_t n) { return (n + 15) & ~size_t{15}; }
 __host__ __device__ inline uint32_t groupsOf(uint32_t patches) { return (patches + kGroup - 1) / kGroup; }
-__host__ __device__ inline uint32_t blocksOf(uint32_t capacity) {
-  return (capacity + kBlockRanks - 1) / kBlockRanks;
+__host__ __device__ inline uint32_t blocksOf(uint32_t capacity, uint32_t items) {
+  return (capacity + kThreads * items - 1) / (kThreads * items);
 }
+// A frame's ranks per lane.
+inline uint32_t itemsFor(uint32_t capacity) { return capacity <= kFewRanks ? 1u : kMostItems; }
 
 // The job of block (or patch group, byGroup) `index` of a pass.
 __device__ __forceinline__ Job jobOf(const BinArgs& a, const Work& w, uint32_t patches,
@@ -167,8 +173,10 @@ __device__ __forceinline__ void visitPatches(const uint4 s, uint32_t shift, uint
 }
 
 // Pass 1: each block's entries per patch; the (survivor, cell) pairs are added up beside them.
+template <uint32_t kItems>
 __global__ void __launch_bounds__(kThreads)
     patchCountKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches) {
+  constexpr uint32_t kBlockRanks = kThreads * kItems;
   chainedKernelStart();
   extern __shared__ uint32_t hist[];
   __shared__ uint32_t warpPairs[kWarps];
@@ -212,6 +220,7 @@ __global__ void __launch_bounds__(kThreads)
 // waits on groups already running). Thread t is row lane t / 8 of the group's patch t % 8: it sums
 // a contiguous share of the block rows, the first 16 of them kept in registers between the two
 // sweeps (a warp reads four rows' 32-byte sectors at a time).
+template <uint32_t kItems>
 __global__ void __launch_bounds__(kScanThreads)
     patchScanKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches, uint2* ranges,
                     uint32_t* entryCount, uint32_t* counters, uint32_t epoch, uint32_t* error) {
@@ -221,7 +230,7 @@ __global__ void __launch_bounds__(kScanThreads)
   const uint32_t group = takeTile(counters);  // over all views of a batch
   const Job job = jobOf(a, work, patches, group, true, ranges);
   patches = job.patches;
-  const uint32_t active = blocksOf(job.n);
+  const uint32_t active = blocksOf(job.n, kItems);
   const uint32_t warp = threadIdx.x >> 5, lane = laneId();
   const uint32_t c = threadIdx.x % kGroup, rowLane = threadIdx.x / kGroup;
   const uint32_t patch = job.block * kGroup + c;
@@ -322,13 +331,15 @@ __global__ void __launch_bounds__(kScanThreads)
 }
 
 // Pass 3. Dynamic shared memory: kWarps x words per-warp slot counters (16-bit halves: a warp's
-// slots count from the block's first slot in the patch, at most kBlockRanks on), then each patch's
+// slots count from the block's first slot in the patch, at most the block's ranks on), then each patch's
 // first slot for the block. A warp's entries, in depth order, are worked out kWindow positions at a
 // time, one position per lane and step (however many patches the items have), and staged as
 // (patch, item, cell mask); a warp of more entries works each further window out when it writes it.
 
+template <uint32_t kItems>
 __global__ void __launch_bounds__(kThreads)
     patchEmitKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches) {
+  constexpr uint32_t kBlockRanks = kThreads * kItems;
   constexpr uint32_t kChunk = 32 * kItems;  // ranks per warp
   constexpr uint32_t kWindow = 4 * kChunk;  // positions staged at a time
   static_assert(kChunk < 256, "an item and a marker are bytes");
@@ -519,7 +530,7 @@ size_t countDynamicBytes(uint32_t patches) { return size_t{patches} * sizeof(uin
 
 bool patchListsFit(uint32_t patches) { return patches > 0 && patches <= kDirectMaxPatches; }
 
-uint32_t patchListBlocks(uint32_t capacity) { return blocksOf(std::max(capacity, 1u)); }
+uint32_t patchListBlocks(uint32_t capacity) { return blocksOf(std::max(capacity, 1u), kMostItems); }
 
 uint32_t patchListGroups(uint32_t patches) { return groupsOf(patches); }
 
@@ -528,7 +539,7 @@ size_t patchListRowBytes(uint32_t capacity, uint32_t patches) {
 }
 
 size_t patchListBytes(uint32_t capacity, uint32_t patches) {
-  return kStatusBytes + patchListRowBytes(capacity, std::max(patches, 1u));
+  return kStatusBytes + align16(size_t{blocksOf(std::max(capacity, 1u), itemsFor(capacity))} * std::max(patches, 1u) * 4);
 }
 
 size_t patchListStatusBytes() { return kStatusBytes; }
@@ -536,33 +547,39 @@ size_t patchListStatusBytes() { return kStatusBytes; }
 cudaError_t patchListsConfigure() {
   static std::atomic<uint64_t> done{0};
   return oncePerDevice(done, [] {
-    return cudaFuncSetAttribute(patchEmitKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(emitDynamicBytes(kDirectMaxPatches)));
+    const int most = static_cast<int>(emitDynamicBytes(kDirectMaxPatches));
+    const cudaError_t e =
+        cudaFuncSetAttribute(patchEmitKernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    return e != cudaSuccess
+               ? e
+               : cudaFuncSetAttribute(patchEmitKernel<kMostItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   });
 }
 
+template <uint32_t kRanks>
 static cudaError_t launchPasses(const BinArgs& a, const Work& work, uint32_t patches, uint32_t blocks,
                                 uint32_t groups, uint2* ranges, uint32_t* entryCount, uint32_t* counters,
                                 uint32_t epoch, uint32_t* error, cudaStream_t stream) {
   cudaError_t e = patchListsConfigure();
   if (e == cudaSuccess)
-    e = launchChainedShared(patchCountKernel, blocks, kThreads, countDynamicBytes(patches), stream, a,
+    e = launchChainedShared(patchCountKernel<kRanks>, blocks, kThreads, countDynamicBytes(patches), stream, a,
                             work, patches);
   if (e == cudaSuccess)
-    e = launchChained(patchScanKernel, groups, kScanThreads, stream, a, work, patches, ranges,
+    e = launchChained(patchScanKernel<kRanks>, groups, kScanThreads, stream, a, work, patches, ranges,
                       entryCount, counters, epoch, error);
   if (e == cudaSuccess)
-    e = launchChainedShared(patchEmitKernel, blocks, kThreads, emitDynamicBytes(patches), stream, a,
+    e = launchChainedShared(patchEmitKernel<kRanks>, blocks, kThreads, emitDynamicBytes(patches), stream, a,
                             work, patches);
   return e;
 }
 
 cudaError_t launchPatchLists(const BinArgs& a, const PatchLists& lists, cudaStream_t stream) {
   const PatchGrid g = patchGrid(a.tilesX, a.tilesY);
-  const uint32_t patches = g.x * g.y;
+  const uint32_t patches = g.x * g.y, items = itemsFor(a.capacity);
   if (!patchListsFit(patches) || a.capacity == 0) return cudaErrorInvalidValue;
-  return launchPasses(a, workOf(lists.workspace), patches, blocksOf(a.capacity),
-                                   groupsOf(patches), lists.ranges, lists.entryCount, lists.counters, lists.epoch, lists.error, stream);
+  const auto launch = items == 1 ? launchPasses<1> : launchPasses<kMostItems>;
+  return launch(a, workOf(lists.workspace), patches, blocksOf(a.capacity, items), groupsOf(patches), lists.ranges,
+                lists.entryCount, lists.counters, lists.epoch, lists.error, stream);
 }
 
 cudaError_t launchPatchListsBatch(const BinArgs& a, const PatchListBatch& lists, cudaStream_t stream) {
@@ -575,7 +592,7 @@ cudaError_t launchPatchListsBatch(const BinArgs& a, const PatchListBatch& lists,
   work.viewFirst = lists.viewFirst;
   work.base = static_cast<uint8_t*>(lists.workspace);
   // each block reads its own view's patches from the table
-  return launchPasses(a, work, lists.mostPatches, lists.blocks, lists.groups, lists.ranges, lists.entryCount,
+  return launchPasses<kMostItems>(a, work, lists.mostPatches, lists.blocks, lists.groups, lists.ranges, lists.entryCount,
                       lists.counters, lists.epoch, lists.error, stream);
 }
 

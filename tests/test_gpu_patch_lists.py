@@ -46,3 +46,16 @@ def test_direct_frames_equal_the_sorted_frames(cuda_device, n, w, h, log_scale):
                                                   draw(cloud, frames, w, h, "sorted")):
         assert (va, pa, ra) == (vb, pb, rb)
         assert np.array_equal(ia, ib)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [255, 256, 257, 512, 513, 151_552, 151_553, 152_065])
+def test_direct_frames_at_the_edges_of_a_blocks_ranks(cuda_device, n):
+    """Count and emission blocks of 256 ranks up to 151,552 sources, of 512 above."""
+    w, h = 500, 400
+    cloud = synthetic.random_cloud(n, seed=23, sh_degree=0, log_scale_mean=-3.5)
+    frames = frames_for(cloud, w, h, (11,))
+    for (ia, va, pa, ra), (ib, vb, pb, rb) in zip(draw(cloud, frames, w, h, "auto"),
+                                                  draw(cloud, frames, w, h, "sorted")):
+        assert (va, pa, ra) == (vb, pb, rb)
+        assert np.array_equal(ia, ib)
