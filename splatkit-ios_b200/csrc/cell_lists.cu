@@ -44,12 +44,14 @@ namespace {
 
 constexpr uint32_t kThreads = 256;
 constexpr uint32_t kWarps = kThreads / 32;
-// Depth ranks per lane: count and emission blocks take 512 depth ranks (1024: a frame's emission 32 ->
-// 50 us, the 24-view batch's 228 -> 262). Up to 151,552 ranks, where all blocks of 256 ranks are on the chip
-// at once and a pass lasts as long as one block, they take 256: 100k splats at 720p emit in 11 us against
-// 16, the frame 213.6 against 217.1; a thumbnail's frame 62.7 against 65.0. Above, 512 ranks halve the
-// rows to scan.
+// Depth ranks per lane. A frame's count and emission blocks take 512 depth ranks (1024: emission 32 -> 50
+// us at 1M). Up to 151,552 ranks, where all blocks of 256 ranks are on the chip at once and a pass lasts as
+// long as one block, they take 256: 100k splats at 720p emit in 11 us against 16, the frame 213.6 against
+// 217.1; a thumbnail's frame 62.7 against 65.0. Above, 512 ranks halve the rows to scan. A batch whose
+// patches are all single cells takes 1024, whose spans then stay in registers (24 views of up to 640 x
+// 480: count, scan and emission 80, 23 and 205 us; at 512 ranks 88, 25 and 211); with larger patches 512.
 constexpr uint32_t kMostItems = 2;
+constexpr uint32_t kCellItems = 4;
 constexpr uint32_t kFewRanks = 148 * 4 * kThreads;
 
 constexpr uint32_t kScanThreads = 512;
@@ -330,6 +332,158 @@ __global__ void __launch_bounds__(kScanThreads)
   finishTile(counters);
 }
 
+// One round of a warp's output: lanes with an entry (valid) write it at their patch's next slots in lane
+// order. Lanes with the same patch take consecutive slots (a match instruction finds them: one ballot per bit
+// of a patch index took 216 us of the 24-view batch's emission against 205, 33.7 of a 1M frame's against 32.5).
+__device__ __forceinline__ void writeRound(const BinArgs& a, const uint32_t* where, uint32_t* mine, bool valid,
+                                           uint32_t patch, uint32_t value, uint32_t mask) {
+  const uint32_t peers = __match_any_sync(0xffffffffu, valid ? patch : 0xffffffffu);
+  const uint32_t half = (patch & 1u) * 16;
+  uint32_t slot = 0;
+  if (valid) slot = where[patch] + ((mine[patch >> 1] >> half) & 0xffffu) + __popc(peers & lanemaskLt());
+  __syncwarp();
+  if (valid && laneId() == 31 - __clz(peers)) atomicAdd(mine + (patch >> 1), __popc(peers) << half);
+  __syncwarp();
+  if (valid && slot < a.instanceCapacity) {
+    a.instanceValues[slot] = value;
+    if (a.instanceMasks) a.instanceMasks[slot] = static_cast<uint16_t>(mask);
+  }
+}
+
+// Zeroes the block's slot counters and fetches its first slots.
+__device__ __forceinline__ void emitSetup(const Job& job, uint32_t* slots, uint32_t* where, uint32_t words) {
+  for (uint32_t i = threadIdx.x; i < kWarps * words; i += kThreads) slots[i] = 0;
+  const uint32_t* starts = job.blockRows + size_t{job.block} * job.patches;
+  for (uint32_t c = threadIdx.x; c < job.patches; c += kThreads) where[c] = __ldcg(starts + c);
+}
+
+// Warp w's first slot per patch: the counts of warps 0..w-1 (both halves of a word at once).
+__device__ __forceinline__ void slotsFromCounts(uint32_t* slots, uint32_t words) {
+  for (uint32_t q = threadIdx.x; q < words; q += kThreads) {
+    uint32_t run = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; ++w) {
+      const uint32_t v = slots[w * words + q];
+      slots[w * words + q] = run;
+      run += v;
+    }
+  }
+}
+
+// Pass 3 where every patch is one cell. The warp's spans stay in registers, and a masked span's cells are
+// staged by the lane that has it (a box of more than 64 cells by the whole warp): most splats of such
+// targets list one or two cells, so that the walk costs less than finding each position's span does (24 views
+// of up to 640 x 480: emission 265 -> 216 us against patchEmitKernel).
+template <uint32_t kItems>
+__global__ void __launch_bounds__(kThreads)
+    cellEmitKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches) {
+  constexpr uint32_t kBlockRanks = kThreads * kItems;
+  constexpr uint32_t kChunk = 32 * kItems;  // ranks per warp
+  constexpr uint32_t kWindow = 8 * kChunk;  // positions staged at a time
+  static_assert(kChunk <= 256, "an item is a byte");
+  chainedKernelStart();
+  extern __shared__ uint32_t patchSmem[];
+  __shared__ uint32_t itemValue[kWarps][kChunk];
+  __shared__ uint16_t stageCell[kWarps][kWindow];
+  __shared__ uint8_t stageItem[kWarps][kWindow];
+  const Job job = jobOf(a, work, patches, blockIdx.x, false, nullptr);
+  const uint32_t n = job.n, cellsX = job.patchesX;
+  const uint32_t* order = a.order + job.first;
+  const uint32_t begin = job.block * kBlockRanks;
+  if (begin >= n) return;
+  const uint32_t warp = threadIdx.x >> 5, lane = laneId();
+  uint32_t value[kItems], offset[kItems];
+  uint4 span[kItems];
+#pragma unroll
+  for (uint32_t r = 0; r < kItems; ++r) {
+    const uint32_t i = begin + warp * kChunk + r * 32 + lane;
+    value[r] = i < n ? order[i] : 0xffffffffu;
+  }
+  const uint32_t words = counterWords(job.patches);
+  uint32_t* slots = patchSmem;
+  uint32_t* where = patchSmem + kWarps * words;
+  emitSetup(job, slots, where, words);
+  uint32_t* mine = slots + warp * words;
+  uint16_t* sCell = stageCell[warp];
+  uint8_t* sItem = stageItem[warp];
+  // the warp's items in (row, lane) order = depth order, with their first output position
+  uint32_t total = 0;
+#pragma unroll
+  for (uint32_t r = 0; r < kItems; ++r) {
+    span[r] = value[r] != 0xffffffffu ? __ldg(a.spans + value[r]) : make_uint4(0, 0, 0, 0);
+    itemValue[warp][r * 32 + lane] = value[r];
+  }
+#pragma unroll
+  for (uint32_t r = 0; r < kItems; ++r) {
+    const uint32_t cnt = spanCount(span[r]);
+    uint32_t inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t up = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= static_cast<uint32_t>(o)) inc += up;
+    }
+    offset[r] = total + inc - cnt;
+    total += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  __syncthreads();  // the counters are zero, the starts there
+
+  // put(cell, position, item) for every entry at a position of [lo, hi)
+  auto walk = [&](uint32_t lo, uint32_t hi, auto put) {
+#pragma unroll
+    for (uint32_t r = 0; r < kItems; ++r) {
+      const uint32_t w = span[r].y & 0xffffu, area = spanArea(span[r]), item = r * 32 + lane;
+      const uint32_t first = (span[r].x >> 16) * cellsX + (span[r].x & 0xffffu);
+      uint32_t pos = offset[r];
+      if (area <= 64 && pos < hi)
+        visitListed(span[r], first, cellsX, [&](uint32_t cell) {
+          if (pos >= lo && pos < hi) put(cell, pos, item);
+          ++pos;
+        });
+      uint32_t big = __ballot_sync(0xffffffffu, area > 64 && offset[r] < hi && offset[r] + area > lo);
+      while (big != 0u) {
+        const uint32_t src = __ffs(big) - 1;
+        big &= big - 1;
+        const uint32_t bw = __shfl_sync(0xffffffffu, w, src), cells = __shfl_sync(0xffffffffu, area, src);
+        const uint32_t at = __shfl_sync(0xffffffffu, first, src), from = __shfl_sync(0xffffffffu, offset[r], src);
+        const uint32_t k0 = lo > from ? lo - from : 0u, k1 = min(cells, hi - from);
+        for (uint32_t k = k0 + lane; k < k1; k += 32) put(boxCell(at, k, bw, cellsX), from + k, r * 32 + src);
+      }
+    }
+  };
+  // every entry counted by cell, the first window staged
+  walk(0u, 0xffffffffu, [&](uint32_t cell, uint32_t pos, uint32_t item) {
+    atomicAdd(mine + (cell >> 1), 1u << ((cell & 1u) * 16));
+    if (pos < kWindow) {
+      sCell[pos] = static_cast<uint16_t>(cell);
+      sItem[pos] = static_cast<uint8_t>(item);
+    }
+  });
+  __syncthreads();
+  slotsFromCounts(slots, words);
+  __syncthreads();
+  for (uint32_t w0 = 0; w0 < total; w0 += kWindow) {
+    const uint32_t w1 = min(total, w0 + kWindow);
+    if (w0 > 0) {
+      __syncwarp();
+      walk(w0, w1, [&](uint32_t cell, uint32_t pos, uint32_t item) {
+        sCell[pos - w0] = static_cast<uint16_t>(cell);
+        sItem[pos - w0] = static_cast<uint8_t>(item);
+      });
+    }
+    __syncwarp();
+    for (uint32_t p0 = w0; p0 < w1; p0 += 32) {
+      const uint32_t p = p0 + lane;
+      const bool valid = p < w1;
+      uint32_t cell = 0, val = 0;
+      if (valid) {
+        cell = sCell[p - w0];
+        val = itemValue[warp][sItem[p - w0]];
+      }
+      writeRound(a, where, mine, valid, cell, val, 1u);
+    }
+  }
+}
+
 // Pass 3. Dynamic shared memory: kWarps x words per-warp slot counters (16-bit halves: a warp's
 // slots count from the block's first slot in the patch, at most the block's ranks on), then each patch's
 // first slot for the block. A warp's entries, in depth order, are worked out kWindow positions at a
@@ -365,10 +519,7 @@ __global__ void __launch_bounds__(kThreads)
   const uint32_t words = counterWords(patches);
   uint32_t* slots = patchSmem;
   uint32_t* where = patchSmem + kWarps * words;
-  for (uint32_t i = threadIdx.x; i < kWarps * words; i += kThreads) slots[i] = 0;
-  const uint32_t* starts = job.blockRows + size_t{job.block} * patches;
-  for (uint32_t c = threadIdx.x; c < patches; c += kThreads) where[c] = __ldcg(starts + c);
-
+  emitSetup(job, slots, where, words);
   uint32_t* mine = slots + warp * words;
   uint16_t* sPatch = stagePatch[warp];
   uint16_t* sMask = stageMask[warp];
@@ -394,8 +545,8 @@ __global__ void __launch_bounds__(kThreads)
   }
   __syncthreads();  // the counters are zero, the starts there
 
-  // Stages the entries at positions [w0, w1). Single-cell patches: every lane walks its items' listed
-  // cells (most items have one or two; a box of more than 64 cells is walked by the whole warp).
+  // Stages the entries at positions [w0, w1). Single-cell patches (a batch's small targets beside larger
+  // ones): every lane walks its items' listed cells (most items have one or two; a box of more than 64 cells is walked by the whole warp).
   // Larger patches: one position per lane and step; every item marks its first position, and an
   // entry's item is the last mark at or before its position (a running maximum).
   auto stageWindow = [&](uint32_t w0, uint32_t w1, uint32_t& carry, bool count) {
@@ -466,20 +617,9 @@ __global__ void __launch_bounds__(kThreads)
   for (uint32_t w0 = 0, carry = 0; w0 < total; w0 += kWindow)
     stageWindow(w0, min(total, w0 + kWindow), carry, true);
   __syncthreads();
-  // warp w's first slot per patch: the counts of warps 0..w-1 (both halves of a word at once)
-  for (uint32_t q = threadIdx.x; q < words; q += kThreads) {
-    uint32_t run = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kWarps; ++w) {
-      const uint32_t v = slots[w * words + q];
-      slots[w * words + q] = run;
-      run += v;
-    }
-  }
+  slotsFromCounts(slots, words);
   __syncthreads();
 
-  const uint32_t below = lanemaskLt();
-  const uint32_t bits = 32 - __clz(max(patches, 2u) - 1);  // of a patch index: at most 12
   for (uint32_t w0 = 0, carry = 0; w0 < total; w0 += kWindow) {
     const uint32_t w1 = min(total, w0 + kWindow);
     if (total > kWindow) {
@@ -496,26 +636,7 @@ __global__ void __launch_bounds__(kThreads)
         mask = sMask[p - w0];
         val = itemValue[warp][sItem[p - w0]];
       }
-      // lanes of this round with the same patch: one ballot per bit of a patch index
-      uint32_t peers = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-      for (uint32_t b = 0; b < 12; ++b) {
-        if (b < bits) {
-          const bool bit = (patch >> b) & 1u;
-          const uint32_t vote = __ballot_sync(0xffffffffu, bit);
-          peers &= bit ? vote : ~vote;
-        }
-      }
-      const uint32_t half = (patch & 1u) * 16;
-      uint32_t slot = 0;
-      if (valid) slot = where[patch] + ((mine[patch >> 1] >> half) & 0xffffu) + __popc(peers & below);
-      __syncwarp();
-      if (valid && lane == 31 - __clz(peers)) atomicAdd(mine + (patch >> 1), __popc(peers) << half);
-      __syncwarp();
-      if (valid && slot < a.instanceCapacity) {
-        a.instanceValues[slot] = val;
-        if (a.instanceMasks) a.instanceMasks[slot] = static_cast<uint16_t>(mask);
-      }
+      writeRound(a, where, mine, valid, patch, val, mask);
     }
   }
 }
@@ -530,12 +651,14 @@ size_t countDynamicBytes(uint32_t patches) { return size_t{patches} * sizeof(uin
 
 bool patchListsFit(uint32_t patches) { return patches > 0 && patches <= kDirectMaxPatches; }
 
-uint32_t patchListBlocks(uint32_t capacity) { return blocksOf(std::max(capacity, 1u), kMostItems); }
+uint32_t patchListBlocks(uint32_t capacity, bool cells) {
+  return blocksOf(std::max(capacity, 1u), cells ? kCellItems : kMostItems);
+}
 
 uint32_t patchListGroups(uint32_t patches) { return groupsOf(patches); }
 
-size_t patchListRowBytes(uint32_t capacity, uint32_t patches) {
-  return align16(size_t{patchListBlocks(capacity)} * patches * 4);
+size_t patchListRowBytes(uint32_t capacity, uint32_t patches, bool cells) {
+  return align16(size_t{patchListBlocks(capacity, cells)} * patches * 4);
 }
 
 size_t patchListBytes(uint32_t capacity, uint32_t patches) {
@@ -544,42 +667,50 @@ size_t patchListBytes(uint32_t capacity, uint32_t patches) {
 
 size_t patchListStatusBytes() { return kStatusBytes; }
 
+namespace {
+
+cudaError_t launchPasses(uint32_t items, bool cells, const BinArgs& a, const Work& work, uint32_t patches,
+                         uint32_t blocks, uint32_t groups, uint2* ranges, uint32_t* entryCount, uint32_t* counters,
+                         uint32_t epoch, uint32_t* error, cudaStream_t stream) {
+  const auto count = items == 1 ? patchCountKernel<1> : items == 2 ? patchCountKernel<2> : patchCountKernel<4>;
+  const auto scan = items == 1 ? patchScanKernel<1> : items == 2 ? patchScanKernel<2> : patchScanKernel<4>;
+  const auto emit = !cells       ? items == 1 ? patchEmitKernel<1> : patchEmitKernel<2>
+                    : items == 1 ? cellEmitKernel<1>
+                    : items == 2 ? cellEmitKernel<2>
+                                 : cellEmitKernel<4>;
+  cudaError_t e = patchListsConfigure();
+  if (e == cudaSuccess)
+    e = launchChainedShared(count, blocks, kThreads, countDynamicBytes(patches), stream, a, work, patches);
+  if (e == cudaSuccess)
+    e = launchChained(scan, groups, kScanThreads, stream, a, work, patches, ranges, entryCount, counters, epoch,
+                      error);
+  if (e == cudaSuccess)
+    e = launchChainedShared(emit, blocks, kThreads, emitDynamicBytes(patches), stream, a, work, patches);
+  return e;
+}
+
+}  // namespace
+
 cudaError_t patchListsConfigure() {
   static std::atomic<uint64_t> done{0};
   return oncePerDevice(done, [] {
+    // targets of single-cell patches have at most kPatchGoal of them: within the default limit
     const int most = static_cast<int>(emitDynamicBytes(kDirectMaxPatches));
     const cudaError_t e =
         cudaFuncSetAttribute(patchEmitKernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     return e != cudaSuccess
                ? e
-               : cudaFuncSetAttribute(patchEmitKernel<kMostItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+               : cudaFuncSetAttribute(patchEmitKernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   });
-}
-
-template <uint32_t kRanks>
-static cudaError_t launchPasses(const BinArgs& a, const Work& work, uint32_t patches, uint32_t blocks,
-                                uint32_t groups, uint2* ranges, uint32_t* entryCount, uint32_t* counters,
-                                uint32_t epoch, uint32_t* error, cudaStream_t stream) {
-  cudaError_t e = patchListsConfigure();
-  if (e == cudaSuccess)
-    e = launchChainedShared(patchCountKernel<kRanks>, blocks, kThreads, countDynamicBytes(patches), stream, a,
-                            work, patches);
-  if (e == cudaSuccess)
-    e = launchChained(patchScanKernel<kRanks>, groups, kScanThreads, stream, a, work, patches, ranges,
-                      entryCount, counters, epoch, error);
-  if (e == cudaSuccess)
-    e = launchChainedShared(patchEmitKernel<kRanks>, blocks, kThreads, emitDynamicBytes(patches), stream, a,
-                            work, patches);
-  return e;
 }
 
 cudaError_t launchPatchLists(const BinArgs& a, const PatchLists& lists, cudaStream_t stream) {
   const PatchGrid g = patchGrid(a.tilesX, a.tilesY);
   const uint32_t patches = g.x * g.y, items = itemsFor(a.capacity);
   if (!patchListsFit(patches) || a.capacity == 0) return cudaErrorInvalidValue;
-  const auto launch = items == 1 ? launchPasses<1> : launchPasses<kMostItems>;
-  return launch(a, workOf(lists.workspace), patches, blocksOf(a.capacity, items), groupsOf(patches), lists.ranges,
-                lists.entryCount, lists.counters, lists.epoch, lists.error, stream);
+  return launchPasses(items, g.shift == 0, a, workOf(lists.workspace), patches, blocksOf(a.capacity, items),
+                      groupsOf(patches), lists.ranges, lists.entryCount, lists.counters, lists.epoch, lists.error,
+                      stream);
 }
 
 cudaError_t launchPatchListsBatch(const BinArgs& a, const PatchListBatch& lists, cudaStream_t stream) {
@@ -592,8 +723,8 @@ cudaError_t launchPatchListsBatch(const BinArgs& a, const PatchListBatch& lists,
   work.viewFirst = lists.viewFirst;
   work.base = static_cast<uint8_t*>(lists.workspace);
   // each block reads its own view's patches from the table
-  return launchPasses<kMostItems>(a, work, lists.mostPatches, lists.blocks, lists.groups, lists.ranges, lists.entryCount,
-                      lists.counters, lists.epoch, lists.error, stream);
+  return launchPasses(lists.cells ? kCellItems : kMostItems, lists.cells, a, work, lists.mostPatches, lists.blocks,
+                      lists.groups, lists.ranges, lists.entryCount, lists.counters, lists.epoch, lists.error, stream);
 }
 
 }  // namespace sk

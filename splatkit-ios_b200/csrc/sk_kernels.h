@@ -174,9 +174,9 @@ cudaError_t launchPatchLists(const BinArgs& args, const PatchLists& lists, cudaS
 
 // Every view of a batch in one launch per pass. View v's ranks are [viewFirst[v], viewFirst[v+1])
 // of args.order (at most `capacity` of them), its patches patchBase .. patchBase + patches of the
-// batch's ranges; its count/emit blocks are blockBase .. blockBase + patchListBlocks(capacity), its
-// patch groups groupBase .. groupBase + patchListGroups(patches), and its block rows the
-// patchListRowBytes(capacity, patches) bytes at workspace + work. The look-back runs over the
+// batch's ranges; its count/emit blocks are blockBase .. blockBase + patchListBlocks(capacity,
+// cells), its patch groups groupBase .. groupBase + patchListGroups(patches), and its block rows the
+// patchListRowBytes(capacity, patches, cells) bytes at workspace + work. The look-back runs over the
 // groups of all views in view order, so view v's entries follow those of views 0..v-1;
 // *entryCount receives the total and args.overflow whether it exceeds args.instanceCapacity.
 struct PatchListView {
@@ -196,10 +196,11 @@ struct PatchListBatch {
   uint32_t epoch;
   uint32_t* error;
   uint32_t blocks, groups, mostPatches;  // totals over the views; the largest view's patches
+  bool cells;                            // every view's patches are single cells
 };
-uint32_t patchListBlocks(uint32_t capacity);
+uint32_t patchListBlocks(uint32_t capacity, bool cells);
 uint32_t patchListGroups(uint32_t patches);
-size_t patchListRowBytes(uint32_t capacity, uint32_t patches);
+size_t patchListRowBytes(uint32_t capacity, uint32_t patches, bool cells);
 cudaError_t launchPatchListsBatch(const BinArgs& args, const PatchListBatch& lists, cudaStream_t stream);
 // Sets the emission kernel's shared-memory limit (once; before any stream capture).
 cudaError_t patchListsConfigure();

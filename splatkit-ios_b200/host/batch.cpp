@@ -299,6 +299,7 @@ sk_status Batch::prepare(BatchLane& l, const sk_batch_view* views, uint32_t coun
     pb = PatchListBatch{};
     pb.viewCount = count;
     pb.mostPatches = mostPatches;
+    pb.cells = !l.patchMasks;
     std::vector<PatchListView> patchViews(count);
     uint64_t rowBytes = 0;
     uint32_t patches = 0;
@@ -315,9 +316,9 @@ sk_status Batch::prepare(BatchLane& l, const sk_batch_view* views, uint32_t coun
       c.groupBase = pb.groups;
       c.work = rowBytes;
       patches += c.patches;
-      pb.blocks += patchListBlocks(c.capacity);
+      pb.blocks += patchListBlocks(c.capacity, pb.cells);
       pb.groups += patchListGroups(c.patches);
-      rowBytes += patchListRowBytes(c.capacity, c.patches);
+      rowBytes += patchListRowBytes(c.capacity, c.patches, pb.cells);
     }
     void* before[3] = {l.patchLists.ptr, l.patchStatus.ptr, l.patchViews.ptr};
     cudaError_t e = l.patchLists.allocateOn(

@@ -59,3 +59,26 @@ def test_direct_frames_at_the_edges_of_a_blocks_ranks(cuda_device, n):
                                                   draw(cloud, frames, w, h, "sorted")):
         assert (va, pa, ra) == (vb, pb, rb)
         assert np.array_equal(ia, ib)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("n,log_scale", [(31, -1.0), (1023, -2.0), (1024, 0.5), (1025, -2.5), (20_000, -1.0)])
+def test_batches_of_small_targets_equal_the_sorted_frames(cuda_device, n, log_scale, mixed):
+    """Single-cell patches of every view (blocks of 1024 ranks, boxes of more than 64 cells, several
+    windows), and beside a view of larger patches (the general emission)."""
+    sizes = [(640, 480), (33, 17), (512, 640)] + [(1280, 720)] * mixed
+    cloud = synthetic.random_cloud(n, seed=29, sh_degree=0, log_scale_mean=log_scale)
+    r = sk.Renderer(64, 64)
+    r.set_binning("sorted")
+    r.upload_world(cloud, 0)
+    frames = [frames_for(cloud, w, h, (11 + 9 * i,))[0] for i, (w, h) in enumerate(sizes)]
+    with sk.Batch(lanes=1, max_views=4) as batch:
+        t = batch.submit([sk.BatchView(r, f, w, h) for f, (w, h) in zip(frames, sizes)])
+        images = [batch.read_image(t, i) for i in range(len(sizes))]
+        assert batch.stats(t)["device_error"] == 0
+    for frame, (w, h), image in zip(frames, sizes, images):
+        r.resize(w, h)
+        r.draw(frame)
+        assert np.array_equal(image, r.read_image(sk.FORMAT_RGBA8))
+    r.close()
