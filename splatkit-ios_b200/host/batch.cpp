@@ -365,12 +365,12 @@ sk_status Batch::enqueueStages(BatchLane& l, bool clearStatus) {
     SortArgs probe{};
     sortBindWorkspaceFor(probe, l.sortWorkspace.ptr, l.sources, kMinSortTileKeys);
     if (e == cudaSuccess)
-      e = cudaMemsetAsync(probe.status, 0, sortWorkspaceBytesFor(l.sources, kMinSortTileKeys) -
-                          (reinterpret_cast<char*>(probe.status) - static_cast<char*>(l.sortWorkspace.ptr)), s);
+      e = cudaMemsetAsync(probe.counters, 0, sortWorkspaceBytesFor(l.sources, kMinSortTileKeys) -
+                          (reinterpret_cast<char*>(probe.counters) - static_cast<char*>(l.sortWorkspace.ptr)), s);
     sortBindWorkspaceFor(probe, l.tileSortWorkspace.ptr, l.instances, kMinSortTileKeys);
     if (e == cudaSuccess)
-      e = cudaMemsetAsync(probe.status, 0, sortWorkspaceBytesFor(l.instances, kMinSortTileKeys) -
-                          (reinterpret_cast<char*>(probe.status) - static_cast<char*>(l.tileSortWorkspace.ptr)), s);
+      e = cudaMemsetAsync(probe.counters, 0, sortWorkspaceBytesFor(l.instances, kMinSortTileKeys) -
+                          (reinterpret_cast<char*>(probe.counters) - static_cast<char*>(l.tileSortWorkspace.ptr)), s);
   }
   // every LOD view's cut, one view after another in the lane's selection scratch
   for (size_t k = 0; e == cudaSuccess && k < l.lodPlans.size(); ++k) {
