@@ -310,8 +310,13 @@ __device__ __forceinline__ void revealGlow(const Camera& cam, float height, uint
 }
 
 __device__ __forceinline__ uint32_t sourceIndex(const VisibilityArgs& a, uint32_t t) {
-  if (a.rangeCount == 1) return a.single.offset + t;
   // SplatVisibility.metal:30-37: the range whose start is the last one <= t.
+  if (a.rangeCount <= kInlineRanges) {
+    uint32_t shift = a.inlineShift[0];
+    for (uint32_t i = 1; i < a.rangeCount; ++i)
+      if (a.inlineStart[i] <= t) shift = a.inlineShift[i];
+    return t + shift;
+  }
   uint32_t lo = 0, hi = a.rangeCount;
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) / 2;
@@ -462,8 +467,8 @@ struct FrameSource {
   // Asks for this thread's record of the tile (and its harmonics) ahead of their loads.
   __device__ __forceinline__ void enter(uint32_t tile, uint32_t) {
     const uint32_t at = tile * kTileSplats + threadIdx.x;
-    if (at >= total || (!kIndexed && a.rangeCount != 1)) return;
-    const uint32_t index = kIndexed ? a.indices[at] : a.single.offset + at;
+    if (at >= total || (!kIndexed && a.rangeCount > kInlineRanges)) return;
+    const uint32_t index = kIndexed ? a.indices[at] : sourceIndex(a, at);
     if (index >= a.worldCount) return;
     asm volatile("prefetch.global.L2 [%0];" ::"l"(a.splats + index));
     if (D > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.sh + size_t{index} * a.shStride));

@@ -316,9 +316,9 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
   }
   if (timed) cudaEventRecord(events[1], s);
 
-  if (e == cudaSuccess && !lod && frame.range_count > 1) {
+  if (e == cudaSuccess && !lod && frame.range_count > kInlineRanges) {
     // Ranges and their starts (SplatVisibility.metal:30-37); pageable copies are staged at once.
-    // A single range travels in the kernel parameters instead.
+    // Up to kInlineRanges travel in the kernel parameters instead.
     std::vector<uint32_t> starts(frame.range_count + 1, 0);
     for (uint32_t i = 0; i < frame.range_count; ++i) starts[i + 1] = starts[i] + frame.ranges[i].count;
     e = cudaMemcpyAsync(f.rangeBuffer.ptr, frame.ranges, size_t{frame.range_count} * sizeof(Range),
@@ -339,7 +339,11 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
     v.ranges = static_cast<const Range*>(f.rangeBuffer.ptr);
     v.rangeStarts = static_cast<const uint32_t*>(f.rangeStarts.ptr);
     v.rangeCount = lod ? 0 : frame.range_count;
-    if (!lod && frame.range_count == 1) v.single = Range{frame.ranges[0].offset, frame.ranges[0].count};
+    for (uint32_t i = 0, start = 0; i < std::min(v.rangeCount, kInlineRanges); ++i) {
+      v.inlineStart[i] = start;
+      v.inlineShift[i] = frame.ranges[i].offset - start;  // modulo 2^32
+      start += frame.ranges[i].count;
+    }
     v.indices = lod ? static_cast<const uint32_t*>(f.lodIndices.ptr) : nullptr;
     v.indexCount = lod ? &fc->lod[0] : nullptr;
     v.total = lod ? world.lodCapacity : total;

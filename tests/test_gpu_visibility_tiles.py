@@ -38,3 +38,31 @@ def test_counts_around_the_tiles(cuda_device, oracle, n, degree, bits):
                                      sk.sh_device_stride(degree), degree, bits, [(0, n)], threads=8)
     assert np.array_equal(keys, okeys)
     assert projected.tobytes() == oproj.tobytes()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 2, 15, 16, 17, 40])
+def test_ranges_passed_with_the_launch_and_in_memory(cuda_device, oracle, count):
+    """Up to 16 ranges are scanned in the kernel's parameters, more are searched in memory: empty ones,
+    gaps, ranges out of order and the world's last splat."""
+    n, rng = 3001, np.random.default_rng(count)
+    cuts = np.sort(rng.integers(0, n + 1, 2 * count))
+    ranges = [(int(a), int(b - a)) for a, b in zip(cuts[::2], cuts[1::2])]
+    ranges[0] = (ranges[0][0], ranges[0][1] // 2)
+    if count > 2:
+        ranges[1] = (n, 0)
+        ranges[-1] = (n - 7, 7) if ranges[-1][1] >= 7 else (n - 1, min(ranges[-1][1], 1))
+        rng.shuffle(ranges)
+        ranges = [(int(a), int(b)) for a, b in ranges]
+    cloud = synthetic.random_cloud(n, seed=5, sh_degree=1)
+    view, eye = skcam.orbit_view(9, radius=15.0)
+    proj = skcam.perspective(math.radians(60.0), W / H, 0.05, 200.0)
+    with sk.Renderer(W, H) as r:
+        r.upload_world(cloud, 1)
+        r.draw(sk.Frame(view, proj, eye, ranges, 1))
+        keys, projected = r.read_visible()
+    cam = oracle.camera(view, proj, eye, W, H, 1.0)
+    okeys, oproj = oracle.visibility(cam, sk.pack_splats(cloud), sk.pack_sh(cloud, 1), sk.sh_device_stride(1), 1, 16,
+                                     ranges, threads=8)
+    assert np.array_equal(keys, okeys)
+    assert projected.tobytes() == oproj.tobytes()
