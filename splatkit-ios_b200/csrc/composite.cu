@@ -246,8 +246,8 @@ __device__ __forceinline__ void writePixel(const CompositeArgs& a, const Target&
   }
 }
 
-// kBatch: block b is batch-wide tile firstTile + b; its view is the last one whose first tile is at or
-// below that.
+// Block b is tile firstTile + b: of the target, or with kBatch of the batch, where its view is the last one
+// whose first tile is at or below that.
 // kCount: count blended fragments (a statistic; without it the loop saves an add per splat).
 // kPatches: the lists are per patch, each entry with its cells (else per cell).
 template <int kFormat, bool kBatch, bool kCount, bool kPatches>
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kThreads) compositeKernel(const __grid_constan
   chainedKernelStart();
   __shared__ CompositeSmem sm;
   __shared__ std::conditional_t<kPatches, FilterSmem, uint32_t> filter;
-  Target t{a.width, a.height, a.tilesX, blockIdx.x, a.binsX, 0u, 0u, 0u, a.image};
+  Target t{a.width, a.height, a.tilesX, a.firstTile + blockIdx.x, a.binsX, 0u, 0u, 0u, a.image};
   if constexpr (kPatches && !kBatch) {
     const PatchGrid g = patchGrid(a.binsX, (a.tilesY + 1) / 2);
     t.patchesX = g.x, t.patchShift = g.shift;
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(kThreads) compositeKernel(const __grid_constan
 }
 
 template <int kFormat, bool kBatch>
-cudaError_t launchKind(const CompositeArgs& a, uint32_t tiles, cudaStream_t stream) {
+cudaError_t launchKind(const CompositeArgs& a, cudaStream_t stream) {
   const bool count = a.countFragments != 0;
   void (*kernel)(CompositeArgs);
   if (a.masks) {
@@ -421,21 +421,19 @@ cudaError_t launchKind(const CompositeArgs& a, uint32_t tiles, cudaStream_t stre
   } else {
     kernel = count ? compositeKernel<kFormat, kBatch, true, false> : compositeKernel<kFormat, kBatch, false, false>;
   }
-  return launchChained(kernel, tiles, kThreads, stream, a);
+  return launchChained(kernel, a.tiles, kThreads, stream, a);
 }
 
 template <int kFormat>
-cudaError_t launchFormat(const CompositeArgs& a, uint32_t tiles, cudaStream_t stream) {
-  return a.viewCount > 0 ? launchKind<kFormat, true>(a, tiles, stream) : launchKind<kFormat, false>(a, tiles, stream);
+cudaError_t launchFormat(const CompositeArgs& a, cudaStream_t stream) {
+  return a.viewCount > 0 ? launchKind<kFormat, true>(a, stream) : launchKind<kFormat, false>(a, stream);
 }
 
 }  // namespace
 
 cudaError_t launchComposite(const CompositeArgs& a, cudaStream_t stream) {
-  const uint32_t tiles = a.viewCount > 0 ? a.batchTiles : a.tilesX * a.tilesY;
-  if (tiles == 0) return cudaSuccess;
-  const bool f32 = a.format == kRgba32f;
-  return f32 ? launchFormat<kRgba32f>(a, tiles, stream) : launchFormat<kRgba8>(a, tiles, stream);
+  if (a.tiles == 0) return cudaSuccess;
+  return a.format == kRgba32f ? launchFormat<kRgba32f>(a, stream) : launchFormat<kRgba8>(a, stream);
 }
 
 }  // namespace sk

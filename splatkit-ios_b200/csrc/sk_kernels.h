@@ -229,11 +229,11 @@ struct CompositeArgs {
   uint32_t* fragments;  // FrameCounters.fragments_lo/hi (64-bit add), when countFragments
   uint32_t countFragments;
   uint32_t* loaded;     // FrameCounters.loaded
-  // a batch (viewCount > 0): one block per batch-wide tile firstTile .. firstTile + batchTiles, image =
-  // the batch image
+  // one block per tile firstTile .. firstTile + tiles of the target, or (viewCount > 0) of a batch's tiles,
+  // view after view, with image = the batch image
+  uint32_t firstTile, tiles;
   const BatchView* views;
   uint32_t viewCount;
-  uint32_t firstTile, batchTiles;
 };
 cudaError_t launchComposite(const CompositeArgs& args, cudaStream_t stream);
 

@@ -551,7 +551,7 @@ sk_status Batch::enqueueImages(BatchLane& l) {
   auto pixelAt = [&](uint32_t v) { return v < l.viewCount ? l.table[v].pixelOffset : l.totalPixels; };
   for (size_t k = 0; k < ends.size() && e == cudaSuccess; ++k) {
     c.firstTile = tileAt(k ? ends[k - 1] : 0u);
-    c.batchTiles = tileAt(ends[k]) - c.firstTile;
+    c.tiles = tileAt(ends[k]) - c.firstTile;
     e = launchComposite(c, s);
     if (aside && e == cudaSuccess) e = cudaEventRecord(l.composited[k], s);
   }

@@ -105,6 +105,11 @@ Context::~Context() {
     for (auto& ev : sl.events)
       if (ev) cudaEventDestroy(ev);
   }
+  for (const cudaStream_t st : {bands.side, bands.copies})
+    if (st) cudaStreamDestroy(st);
+  if (bands.listed) cudaEventDestroy(bands.listed);
+  for (auto& ev : bands.drawn)
+    if (ev) cudaEventDestroy(ev);
   if (stream) cudaStreamDestroy(stream);
   if (stream2) cudaStreamDestroy(stream2);
 }
@@ -206,6 +211,19 @@ sk_status Context::reserveLod(FrameScratch& f, const World& w, cudaStream_t s) {
   return SK_OK;
 }
 
+// Rows of tiles per band: up to kMaxBands bands of at least kBandTiles tiles (8 blocks for each of 148
+// multiprocessors: fewer wait for their deepest tiles more than they work), or 0, one launch, where that
+// leaves one. Draw and read, in one launch and in bands (us): 100k splats at 720p (3 bands) 208.5 and 193;
+// a 2M-leaf LOD frame at 1080p (6) 427 and 400; 1M at 1080p (6) 560 and 448; 3M at 3840 x 2160 (8) 1590 and
+// 1112. Bands of 600 tiles: 201, 460, 480 and 1117; of 2400: 211, 411, 462 and 1112.
+constexpr uint32_t kBandTiles = 1184;
+
+uint32_t Context::bandRowsFor(uint32_t w, uint32_t h) const {
+  const uint32_t tilesX = (w + kTileSize - 1) / kTileSize, tilesY = (h + kTileSize - 1) / kTileSize;
+  const uint32_t count = std::min(tilesX * tilesY / kBandTiles, kMaxBands);
+  return count < 2 ? 0 : (tilesY + count - 1) / count;
+}
+
 sk_status Context::reserveView(uint32_t w, uint32_t h) {
   const size_t pixelBytes = imageFormat == SK_FORMAT_RGBA32F ? 16 : 4;
   if (copyStream) cudaStreamSynchronize(copyStream);  // no capture copy reads an image freed here
@@ -216,6 +234,13 @@ sk_status Context::reserveView(uint32_t w, uint32_t h) {
   for (auto& sl : slots) {
     if (e == cudaSuccess) e = sl.hostCounters.allocate(sizeof(FrameCounters));
     if (e == cudaSuccess) e = sl.hostCamera.allocate(sizeof(Camera));
+  }
+  if (bandRowsFor(w, h)) {  // made with the view: a first frame would wait 120 us for them
+    for (cudaStream_t* st : {&bands.side, &bands.copies})
+      if (e == cudaSuccess && !*st) e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !bands.listed) e = cudaEventCreateWithFlags(&bands.listed, cudaEventDisableTiming);
+    for (auto& ev : bands.drawn)
+      if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   }
   return check(e, "view buffers");
 }
@@ -426,12 +451,45 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
     c.fragments = &fc->fragments_lo;
     c.countFragments = timing == 1 ? 1u : 0u;
     c.loaded = &fc->loaded;
-    e = launchComposite(c, s);
+    c.tiles = tilesX * tilesY;
+    e = view.bandRows ? enqueueBands(c, view.bandRows, s) : launchComposite(c, s);
   }
   if (timing != 0) cudaEventRecord(events[5], s);
   if (e == cudaSuccess && view.hostCounters)
     e = cudaMemcpyAsync(view.hostCounters, fc, sizeof(FrameCounters), cudaMemcpyDeviceToHost, s);
   return check(e, "frame");
+}
+
+cudaError_t Context::enqueueBands(const CompositeArgs& whole, uint32_t bandRows, cudaStream_t s) {
+  cudaError_t e = cudaEventRecord(bands.listed, s);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(bands.side, bands.listed, 0);
+  uint32_t k = 0;
+  for (uint32_t row = 0; row < whole.tilesY && e == cudaSuccess; row += bandRows, ++k) {
+    CompositeArgs c = whole;
+    c.firstTile = row * c.tilesX;
+    c.tiles = std::min(bandRows, c.tilesY - row) * c.tilesX;
+    const cudaStream_t on = k & 1u ? bands.side : s;
+    e = launchComposite(c, on);
+    if (e == cudaSuccess) e = cudaEventRecord(bands.drawn[k], on);
+  }
+  // the frame is done when the last band of the side stream is, too
+  if (k > 1 && e == cudaSuccess) e = cudaStreamWaitEvent(s, bands.drawn[k & 1u ? k - 2 : k - 1], 0);
+  return e;
+}
+
+cudaError_t Context::copyBands(void* host, const Slot& slot) {
+  const size_t row = size_t{slot.width} * (imageFormat == SK_FORMAT_RGBA32F ? 16 : 4);
+  const uint32_t pixels = slot.bandRows * kTileSize;
+  const auto* image = static_cast<const uint8_t*>(imageOf(slot.image));
+  cudaError_t e = cudaSuccess;
+  for (uint32_t k = 0; k * pixels < slot.height && e == cudaSuccess; ++k) {
+    const uint32_t first = k * pixels, rows = std::min(pixels, slot.height - first);
+    e = cudaStreamWaitEvent(bands.copies, bands.drawn[k], 0);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(static_cast<uint8_t*>(host) + first * row, image + first * row, rows * row,
+                          cudaMemcpyDeviceToHost, bands.copies);
+  }
+  return e;
 }
 
 cudaError_t Context::enqueueSortedLists(FrameScratch& f, const ViewTarget& view, cudaStream_t s) {
@@ -497,6 +555,7 @@ ViewTarget Context::plainView(const Slot& slot) {
   v.width = width;
   v.height = height;
   v.direct = slot.direct;
+  v.bandRows = slot.bandRows;
   v.image = imageOf(slot.image);
   v.counters = static_cast<FrameCounters*>(second ? frameCounters2.ptr : frameCounters.ptr);
   v.hostCounters = static_cast<FrameCounters*>(slot.hostCounters.ptr);
@@ -611,7 +670,10 @@ sk_status Context::finishOldest() {
     ++redraws;
     sk_status st = reserveScratch(scratch, scratch.sources, need, scratch.maxTiles, stream);
     if (st == SK_OK && stream2) st = prepareSecondSlot();
-    for (size_t k = 0; st == SK_OK && k < inFlight.size(); ++k) st = enqueueSlot(inFlight[k]);
+    for (size_t k = 0; st == SK_OK && k < inFlight.size(); ++k) {
+      slots[inFlight[k]].bandRows = 0;  // the band events were those of the first drawing
+      st = enqueueSlot(inFlight[k]);
+    }
     if (st != SK_OK) {
       inFlight.clear();  // nothing of theirs is left running
       return st;
@@ -989,8 +1051,13 @@ sk_status sk_draw(sk_context* handle, const sk_frame* frame) {
   slot.frame.ranges = slot.ranges.data();
   slot.image = ctx->imageSlot;
   slot.number = ++ctx->submitted;  // pending captures are bound to this number
+  bool captured = false;
   for (auto& c : ctx->captures)
-    if (c.frame == 0) c.frame = slot.number;
+    if (c.frame == 0) c.frame = slot.number, captured = true;
+  slot.bandRows = ctx->bands.wanted && ctx->inFlight.empty() && !captured
+                      ? ctx->bandRowsFor(ctx->width, ctx->height)
+                      : 0;
+  if (slot.bandRows) ctx->bands.wanted = false;  // until it is read
   const sk_status st = ctx->enqueueSlot(index);
   if (st != SK_OK) {
     for (auto& c : ctx->captures)
@@ -1021,9 +1088,12 @@ sk_status sk_read_image(sk_context* handle, void* host, size_t bytes, int32_t fo
   if (own && bytes >= need && !ctx->inFlight.empty()) {
     const uint32_t newest = ctx->inFlight.back();
     const uint64_t redraws = ctx->redraws;
-    cudaError_t e = cudaMemcpyAsync(host, ctx->imageOf(ctx->slots[newest].image), need, cudaMemcpyDeviceToHost,
-                                    ctx->streamOf(newest));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->streamOf(newest));
+    const sk::Context::Slot& slot = ctx->slots[newest];
+    const cudaStream_t copies = slot.bandRows ? ctx->bands.copies : ctx->streamOf(newest);
+    if (ctx->inFlight.size() == 1) ctx->bands.wanted = true;
+    cudaError_t e = slot.bandRows ? ctx->copyBands(host, slot)
+                                  : cudaMemcpyAsync(host, ctx->imageOf(slot.image), need, cudaMemcpyDeviceToHost, copies);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(copies);
     const sk_status copied = ctx->check(e, "readback");
     if (copied != SK_OK) return copied;
     const sk_status finished = ctx->finishFrame(true);

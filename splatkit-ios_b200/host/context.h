@@ -109,6 +109,7 @@ struct ViewTarget {
   const Camera* camera = nullptr;          // device, written before the pipeline runs (LOD worlds)
   const Camera* hostCamera = nullptr;      // the same on the host
   bool direct = false;                     // lists per patch, written in place
+  uint32_t bandRows = 0;                   // rows of tiles per band (Context::Bands); 0: one launch
   uint32_t tilesX() const { return (width + kTileSize - 1) / kTileSize; }
   uint32_t tilesY() const { return (height + kTileSize - 1) / kTileSize; }
   uint32_t binsX() const { return (width + kBinSize - 1) / kBinSize; }
@@ -162,10 +163,27 @@ struct Context {
     uint32_t total = 0, image = 0;
     uint32_t width = 0, height = 0;  // target it was drawn on
     bool direct = false;             // its lists are per patch (csrc/cell_lists.cu)
+    uint32_t bandRows = 0;           // rows of tiles per band it was drawn in; 0: one launch
     uint64_t number = 0;  // the submitted-frame count it was drawn as
   };
   Slot slots[kFrameSlots];
   std::deque<uint32_t> inFlight;  // slots of the frames in flight, oldest first
+  // A frame that is read as soon as it is drawn (sk_read_image with no other frame in flight) is drawn in
+  // bands, launches of some rows of tiles each, and the image of one band crosses to the host while the
+  // next ones are drawn. The bands take turns on the frame's stream and a side stream, so that a band's
+  // blocks fill the chip as the one before it drains.
+  static constexpr uint32_t kMaxBands = 8;
+  struct Bands {
+    cudaStream_t side = nullptr, copies = nullptr;
+    cudaEvent_t listed = nullptr, drawn[kMaxBands] = {};
+    // Whether the last frame drawn in bands was read while it was the only one in flight. A program that
+    // draws without reading goes without them after one frame: short bands wait for their deepest tiles
+    // one after the other (a LOD frame at 1080p, not read: 277 us in one launch, 340 in six).
+    bool wanted = true;
+  } bands;
+  uint32_t bandRowsFor(uint32_t width, uint32_t height) const;
+  cudaError_t enqueueBands(const CompositeArgs& c, uint32_t bandRows, cudaStream_t s);
+  cudaError_t copyBands(void* host, const Slot& slot);
   // Frame captures (captureNextFrame): once one is requested the frames alternate between two
   // images, so the copy of one frame's image to the host (on copyStream) overlaps the drawing of
   // the next; a frame waits for the copy that still reads its image before it draws.
