@@ -136,8 +136,10 @@ class ClockSampler:
 # ---- algorithmic bytes per stage ---------------------------------------------------------------
 def stage_bytes(stats, bits, n=SPLATS, width=WIDTH, height=HEIGHT, sh_words=24):
     v, inst, read = stats["draw_count"], stats["instances"], stats["instances_read"]
-    cells = ((width + 31) // 32) * ((height + 31) // 32)
-    blocks = (v + 1023) // 1024
+    columns, rows = (width + 31) // 32, (height + 31) // 32
+    edge = next((k for k in (1, 2) if -(-columns // k) * -(-rows // k) <= 320), 4)  # cells per patch side
+    patches = -(-columns // edge) * -(-rows // edge)
+    blocks = (v + 511) // 512
     return {
         # 32 B record per source splat, the SH record (96 B at SH3, device stride) of each
         # survivor, then a 4 B key, a 32 B projected record and a 16 B tile span per survivor
@@ -146,10 +148,11 @@ def stage_bytes(stats, bits, n=SPLATS, width=WIDTH, height=HEIGHT, sh_words=24):
         # digit histogram is summed by the cull as it writes the keys): 56 B/key at 32 bits,
         # 24 B/key at 16 bits
         "sort": (56 if bits == 32 else 24) * v,
-        # direct cell lists: count and emit each read order + span (20 B per survivor); the
-        # per-block cell counts are written, read and turned into block starts (read again by
-        # the emission): 3 x 4 B per (block, cell); 8 B range per cell; 4 B written per entry
-        "bin": 40 * v + 12 * blocks * cells + 8 * cells + 4 * inst,
+        # lists per patch: count and emit each read order + span (20 B per survivor); the per-block patch
+        # counts are written, read and turned into block starts (read again by the emission): 3 x 4 B
+        # per (block, patch); 8 B range per patch; an index and a cell mask written per entry (at most
+        # one entry per (survivor, cell) pair, the figure the frame reports)
+        "bin": 40 * v + 12 * blocks * patches + 8 * patches + 6 * inst,
         # index + projected record per list entry read, RGBA8 image write
         "composite": 36 * read + width * height * 4,
     }
@@ -416,14 +419,14 @@ def run_ours(args):
         dominant = max(("cull", "sort", "bin", "composite"), key=lambda k: mean[k + "_ms"])
         peak, peak_kind = measured_peaks()
         achieved = bytes_by_stage[dominant] / (mean[dominant + "_ms"] / 1000.0) / 1e9
-        kernel_tag = {"cull": "visibility", "sort": "radix_sort", "bin": "cell_lists",
+        kernel_tag = {"cull": "visibility", "sort": "radix_sort", "bin": "patch_lists",
                       "composite": "composite"}[dominant]
         profile = {"cull": "visibility_1m_sh3_1080p", "sort": "radix_sort_scatter_depth_1m_sh3_1080p",
-                   "bin": "cell_lists_emit_1m_sh3_1080p", "composite": "composite_1m_sh3_1080p"}[dominant]
+                   "bin": "patch_lists_emit_1m_sh3_1080p", "composite": "composite_1m_sh3_1080p"}[dominant]
         traffic = traffic_from_profiles(profile) if args.bits == 16 else None
         passes = 2 if args.bits == 16 else 4
-        # visibility (with the depth keys' digit histogram), the depth sort's scatter passes, cell
-        # lists (count, scan, emit), composite
+        # visibility (with the depth keys' digit histogram), the depth sort's scatter passes, patch
+        # lists (count, scan, emit), composite (one launch: these frames are not read as soon as drawn)
         launches_per_frame = 1 + passes + 3 + 1
         line = {
             "metric": METRIC, "value": value, "unit": "frames/s", "n_gpus": world,

@@ -353,7 +353,7 @@ typedef struct {
                                  each warp's tile instances evenly over its lanes */
   uint32_t sort_tile_keys;    /* keys per radix-sort scatter tile: 2048, 4096 or 6144 */
   uint32_t lanes;             /* submissions in flight (<= the batch's lanes) */
-  uint32_t sorted_lists;      /* cell lists: 0 written in place per view (where every view's
+  uint32_t sorted_lists;      /* lists: 0 per patch, written in place per view (where every view's
                                  target is one they fit), 1 always by the batch-wide stable sort
                                  of (cell, splat) pairs */
   double gpu_ms;              /* autotune: device time of the chosen kernels for the sample */

@@ -9,8 +9,8 @@
 // the sorted order downstream is deterministic and equal to a stable sort of (key, source
 // position).
 //
-// A frame larger than L2 is bound by latency (1M SH3 splats, 128 MB: 65 us, 2 TB/s, 22 us at the measured
-// peak), a batch of many waves by instructions (12M splats in 560 us, 476 without the harmonics' arithmetic).
+// Bound by instruction issue and latency (1M SH3 splats, 128 MB: 65 us, 2 TB/s, 22 us at the measured peak,
+// 68% of the issue slots; 3M: 201 us, 75%, 60 us of it the span masks at 3840 x 2160), a batch of many waves by instructions (12M splats in 560 us, 476 without the harmonics' arithmetic).
 // One splat per thread, four blocks per SM that take tiles in turn and look a tile's place up one tile
 // later: 80 -> 65 us (1M), 222 -> 201 (3M), 30 -> 18 (a 0.4M-splat LOD cut), 15.5 -> 8.0 (4k) against 1024-splat
 // tiles that waited at once. With two splats per thread 78 us (1M), with three blocks per SM 71, with five 74.
