@@ -10,7 +10,9 @@ import pytest
 import splatkit_b200 as sk
 from splatkit_b200 import synthetic
 
+from scenes import lod_camera
 from test_gpu_cell_lists import frames_for
+from test_gpu_lod_one_launch import fan_tree
 
 
 def banded(r, frame, fmt):
@@ -75,3 +77,21 @@ def test_bands_of_a_frame_drawn_again(cuda_device):
         second = banded(r, frame, sk.FORMAT_RGBA8)
         want = captured(r, frame, buffer_for(r, w, h, sk.FORMAT_RGBA8))
     assert np.array_equal(first, want) and np.array_equal(second, want)
+
+
+@pytest.mark.gpu
+def test_bands_of_a_lod_frame(cuda_device):
+    w, h = 1920, 1080
+    tree = fan_tree(8, 4)
+    view, proj, pos = lod_camera(0.0)
+    images = []
+    for capture in (False, True):  # fresh worlds: the threshold adapts from frame to frame
+        with sk.Renderer(w, h) as r:
+            r.upload_lod_world(tree, 0, 100_000)
+            frame = sk.Frame(view, proj, pos, [], 0)
+            out = buffer_for(r, w, h, sk.FORMAT_RGBA8)
+            images.append([captured(r, frame, out) if capture else banded(r, frame, sk.FORMAT_RGBA8)
+                           for _ in range(2)])
+    for a, b in zip(*images):
+        assert np.array_equal(a, b)
+    assert images[0][0].any()
