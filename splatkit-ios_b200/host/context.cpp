@@ -516,7 +516,7 @@ cudaError_t Context::enqueueSortedLists(FrameScratch& f, const ViewTarget& view,
     a.valuesOut = static_cast<uint32_t*>(f.instValuesSorted.ptr);
     a.count = &fc->instances;
     a.capacity = f.instanceCapacity;
-    a.bits = 16;
+    a.bits = view.binsX() * view.binsY() > 65536 ? 24 : 16;  // of a cell id
     sortBindWorkspaceFor(a, f.tileSortWorkspace.ptr, f.instanceCapacity, kTileSortTileKeys);
     a.tileKeys = kTileSortTileKeys;
     a.epoch = nextEpoch(4);

@@ -82,3 +82,34 @@ def test_batches_of_small_targets_equal_the_sorted_frames(cuda_device, n, log_sc
         r.draw(frame)
         assert np.array_equal(image, r.read_image(sk.FORMAT_RGBA8))
     r.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(8192, 8192), (8224, 8224), (16384, 4160)])
+def test_sorted_lists_of_65536_cells_and_more(cuda_device, w, h):
+    """Cell ids of more than 16 bits: every pair is in one list, and the lists are those of the cells: a
+    splat's list entries form the rows and columns of a box."""
+    cloud = synthetic.random_cloud(200, seed=31, sh_degree=0, log_scale_mean=-1.0)
+    frame = frames_for(cloud, w, h, (11,))[0]
+    with sk.Renderer(w, h) as r:
+        r.set_binning("sorted")
+        r.upload_world(cloud, 0)
+        r.draw(frame)
+        ranges, values = r.read_tile_lists()
+        order = r.read_order()
+        assert r.stats()["instances"] == len(values) == int((ranges[:, 1] - ranges[:, 0]).sum())
+    rank = np.empty(int(order.max()) + 1, np.int64)
+    rank[order] = np.arange(len(order))
+    columns, seen = (w + 31) // 32, {}
+    for cell in np.flatnonzero(ranges[:, 1] > ranges[:, 0]):
+        entries = values[ranges[cell, 0]:ranges[cell, 1]]
+        assert (np.diff(rank[entries]) > 0).all()  # front to back, each splat once
+        for v in entries:
+            seen.setdefault(int(v), []).append((cell // columns, cell % columns))
+    for cells in seen.values():  # convex: every row of a splat's cells is one run, in adjacent rows
+        rows = {}
+        for y, x in cells:
+            rows.setdefault(y, []).append(x)
+        assert max(rows) - min(rows) + 1 == len(rows)
+        for xs in rows.values():
+            assert max(xs) - min(xs) + 1 == len(xs)
