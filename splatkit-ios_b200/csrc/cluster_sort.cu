@@ -7,7 +7,8 @@
 // radix_sort.cu does: per warp, row by row, in source order), writes the block's digit counts into every
 // block of the cluster, and writes the digit runs, staged in order, to the blocks that hold their
 // positions (the last pass: to the output); two cluster barriers (hardware barriers of co-scheduled
-// blocks, nothing polls) stand in for the kernel boundaries and the look-back. The order is the same.
+// blocks, nothing polls) stand in for the kernel boundaries and the look-back, and one more, under the
+// loads and the first ranking, makes sure that every block has started. The order is the same.
 //
 // Bound by the chain of barriers and shared-memory round trips, about 4.5 us a pass: 20,011 32-bit keys
 // 37 -> 19.5 us (8 blocks of 1024 threads 29.5, 16 of 1024 21.4, 16 of 256 19.7; counts read from the other
@@ -15,6 +16,7 @@
 // 16 SMs are too few: at 100k keys a pass would take as long as a scatter kernel.
 #include <cuda_runtime.h>
 
+#include "sk_cluster.cuh"
 #include "sk_device.cuh"
 #include "sk_kernels.h"
 #include "sk_launch.cuh"
@@ -48,23 +50,6 @@ struct Smem {
   uint32_t warpSums[kWarps];
 };
 
-__device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t clusterRank() {
-  uint32_t r;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// Stores to the word at `p` of this block's shared memory, in block `rank` of the cluster.
-__device__ __forceinline__ void storeRemote(uint32_t* p, uint32_t rank, uint32_t v) {
-  const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-  asm volatile(
-      "{\n\t.reg .u32 a;\n\t"
-      "mapa.shared::cluster.u32 a, %0, %1;\n\t"
-      "st.shared::cluster.u32 [a], %2;\n\t}" ::"r"(at),
-      "r"(rank), "r"(v)
-      : "memory");
-}
 // Exclusive sum over the 256 values of each group of threads (every group holds the same ones).
 __device__ __forceinline__ uint32_t digitScan(uint32_t v, uint32_t* warpSums) {
   const uint32_t warp = threadIdx.x >> 5, lane = laneId();
@@ -86,6 +71,7 @@ __device__ __forceinline__ uint32_t digitScan(uint32_t v, uint32_t* warpSums) {
 template <uint32_t kRows>
 __global__ void __launch_bounds__(kThreads, 1) clusterSortKernel(const __grid_constant__ ClusterSortArgs a) {
   constexpr uint32_t kShare = kThreads * kRows;
+  clusterArrive();
   extern __shared__ uint32_t dynamic[];
   Smem& s = *reinterpret_cast<Smem*>(dynamic);
   uint32_t* stageKey = dynamic + sizeof(Smem) / 4;
@@ -144,6 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) clusterSortKernel(const __grid_co
       if (g < group) lower += t;
       total += t;
     }
+    if (p == 0) clusterWait();  // every block of the cluster has started
     // The padding of a last block counts as digit 255 here, but no block after it has keys.
     for (uint32_t b = group; b < blocks; b += kGroups) storeRemote(&s.blockTotal[rank][d], b, total);
     const uint32_t local = digitScan(total, s.warpSums);

@@ -27,6 +27,7 @@
 
 #include <algorithm>
 
+#include "sk_cluster.cuh"
 #include "sk_device.cuh"
 #include "sk_kernels.h"
 #include "sk_launch.cuh"
@@ -472,23 +473,6 @@ struct WalkSmem {
   uint32_t warpRed[8][kClusterWarps];
 };
 
-__device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t clusterRank() {
-  uint32_t r;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void storeRemote(uint32_t* p, uint32_t rank, uint32_t v) {
-  const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-  asm volatile(
-      "{\n\t.reg .u32 a;\n\t"
-      "mapa.shared::cluster.u32 a, %0, %1;\n\t"
-      "st.shared::cluster.u32 [a], %2;\n\t}" ::"r"(at),
-      "r"(rank), "r"(v)
-      : "memory");
-}
-
 // Adds up each thread's kSums values over the cluster: s.totals (all blocks) and s.before (the blocks
 // before this one); value 6 is a maximum. Every thread of the cluster calls this.
 __device__ __forceinline__ void exchange(WalkSmem& s, uint32_t which, uint32_t rank, const uint32_t (&mine)[kSums],
@@ -546,10 +530,12 @@ __device__ __forceinline__ void blockScan(WalkSmem& s, const uint32_t (&v)[kCoun
 
 __global__ void __launch_bounds__(kClusterThreads, 1)
     lodWalkKernel(const Camera* __restrict__ camera, const __grid_constant__ LodArgs a) {
+  clusterArrive();
   chainedKernelStart();
   __shared__ WalkSmem s;
   loadCamera(camera, &s.cam);
   __syncthreads();
+  clusterWait();  // every block of the cluster has started
   const uint32_t rank = clusterRank();
   uint32_t* words = reinterpret_cast<uint32_t*>(a.costs);  // an item's flags and cost, kept by its own thread
   uint32_t count = 0, packets = 0, records = 0, limited = 0, evaluated = 0, accepted = 0, active = 1;
