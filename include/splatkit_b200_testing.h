@@ -23,6 +23,10 @@ extern "C" {
  * allocations and do not count. */
 void sk_testing_fail_device_allocations(uint32_t count);
 
+/* `count` device allocations pass before those that sk_testing_fail_device_allocations (called
+ * first) makes fail, so that an upload can fail half way. */
+void sk_testing_pass_device_allocations(uint32_t count);
+
 /* The next CUDA status `ctx` checks reads as `cuda_error` (a cudaError_t value) instead of its
  * own: a stand-in for a failing CUDA call. An error other than out-of-memory latches the context
  * failed, as a real one would (sk_gpu_failed, SK_E_DEVICE from every later call). */

@@ -26,14 +26,24 @@ namespace sk {
 
 // ---- buffers ------------------------------------------------------------------------------
 
-std::atomic<uint32_t> gTestFailedAllocations{0};
+std::atomic<uint32_t> gTestFailedAllocations{0}, gTestPassedAllocations{0};
+
+namespace {
+// Test hooks (sk_testing_pass_device_allocations, sk_testing_fail_device_allocations): whether this
+// allocation fails as if out of memory.
+bool testAllocationFails() {
+  if (gTestFailedAllocations.load() == 0) return false;
+  for (std::atomic<uint32_t>* count : {&gTestPassedAllocations, &gTestFailedAllocations})
+    for (uint32_t left = count->load(); left > 0;)
+      if (count->compare_exchange_weak(left, left - 1)) return count == &gTestFailedAllocations;
+  return false;
+}
+}  // namespace
 
 cudaError_t DeviceBuffer::allocate(size_t n) {
   n = std::max<size_t>(n, 256);
   if (n <= bytes && ptr) return cudaSuccess;
-  // test hook (sk_testing_fail_device_allocations): this allocation fails as if out of memory
-  for (uint32_t left = gTestFailedAllocations.load(); left > 0;)
-    if (gTestFailedAllocations.compare_exchange_weak(left, left - 1)) return cudaErrorMemoryAllocation;
+  if (testAllocationFails()) return cudaErrorMemoryAllocation;
   void* fresh = nullptr;
   const cudaError_t e = cudaMalloc(&fresh, n);
   if (e != cudaSuccess) {
@@ -49,8 +59,7 @@ cudaError_t DeviceBuffer::allocate(size_t n) {
 cudaError_t DeviceBuffer::allocateOn(size_t n, cudaStream_t s) {
   n = std::max<size_t>(n, 256);
   if (n <= bytes && ptr) return cudaSuccess;
-  for (uint32_t left = gTestFailedAllocations.load(); left > 0;)
-    if (gTestFailedAllocations.compare_exchange_weak(left, left - 1)) return cudaErrorMemoryAllocation;
+  if (testAllocationFails()) return cudaErrorMemoryAllocation;
   void* fresh = nullptr;
   const cudaError_t e = cudaMallocAsync(&fresh, n, s);
   if (e != cudaSuccess) {
@@ -174,12 +183,17 @@ sk_status Context::reserveScratch(FrameScratch& f, uint32_t sources, uint32_t in
   grab(f.rangeStarts, size_t{kMaxRanges + 1} * 4);
   const bool fresh = f.counters.ptr == nullptr;
   grab(f.counters, 64 * 4);
-  if (e == cudaSuccess && fresh) e = cudaMemsetAsync(f.counters.ptr, 0, 64 * 4, s);
-  // Sort workspaces hold counters that must start at zero; status words carry epochs.
-  if (e == cudaSuccess) e = cudaMemsetAsync(f.sortWorkspace.ptr, 0, f.sortWorkspace.bytes, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(f.tileSortWorkspace.ptr, 0, f.tileSortWorkspace.bytes, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(f.visStatus.ptr, 0, f.visStatus.bytes, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(f.patchLists.ptr, 0, patchListStatusBytes(), s);
+  // Sort workspaces hold counters that must start at zero; status words carry epochs. Cleared also when a
+  // buffer could not be had: the frames after that draw with those that are there, moved ones among them.
+  auto clear = [&](const DeviceBuffer& b, size_t n) {
+    const cudaError_t c = b.ptr ? cudaMemsetAsync(b.ptr, 0, std::min(n, b.bytes), s) : cudaSuccess;
+    if (e == cudaSuccess) e = c;
+  };
+  if (fresh) clear(f.counters, 64 * 4);
+  clear(f.sortWorkspace, f.sortWorkspace.bytes);
+  clear(f.tileSortWorkspace, f.tileSortWorkspace.bytes);
+  clear(f.visStatus, f.visStatus.bytes);
+  clear(f.patchLists, patchListStatusBytes());
   if (e != cudaSuccess) return check(e, "frame buffers");
   f.sources = sources;
   f.instanceCapacity = instances;

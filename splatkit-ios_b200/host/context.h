@@ -27,8 +27,9 @@ inline int hostThreadsPublic() {
   return static_cast<int>(std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
 }
 
-// Test hook (sk_testing_fail_device_allocations): how many of the next device allocations fail.
-extern std::atomic<uint32_t> gTestFailedAllocations;
+// Test hooks (sk_testing_fail_device_allocations, sk_testing_pass_device_allocations): how many of the
+// next device allocations fail, and how many pass before those.
+extern std::atomic<uint32_t> gTestFailedAllocations, gTestPassedAllocations;
 
 // Owning device allocation; allocate() only grows, and keeps the old memory when it fails.
 struct DeviceBuffer {

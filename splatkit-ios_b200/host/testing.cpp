@@ -6,7 +6,12 @@
 
 extern "C" {
 
-void sk_testing_fail_device_allocations(uint32_t count) { sk::gTestFailedAllocations.store(count); }
+void sk_testing_fail_device_allocations(uint32_t count) {
+  sk::gTestFailedAllocations.store(count);
+  sk::gTestPassedAllocations.store(0);
+}
+
+void sk_testing_pass_device_allocations(uint32_t count) { sk::gTestPassedAllocations.store(count); }
 
 sk_status sk_testing_fail_next_check(sk_context* handle, int32_t cuda_error) {
   auto* ctx = reinterpret_cast<sk::Context*>(handle);

@@ -275,6 +275,7 @@ _SIGNATURES = {
                                                   ctypes.c_void_p]),
     # test hooks (include/splatkit_b200_testing.h)
     "sk_testing_fail_device_allocations": (None, [ctypes.c_uint32]),
+    "sk_testing_pass_device_allocations": (None, [ctypes.c_uint32]),
     "sk_testing_fail_next_check": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32]),
     "sk_testing_withhold_sort_status": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_uint32]),
 }
@@ -1014,9 +1015,11 @@ def radix_argsort_noalloc(keys_ptr: int, count_ptr: int, capacity: int, bits: in
         raise SplatError(st, "sk_radix_argsort_noalloc")
 
 
-def testing_fail_device_allocations(count: int):
-    """Test hook: the next `count` device allocations of the library fail as out of memory."""
+def testing_fail_device_allocations(count: int, after: int = 0):
+    """Test hook: `count` device allocations of the library fail as out of memory, the next ones or
+    those after `after` that pass."""
     library().sk_testing_fail_device_allocations(count)
+    library().sk_testing_pass_device_allocations(after)
 
 
 def sort_workspace_bytes(capacity: int) -> int:
