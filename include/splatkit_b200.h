@@ -285,7 +285,11 @@ sk_status sk_read_cut(sk_context* ctx, uint32_t* indices, uint32_t capacity, uin
                       uint32_t* lod_counters6);
 /* The last frame's binning lists: ranges[2 * c], ranges[2 * c + 1] = [start, end) of 32x32
  * binning cell c (row major) in `values`, which holds projected-record indices front to back
- * per cell. ranges needs 2 * cells words; *count receives the number of list entries. */
+ * per cell. ranges needs 2 * cells words; *count receives the number of list entries. A frame
+ * drawn from lists written in place keeps none per cell: the first call after it makes them, and
+ * grows the list buffers where the (splat, cell) pairs need more room (SK_E_OOM when there is
+ * none). Once a world larger than those before it has been uploaded, the lists of a frame drawn
+ * before that may be gone: the call then returns no entries and empty ranges. */
 sk_status sk_read_tile_lists(sk_context* ctx, uint32_t* ranges, uint32_t* values,
                              uint32_t capacity, uint32_t* count);
 

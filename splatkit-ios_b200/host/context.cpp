@@ -163,6 +163,7 @@ sk_status Context::reserveScratch(FrameScratch& f, uint32_t sources, uint32_t in
     if (e == cudaSuccess) e = b.allocate(n);
   };
   const uint32_t visTiles = (sources + visibilityTileSplats() - 1) / visibilityTileSplats();
+  const void* const before[4] = {f.spans.ptr, f.order.ptr, f.instValuesSorted.ptr, f.ranges.ptr};
   grab(f.keys, size_t{sources} * 4);
   grab(f.projected, size_t{sources} * sizeof(Projected));
   grab(f.spans, size_t{sources} * 16);
@@ -194,11 +195,24 @@ sk_status Context::reserveScratch(FrameScratch& f, uint32_t sources, uint32_t in
   clear(f.tileSortWorkspace, f.tileSortWorkspace.bytes);
   clear(f.visStatus, f.visStatus.bytes);
   clear(f.patchLists, patchListStatusBytes());
+  // A buffer that moved no longer holds what the last frame left in it.
+  if (before[0] != f.spans.ptr || before[1] != f.order.ptr) f.spansKept = false;
+  if (&f == &scratchOf(lastSlot) && (before[2] != f.instValuesSorted.ptr || before[3] != f.ranges.ptr))
+    listsPerCell = false;
   if (e != cudaSuccess) return check(e, "frame buffers");
   f.sources = sources;
   f.instanceCapacity = instances;
   f.maxTiles = std::max(f.maxTiles, maxTiles);
   return SK_OK;
+}
+
+sk_status Context::reserveForWorld(uint32_t count) {
+  const uint32_t instances = std::max(scratch.instanceCapacity, instanceGuess(count));
+  // Where only the spans move, the last frame's lists stay readable: expanded while the spans are there.
+  if (lastSlot == 0 && instances == scratch.instanceCapacity && size_t{count} * 16 > scratch.spans.bytes &&
+      expandLists() == SK_E_DEVICE)
+    return SK_E_DEVICE;
+  return reserveScratch(scratch, count, instances, scratch.maxTiles, stream);
 }
 
 sk_status Context::reserveLod(FrameScratch& f, const World& w, cudaStream_t s) {
@@ -447,7 +461,7 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
     pl.error = error;
     e = launchPatchLists(b, pl, s);
   }
-  if (e == cudaSuccess && !direct) e = enqueueSortedLists(f, view, s);
+  if (e == cudaSuccess && !direct) e = enqueueSortedLists(f, view, f.sources, s);
   if (timed) cudaEventRecord(events[4], s);
   if (e == cudaSuccess) {
     CompositeArgs c{};
@@ -506,13 +520,14 @@ cudaError_t Context::copyBands(void* host, const Slot& slot) {
   return e;
 }
 
-cudaError_t Context::enqueueSortedLists(FrameScratch& f, const ViewTarget& view, cudaStream_t s) {
+cudaError_t Context::enqueueSortedLists(FrameScratch& f, const ViewTarget& view, uint32_t sources,
+                                        cudaStream_t s) {
   FrameCounters* fc = view.counters;
   BinArgs b{};
   b.spans = static_cast<const uint4*>(f.spans.ptr);
   b.order = static_cast<const uint32_t*>(f.order.ptr);
   b.count = &fc->visible;
-  b.capacity = f.sources;
+  b.capacity = sources;
   b.width = view.width, b.height = view.height, b.tilesX = view.binsX(), b.tilesY = view.binsY();
   b.instanceKeys = static_cast<uint32_t*>(f.instKeys.ptr);
   b.instanceValues = static_cast<uint32_t*>(f.instValues.ptr);
@@ -546,8 +561,8 @@ cudaError_t Context::enqueueSortedLists(FrameScratch& f, const ViewTarget& view,
 
 sk_status Context::expandLists() {
   const Slot& slot = slots[lastSlot];
-  if (!slot.direct || listsExpanded) return SK_OK;
   FrameScratch& f = scratchOf(lastSlot);
+  if (listsPerCell || !f.spansKept) return SK_OK;
   const cudaStream_t s = streamOf(lastSlot);
   if (lastCounters.instances > f.instanceCapacity) {  // a pair per cell where the frame needed one per patch
     const sk_status st = reserveScratch(f, f.sources, lastCounters.instances, f.maxTiles, s);
@@ -557,9 +572,9 @@ sk_status Context::expandLists() {
   view.width = slot.width;
   view.height = slot.height;
   cudaError_t e = clearTileRanges(static_cast<uint2*>(f.ranges.ptr), view.binsX() * view.binsY(), s);
-  if (e == cudaSuccess) e = enqueueSortedLists(f, view, s);
+  if (e == cudaSuccess) e = enqueueSortedLists(f, view, slot.sources, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  listsExpanded = e == cudaSuccess;
+  listsPerCell = e == cudaSuccess;
   return check(e, "tile lists");
 }
 
@@ -621,6 +636,7 @@ sk_status Context::enqueueSlot(uint32_t index) {
   slot.direct = view.direct;
   slot.width = width;
   slot.height = height;
+  slot.sources = f.sources;
   // A flat frame's camera travels in the cull's parameters; a LOD world's walk reads it from memory too.
   cudaError_t e = cudaSuccess;
   if (world.lod)
@@ -635,6 +651,7 @@ sk_status Context::enqueueSlot(uint32_t index) {
   sk_status st = enqueuePipeline(f, view, slot.frame, slot.total, s, timeStages,
                                  slot.events);
   if (st != SK_OK) return st;
+  f.spansKept = true;
   st = check(cudaEventRecord(slot.done, s), "frame");
   if (st != SK_OK) return st;
   // captures of this frame copy its image once it is drawn (again after a redraw)
@@ -695,7 +712,7 @@ sk_status Context::finishOldest() {
     return finishOldest();
   }
   lastSlot = inFlight.front();
-  listsExpanded = false;
+  listsPerCell = !slot.direct;
   inFlight.pop_front();
   ++completed;
   lastCounters = c;
@@ -912,9 +929,7 @@ sk_status sk_upload_world(sk_context* handle, const sk_cloud_view* cloud, int32_
   sk::World fresh;
   st = ctx->uploadCloud(*cloud, maxSh, fresh);
   if (st != SK_OK) return st;
-  st = ctx->reserveScratch(ctx->scratch, cloud->count,
-                           std::max(ctx->scratch.instanceCapacity, ctx->instanceGuess(cloud->count)),
-                           ctx->scratch.maxTiles, ctx->stream);
+  st = ctx->reserveForWorld(cloud->count);
   if (st != SK_OK) return st;
   ctx->world = std::move(fresh);
   ctx->labels.release();  // labels belong to the world they were uploaded for
@@ -933,9 +948,7 @@ sk_status sk_create_slab(sk_context* handle, uint32_t capacity, int32_t shDegree
   if (e == cudaSuccess) e = cudaMemset(fresh.splats.ptr, 0, fresh.splats.bytes);
   if (e == cudaSuccess) e = cudaMemset(fresh.sh.ptr, 0, fresh.sh.bytes);
   if (e != cudaSuccess) return ctx->check(e, "slab");
-  st = ctx->reserveScratch(ctx->scratch, capacity,
-                           std::max(ctx->scratch.instanceCapacity, ctx->instanceGuess(capacity)),
-                           ctx->scratch.maxTiles, ctx->stream);
+  st = ctx->reserveForWorld(capacity);
   if (st != SK_OK) return st;
   fresh.count = capacity;
   fresh.shDegree = shDegree;
@@ -1018,9 +1031,7 @@ sk_status sk_upload_lod_world(sk_context* handle, const sk_lod_view* tree, int32
   st = ctx->reserveLod(ctx->scratch, fresh, ctx->stream);
   if (st != SK_OK) return st;
   // Projections and sort scratch scale with the cut, not with all resident nodes.
-  st = ctx->reserveScratch(ctx->scratch, capacity,
-                           std::max(ctx->scratch.instanceCapacity, ctx->instanceGuess(capacity)),
-                           ctx->scratch.maxTiles, ctx->stream);
+  st = ctx->reserveForWorld(capacity);
   if (st != SK_OK) return st;
   ctx->world = std::move(fresh);
   ctx->labels.release();  // labels belong to the world they were uploaded for
@@ -1284,12 +1295,17 @@ sk_status sk_read_tile_lists(sk_context* handle, uint32_t* ranges, uint32_t* val
   sk_status st = ctx->finishFrame(true);
   if (st != SK_OK) return st;
   const bool direct = ctx->slots[ctx->lastSlot].direct;
-  if (direct && (st = ctx->expandLists()) != SK_OK) return st;
+  if ((st = ctx->expandLists()) != SK_OK) return st;
+  const size_t bins = size_t{(ctx->width + sk::kBinSize - 1) / sk::kBinSize} *
+                      ((ctx->height + sk::kBinSize - 1) / sk::kBinSize);
+  if (!ctx->listsPerCell) {  // a larger world took the place of what the lists are made from
+    if (count) *count = 0;
+    if (ranges) std::fill_n(ranges, 2 * bins, 0u);
+    return SK_OK;
+  }
   const uint32_t n = std::min(ctx->lastCounters.instances, ctx->scratchOf(ctx->lastSlot).instanceCapacity);
   if (count) *count = n;
   cudaError_t e = cudaSuccess;
-  const size_t bins = size_t{(ctx->width + sk::kBinSize - 1) / sk::kBinSize} *
-                      ((ctx->height + sk::kBinSize - 1) / sk::kBinSize);
   if (ranges) e = cudaMemcpy(ranges, ctx->scratchOf(ctx->lastSlot).ranges.ptr, bins * 8, cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && ranges && direct)  // an empty cell's range sits after the cells before it
     for (size_t c = 0, run = 0; c < bins; ++c) {

@@ -96,6 +96,7 @@ struct FrameScratch {
   DeviceBuffer lodIndices, lodFrontier[2], lodCosts, lodOffsets, lodPackets, lodState, lodStatus,
       lodCounters;
   uint32_t lodFrontierCapacity = 0;
+  bool spansKept = false;  // spans and order are still where the last frame wrote them
   FrameScratch() = default;
   FrameScratch(const FrameScratch&) = delete;
   FrameScratch& operator=(const FrameScratch&) = delete;
@@ -163,6 +164,7 @@ struct Context {
     std::vector<sk_range> ranges;
     uint32_t total = 0, image = 0;
     uint32_t width = 0, height = 0;  // target it was drawn on
+    uint32_t sources = 0;            // of its scratch when it was drawn
     bool direct = false;             // its lists are per patch (csrc/cell_lists.cu)
     uint32_t bandRows = 0;           // rows of tiles per band it was drawn in; 0: one launch
     uint64_t number = 0;  // the submitted-frame count it was drawn as
@@ -226,6 +228,8 @@ struct Context {
   // Scratch for `sources` splats, `instances` tile instances and targets up to maxTiles tiles.
   sk_status reserveScratch(FrameScratch& f, uint32_t sources, uint32_t instances, uint32_t maxTiles,
                            cudaStream_t s);
+  // Slot 0's scratch for a new world of `count` records.
+  sk_status reserveForWorld(uint32_t count);
   sk_status reserveLod(FrameScratch& f, const World& w, cudaStream_t s);
   sk_status reserveView(uint32_t width, uint32_t height);
   Camera cameraFor(const sk_frame& frame, uint32_t width, uint32_t height) const;
@@ -233,12 +237,13 @@ struct Context {
   // The whole frame pipeline for one view on stream s; nothing waits on the host.
   sk_status enqueuePipeline(FrameScratch& f, const ViewTarget& v, const sk_frame& frame,
                             uint32_t total, cudaStream_t s, uint32_t timing, cudaEvent_t* events);
-  // The lists by a stable sort of (cell, splat) pairs: binning, sort, ranges.
-  cudaError_t enqueueSortedLists(FrameScratch& f, const ViewTarget& v, cudaStream_t s);
-  // The last finished frame's per-cell lists from its spans and order, where it drew from direct
-  // lists (the read-back is per cell); its patch lists are overwritten.
+  // The lists by a stable sort of (cell, splat) pairs: binning, sort, ranges. sources bounds the survivors.
+  cudaError_t enqueueSortedLists(FrameScratch& f, const ViewTarget& v, uint32_t sources, cudaStream_t s);
+  // The last finished frame's per-cell lists from its spans and order, where the list buffers hold
+  // others (a direct frame's are per patch, and are overwritten). Does nothing, and leaves
+  // listsPerCell false, where the spans are gone (a larger world's buffers took their place).
   sk_status expandLists();
-  bool listsExpanded = false;  // of the last finished frame
+  bool listsPerCell = false;  // the list buffers hold the last finished frame's per-cell lists
   uint64_t redraws = 0;        // times the frames in flight were drawn again
   ViewTarget plainView(const Slot& slot);
   sk_status enqueueSlot(uint32_t slot);

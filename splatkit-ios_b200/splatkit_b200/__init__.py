@@ -624,7 +624,8 @@ class Renderer:
 
     def read_tile_lists(self):
         """(ranges (cells, 2), values): each 32x32 binning cell's front-to-back projected indices
-        (a composite tile of 16x16 pixels reads the list of the cell it lies in)."""
+        (a composite tile of 16x16 pixels reads the list of the cell it lies in); no entries where a
+        larger world has been uploaded since the frame."""
         cells = ((self.width + 31) // 32) * ((self.height + 31) // 32)
         ranges = np.zeros((cells, 2), np.uint32)
         n = ctypes.c_uint32()
