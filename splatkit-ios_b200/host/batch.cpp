@@ -581,14 +581,21 @@ sk_status Batch::enqueueImages(BatchLane& l) {
 
 sk_status Batch::enqueue(BatchLane& l) {
   const cudaStream_t s = l.stream;
-  // the shape a captured graph is valid for: every view's world, range and size
+  // what a captured graph is valid for: the policy and every view's world, range and size
   std::vector<uint64_t> shape;
   // a LOD view's selection bakes its context's threshold into the launch: no graph replay
   const bool useGraph = tuning.graphs && l.lodPlans.empty();
   if (useGraph) {
-    shape.reserve(size_t{l.viewCount} * 4 + 2);
+    shape.reserve(size_t{l.viewCount} * 4 + 7);
     shape.push_back(l.viewCount);
     shape.push_back(l.shDegree);
+    // the policy in the composite's parameters (the cull's part of it is in the cameras)
+    for (const double c : policy.background) {
+      uint64_t bits;
+      std::memcpy(&bits, &c, sizeof(bits));
+      shape.push_back(bits);
+    }
+    shape.push_back(policy.enable_early_termination ? 1u : 0u);
     // the launch shapes it was captured with
     shape.push_back((uint64_t{tuning.sortTileKeys} << 2) | (tuning.balancedEmit ? 2u : 0u) |
                     (l.directLists ? 1u : 0u));
