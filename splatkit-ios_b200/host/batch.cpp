@@ -81,6 +81,12 @@ uint32_t bitsFor(uint64_t values) {  // key bits, a multiple of 8, for keys < va
 }
 }  // namespace
 
+void Batch::dropGraph(BatchLane& l) {
+  if (l.graph) cudaGraphExecDestroy(l.graph);
+  l.graph = nullptr;
+  l.graphShape.clear();
+}
+
 sk_status Batch::reserve(BatchLane& l, uint32_t sources, uint32_t instances, uint32_t items,
                          uint32_t tiles, uint32_t views, uint64_t pixels) {
   // A buffer that must grow grows by at least half again: freeing the old one waits for the
@@ -105,6 +111,7 @@ sk_status Batch::reserve(BatchLane& l, uint32_t sources, uint32_t instances, uin
   };
   const bool grewSources = sources > l.sources, grewInstances = instances > l.instances;
   const bool grewItems = items > l.items;
+  const void* const before[3] = {l.sortWorkspace.ptr, l.tileSortWorkspace.ptr, l.visStatus.ptr};
   grab(l.keys, size_t{sources} * 4);
   grab(l.projected, size_t{sources} * sizeof(Projected));
   grab(l.spans, size_t{sources} * 16);
@@ -130,22 +137,22 @@ sk_status Batch::reserve(BatchLane& l, uint32_t sources, uint32_t instances, uin
   pin(l.hostCounters, sizeof(FrameCounters));
   pin(l.hostViewFirst, size_t{views + 1} * 4);
   if (l.destinations.empty()) pin(l.hostImage, pixels * 4);  // else views go to the caller's buffers
-  if (e == cudaSuccess && freshCounters) e = cudaMemsetAsync(l.counters.ptr, 0, 64 * 4, l.stream);
+  // Cleared also when a later buffer could not be had: the submissions after that draw with those that moved.
+  auto clear = [&](const DeviceBuffer& b) {
+    const cudaError_t c = b.ptr ? cudaMemsetAsync(b.ptr, 0, b.bytes, l.stream) : cudaSuccess;
+    if (e == cudaSuccess) e = c;
+  };
+  if (freshCounters) clear(l.counters);
   // fresh sort workspaces: counters and histogram accumulators start at zero
-  if (e == cudaSuccess && grewSources)
-    e = cudaMemsetAsync(l.sortWorkspace.ptr, 0, l.sortWorkspace.bytes, l.stream);
-  if (e == cudaSuccess && grewInstances)
-    e = cudaMemsetAsync(l.tileSortWorkspace.ptr, 0, l.tileSortWorkspace.bytes, l.stream);
+  if (grewSources || before[0] != l.sortWorkspace.ptr) clear(l.sortWorkspace);
+  if (grewInstances || before[1] != l.tileSortWorkspace.ptr) clear(l.tileSortWorkspace);
   // look-back status words of a fresh buffer must read "not ready"
-  if (e == cudaSuccess && grewItems) e = cudaMemsetAsync(l.visStatus.ptr, 0, l.visStatus.bytes, l.stream);
+  if (grewItems || before[2] != l.visStatus.ptr) clear(l.visStatus);
+  // buffers moved, or some of them did: a captured graph points at the old ones
+  if (e != cudaSuccess || grewSources || grewInstances || items > l.items || tiles > l.tiles || views > l.views ||
+      pixels > l.pixels)
+    dropGraph(l);
   if (e != cudaSuccess) return check(e, "batch buffers");
-  if (grewSources || grewInstances || items > l.items || tiles > l.tiles || views > l.views ||
-      pixels > l.pixels) {
-    // buffers moved: a captured graph points at the old ones
-    if (l.graph) cudaGraphExecDestroy(l.graph);
-    l.graph = nullptr;
-    l.graphShape.clear();
-  }
   l.sources = std::max(l.sources, sources);
   l.instances = std::max(l.instances, instances);
   l.items = std::max(l.items, items);
@@ -174,12 +181,13 @@ sk_status Batch::reserveLod(BatchLane& l, uint32_t indices, uint32_t frontier, u
   grab(l.lodStatus, size_t{tiles} * 3 * 8);
   grab(l.lodCounters, 2 * 4);
   if (e == cudaSuccess) e = l.hostLodReports.allocate(size_t{std::max(views, 1u)} * 8 * 4);
-  // fresh selection scratch: status words read "not ready", counters and state start at zero
-  if (e == cudaSuccess && (before[0] != l.lodStatus.ptr || before[1] != l.lodCounters.ptr ||
-                           before[2] != l.lodState.ptr)) {
-    e = cudaMemsetAsync(l.lodStatus.ptr, 0, l.lodStatus.bytes, l.stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(l.lodCounters.ptr, 0, l.lodCounters.bytes, l.stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(l.lodState.ptr, 0, l.lodState.bytes, l.stream);
+  // fresh selection scratch (also when a later buffer could not be had): status words read "not ready",
+  // counters and state start at zero
+  if (before[0] != l.lodStatus.ptr || before[1] != l.lodCounters.ptr || before[2] != l.lodState.ptr) {
+    for (const DeviceBuffer* b : {&l.lodStatus, &l.lodCounters, &l.lodState}) {
+      const cudaError_t c = b->ptr ? cudaMemsetAsync(b->ptr, 0, b->bytes, l.stream) : cudaSuccess;
+      if (e == cudaSuccess) e = c;
+    }
   }
   if (e != cudaSuccess) return check(e, "batch LOD buffers");
   l.lodFrontierCapacity = frontier;
@@ -320,20 +328,18 @@ sk_status Batch::prepare(BatchLane& l, const sk_batch_view* views, uint32_t coun
       pb.groups += patchListGroups(c.patches);
       rowBytes += patchListRowBytes(c.capacity, c.patches, pb.cells);
     }
-    void* before[3] = {l.patchLists.ptr, l.patchStatus.ptr, l.patchViews.ptr};
+    const void* const before[4] = {l.patchLists.ptr, l.patchStatus.ptr, l.patchViews.ptr, l.hostPatchViews.ptr};
     cudaError_t e = l.patchLists.allocateOn(
         rowBytes > l.patchLists.bytes ? std::max<uint64_t>(rowBytes, l.patchLists.bytes + l.patchLists.bytes / 2)
                                       : rowBytes, l.stream);
     if (e == cudaSuccess) e = l.patchStatus.allocateOn(size_t{pb.groups} * 8, l.stream);
     if (e == cudaSuccess) e = l.patchViews.allocateOn(size_t{count} * sizeof(PatchListView), l.stream);
     if (e == cudaSuccess) e = l.hostPatchViews.allocate(size_t{count} * sizeof(PatchListView));
+    if (before[0] != l.patchLists.ptr || before[1] != l.patchStatus.ptr || before[2] != l.patchViews.ptr ||
+        before[3] != l.hostPatchViews.ptr)
+      dropGraph(l);  // a captured graph points at the old buffers
     if (e != cudaSuccess) return check(e, "batch lists");
     std::memcpy(l.hostPatchViews.ptr, patchViews.data(), size_t{count} * sizeof(PatchListView));
-    if (before[0] != l.patchLists.ptr || before[1] != l.patchStatus.ptr || before[2] != l.patchViews.ptr) {
-      if (l.graph) cudaGraphExecDestroy(l.graph);  // a captured graph points at the old buffers
-      l.graph = nullptr;
-      l.graphShape.clear();
-    }
   }
   std::memcpy(l.hostViews.ptr, l.table.data(), size_t{count} * sizeof(BatchView));
   std::memcpy(l.hostCameras.ptr, l.cams.data(), size_t{count} * sizeof(Camera));
@@ -632,8 +638,7 @@ sk_status Batch::enqueue(BatchLane& l) {
   if (e != cudaSuccess) return check(e, "batch");
   if (useGraph) {
     if (!l.graph || l.graphShape != shape) {
-      if (l.graph) cudaGraphExecDestroy(l.graph);
-      l.graph = nullptr;
+      dropGraph(l);
       cudaGraph_t g = nullptr;
       e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
       if (e != cudaSuccess) return check(e, "graph capture");

@@ -117,6 +117,8 @@ struct Batch {
   sk_status fail(sk_status code, const std::string& message);
   sk_status check(cudaError_t e, const char* what);
   uint32_t nextEpoch(uint32_t n);
+  // Forgets the lane's captured graph (buffers it points at have moved).
+  void dropGraph(BatchLane& lane);
   sk_status reserve(BatchLane& lane, uint32_t sources, uint32_t instances, uint32_t items,
                     uint32_t tiles, uint32_t views, uint64_t pixels);
   // The LOD views' cuts (indices in total), reports and selection scratch (frontier entries).
