@@ -39,6 +39,12 @@ sk_status sk_testing_fail_next_check(sk_context* ctx, int32_t cuda_error);
  * past the frame's last does nothing. */
 sk_status sk_testing_withhold_sort_status(sk_context* ctx, uint32_t tile);
 
+/* After `after` that pass, one step on an image's way to the host fails as if the device were out of
+ * memory: the launch of a band (a large target drawn to be read at once is drawn in up to 8), the
+ * copy of a band, or the copy of a batch view's (or several views') image. Steps are counted over all
+ * contexts and batches. */
+void sk_testing_fail_image_step(uint32_t after);
+
 #ifdef __cplusplus
 }
 #endif

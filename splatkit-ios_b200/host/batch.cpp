@@ -566,13 +566,16 @@ sk_status Batch::enqueueImages(BatchLane& l) {
     const uint32_t first = k ? ends[k - 1] : 0u, last = ends[k];
     if (aside) e = cudaStreamWaitEvent(copies, l.composited[k], 0);
     if (l.destinations.empty()) {
+      if (e == cudaSuccess && testImageStepFails()) e = cudaErrorMemoryAllocation;
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(static_cast<uint8_t*>(l.hostImage.ptr) + pixelAt(first) * 4, image + pixelAt(first) * 4,
                             (pixelAt(last) - pixelAt(first)) * 4, cudaMemcpyDeviceToHost, copies);
     } else {
       for (uint32_t v = first; v < last && e == cudaSuccess; ++v) {
         const BatchView& t = l.table[v];
-        if (l.destinations[v])
+        if (testImageStepFails())
+          e = cudaErrorMemoryAllocation;
+        else if (l.destinations[v])
           e = cudaMemcpyAsync(l.destinations[v], image + t.pixelOffset * 4, size_t{t.width} * t.height * 4,
                               cudaMemcpyDeviceToHost, copies);
       }
@@ -661,7 +664,11 @@ sk_status Batch::enqueue(BatchLane& l) {
     if (e != cudaSuccess) return check(e, "graph launch");
   } else {
     st = body(false);
-    if (st != SK_OK) return st;
+    if (st != SK_OK) {  // copies into the caller's buffers may be on their way
+      cudaStreamSynchronize(s);
+      if (l.copyStream) cudaStreamSynchronize(l.copyStream);
+      return st;
+    }
   }
   e = cudaEventRecord(l.end, s);
   if (e == cudaSuccess) e = cudaEventRecord(l.done, s);

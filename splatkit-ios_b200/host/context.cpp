@@ -40,6 +40,14 @@ bool testAllocationFails() {
 }
 }  // namespace
 
+std::atomic<uint32_t> gTestFailedImageStep{0};
+
+bool testImageStepFails() {
+  for (uint32_t left = gTestFailedImageStep.load(); left > 0;)
+    if (gTestFailedImageStep.compare_exchange_weak(left, left - 1)) return left == 1;
+  return false;
+}
+
 cudaError_t DeviceBuffer::allocate(size_t n) {
   n = std::max<size_t>(n, 256);
   if (n <= bytes && ptr) return cudaSuccess;
@@ -497,11 +505,13 @@ cudaError_t Context::enqueueBands(const CompositeArgs& whole, uint32_t bandRows,
     c.firstTile = row * c.tilesX;
     c.tiles = std::min(bandRows, c.tilesY - row) * c.tilesX;
     const cudaStream_t on = k & 1u ? bands.side : s;
-    e = launchComposite(c, on);
+    e = testImageStepFails() ? cudaErrorMemoryAllocation : launchComposite(c, on);
     if (e == cudaSuccess) e = cudaEventRecord(bands.drawn[k], on);
   }
   // the frame is done when the last band of the side stream is, too
   if (k > 1 && e == cudaSuccess) e = cudaStreamWaitEvent(s, bands.drawn[k & 1u ? k - 2 : k - 1], 0);
+  // a failed frame: the next one on the frame's stream would not wait for the side stream's bands
+  if (e != cudaSuccess) cudaStreamSynchronize(bands.side);
   return e;
 }
 
@@ -512,7 +522,7 @@ cudaError_t Context::copyBands(void* host, const Slot& slot) {
   cudaError_t e = cudaSuccess;
   for (uint32_t k = 0; k * pixels < slot.height && e == cudaSuccess; ++k) {
     const uint32_t first = k * pixels, rows = std::min(pixels, slot.height - first);
-    e = cudaStreamWaitEvent(bands.copies, bands.drawn[k], 0);
+    e = testImageStepFails() ? cudaErrorMemoryAllocation : cudaStreamWaitEvent(bands.copies, bands.drawn[k], 0);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(static_cast<uint8_t*>(host) + first * row, image + first * row, rows * row,
                           cudaMemcpyDeviceToHost, bands.copies);
@@ -1118,7 +1128,9 @@ sk_status sk_read_image(sk_context* handle, void* host, size_t bytes, int32_t fo
     if (ctx->inFlight.size() == 1) ctx->bands.wanted = true;
     cudaError_t e = slot.bandRows ? ctx->copyBands(host, slot)
                                   : cudaMemcpyAsync(host, ctx->imageOf(slot.image), need, cudaMemcpyDeviceToHost, copies);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(copies);
+    // (also after a failure: the buffer is the caller's again when the call returns)
+    const cudaError_t landed = cudaStreamSynchronize(copies);
+    if (e == cudaSuccess) e = landed;
     const sk_status copied = ctx->check(e, "readback");
     if (copied != SK_OK) return copied;
     const sk_status finished = ctx->finishFrame(true);

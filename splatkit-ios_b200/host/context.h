@@ -30,6 +30,10 @@ inline int hostThreadsPublic() {
 // Test hooks (sk_testing_fail_device_allocations, sk_testing_pass_device_allocations): how many of the
 // next device allocations fail, and how many pass before those.
 extern std::atomic<uint32_t> gTestFailedAllocations, gTestPassedAllocations;
+// Test hook (sk_testing_fail_image_step): how many band launches and image copies on, counted from 1,
+// one fails (0: none); and whether the one asked about now does.
+extern std::atomic<uint32_t> gTestFailedImageStep;
+bool testImageStepFails();
 
 // Owning device allocation; allocate() only grows, and keeps the old memory when it fails.
 struct DeviceBuffer {

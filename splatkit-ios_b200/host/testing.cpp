@@ -27,4 +27,6 @@ sk_status sk_testing_withhold_sort_status(sk_context* handle, uint32_t tile) {
   return SK_OK;
 }
 
+void sk_testing_fail_image_step(uint32_t after) { sk::gTestFailedImageStep.store(after + 1); }
+
 }  // extern "C"

@@ -278,6 +278,7 @@ _SIGNATURES = {
     "sk_testing_pass_device_allocations": (None, [ctypes.c_uint32]),
     "sk_testing_fail_next_check": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32]),
     "sk_testing_withhold_sort_status": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_uint32]),
+    "sk_testing_fail_image_step": (None, [ctypes.c_uint32]),
 }
 
 _lib: Optional[ctypes.CDLL] = None
@@ -1021,6 +1022,11 @@ def testing_fail_device_allocations(count: int, after: int = 0):
     those after `after` that pass."""
     library().sk_testing_fail_device_allocations(count)
     library().sk_testing_pass_device_allocations(after)
+
+
+def testing_fail_image_step(after: int):
+    """Test hook: after `after` that pass, one band launch or image copy fails as out of memory."""
+    library().sk_testing_fail_image_step(after)
 
 
 def sort_workspace_bytes(capacity: int) -> int:
