@@ -45,6 +45,15 @@ sk_status sk_testing_withhold_sort_status(sk_context* ctx, uint32_t tile);
  * contexts and batches. */
 void sk_testing_fail_image_step(uint32_t after);
 
+/* The last finished frame's lists as its kernels wrote them, where it drew from direct lists that
+ * nothing has overwritten since (else SK_E_INVALID): grid[3] = log2 of a patch's edge in 32x32
+ * binning cells, patches per row and per column; ranges[2 * p] .. ranges[2 * p + 1] the entries of
+ * patch p (row major); per entry the projected index and the cells of the patch it touches (bit
+ * (y % edge) * edge + x % edge of cell (x, y); 1 where a patch is one cell). *count receives the
+ * number of entries, of which min(count, capacity) are copied. */
+sk_status sk_testing_read_patch_lists(sk_context* ctx, uint32_t* grid, uint32_t* ranges, uint32_t* values,
+                                      uint16_t* masks, uint32_t capacity, uint32_t* count);
+
 #ifdef __cplusplus
 }
 #endif

@@ -279,6 +279,9 @@ _SIGNATURES = {
     "sk_testing_fail_next_check": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32]),
     "sk_testing_withhold_sort_status": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_uint32]),
     "sk_testing_fail_image_step": (None, [ctypes.c_uint32]),
+    "sk_testing_read_patch_lists": (ctypes.c_int32, [ctypes.c_void_p, _u32p, _u32p, _u32p,
+                                                     ctypes.POINTER(ctypes.c_uint16), ctypes.c_uint32,
+                                                     _u32p]),
 }
 
 _lib: Optional[ctypes.CDLL] = None
@@ -546,6 +549,18 @@ class Renderer:
     def upload_tile(self, offset: int, cloud: Cloud):
         v = cloud.view()
         self._check(self._lib.sk_upload_tile(self._h, offset, ctypes.byref(v)), "tile")
+
+    def testing_read_patch_lists(self):
+        """Test hook: (shift, patches per row, ranges, values, masks) of the last frame's direct lists."""
+        grid, n = np.zeros(3, np.uint32), ctypes.c_uint32()
+        self._check(self._lib.sk_testing_read_patch_lists(self._h, _ptr(grid, _u32p), None, None, None, 0,
+                                                          ctypes.byref(n)), "testing")
+        ranges = np.zeros((int(grid[1]) * int(grid[2]), 2), np.uint32)
+        values, masks = np.empty(n.value, np.uint32), np.empty(n.value, np.uint16)
+        self._check(self._lib.sk_testing_read_patch_lists(
+            self._h, _ptr(grid, _u32p), _ptr(ranges, _u32p), _ptr(values, _u32p),
+            _ptr(masks, ctypes.POINTER(ctypes.c_uint16)), n.value, ctypes.byref(n)), "testing")
+        return int(grid[0]), int(grid[1]), ranges, values, masks
 
     def testing_fail_next_check(self, cuda_error: int):
         """Test hook: the next CUDA status this context checks reads as `cuda_error`."""
