@@ -250,7 +250,9 @@ sk_status sk_set_part_styles(sk_context* ctx, const sk_part_style* palette, cons
  * two frames in flight (MetalFrameSlots.h:8): with both slots busy the call first finishes the
  * older frame. A LOD world keeps one. */
 sk_status sk_draw(sk_context* ctx, const sk_frame* frame);
-/* Waits for the last frame and copies its image (captureNextFrame). */
+/* Waits for the last frame and copies its image (captureNextFrame). The copy follows the drawing on
+ * the device, so that `host` may have been written when the call returns an error (SK_E_TIMEOUT of
+ * the frame among them); nothing writes it after the call returns. */
 sk_status sk_read_image(sk_context* ctx, void* host, size_t bytes, int32_t format);
 sk_status sk_wait_idle(sk_context* ctx);
 /* captureNextFrame (MetalSplatRenderer.mm:310-316): the next sk_draw also copies its image, in the
@@ -458,14 +460,15 @@ sk_status sk_radix_argsort_device(const uint32_t* d_keys, const uint32_t* d_coun
  * reference: its Metal sort owns its buffers. For callers that may not allocate device memory
  * while they run (cudaMalloc/cudaFree synchronise the whole device, which a render callback
  * with a frame deadline cannot afford) and for code that owns no device allocator. The call
- * allocates nothing and calls no allocating library; it enqueues two small memsets and the
- * sort kernels on `stream` and returns.
+ * allocates nothing and calls no allocating library; it enqueues the sort kernels on `stream`,
+ * above 32,768 keys after one small memset, and returns.
  *
  * Limit: capacity <= SK_NOALLOC_SORT_MAX_KEYS (1,048,576 keys); a larger capacity returns
  * SK_E_LIMIT and enqueues nothing. The workspace is a 13,115,648-byte array of this library's
- * device module, zero when the module loads. The histogram accumulators and tile counters in
- * it must be zero when a sort starts; each sort leaves them at zero and each call clears them
- * again first, so the caller clears nothing. d_keys, d_count, d_order, d_error and bits mean
+ * device module, zero when the module loads; a capacity of up to 32,768 keys is sorted in one
+ * launch that does not use it. The histogram accumulators and tile counters in it must be zero
+ * when another sort starts; each leaves them at zero and each call clears them again first, so
+ * the caller clears nothing. d_keys, d_count, d_order, d_error and bits mean
  * what they mean for sk_radix_argsort_device.
  *
  * Setup: the first call on each device (the device current on the calling thread) looks up the

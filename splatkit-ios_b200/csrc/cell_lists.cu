@@ -49,7 +49,7 @@ constexpr uint32_t kWarps = kThreads / 32;
 // long as one block, they take 256: 100k splats at 720p emit in 11 us against 16, the frame 213.6 against
 // 217.1; a thumbnail's frame 62.7 against 65.0. Above, 512 ranks halve the rows to scan. A batch whose
 // patches are all single cells takes 1024, whose spans then stay in registers (24 views of up to 640 x
-// 480: count, scan and emission 80, 23 and 205 us; at 512 ranks 88, 25 and 211); with larger patches 512.
+// 480: count, scan and emission 84, 23 and 205 us; at 512 ranks 88, 25 and 211); with larger patches 512.
 constexpr uint32_t kMostItems = 2;
 constexpr uint32_t kCellItems = 4;
 constexpr uint32_t kFewRanks = 148 * 4 * kThreads;
@@ -372,8 +372,11 @@ __device__ __forceinline__ void slotsFromCounts(uint32_t* slots, uint32_t words)
 
 // Pass 3 where every patch is one cell. The warp's spans stay in registers, and a masked span's cells are
 // staged by the lane that has it (a box of more than 64 cells by the whole warp): most splats of such
-// targets list one or two cells, so that the walk costs less than finding each position's span does (24 views
-// of up to 640 x 480: emission 265 -> 216 us against patchEmitKernel).
+// targets list one or two cells, so that the walk costs less than finding each position's span does, and a
+// box of many cells is walked twice, where patchEmitKernel's windows each walk it again. Whole frames against
+// patchEmitKernel's single-cell branch: 200k splats at 640 x 480 from 4 m 120 us and 177, 20k from 6 m 53 and
+// 67, 30k at 517 x 389 from 15 m 52.6 and 54.5, 1M at 400 x 300 210 and 201. 24 views of up to 640 x 480:
+// count, scan and emission 84, 23 and 205 us, there (at 512 ranks) 97, 25 and 192.
 template <uint32_t kItems>
 __global__ void __launch_bounds__(kThreads)
     cellEmitKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches) {
@@ -489,7 +492,6 @@ __global__ void __launch_bounds__(kThreads)
 // first slot for the block. A warp's entries, in depth order, are worked out kWindow positions at a
 // time, one position per lane and step (however many patches the items have), and staged as
 // (patch, item, cell mask); a warp of more entries works each further window out when it writes it.
-
 template <uint32_t kItems>
 __global__ void __launch_bounds__(kThreads)
     patchEmitKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches) {
@@ -546,11 +548,12 @@ __global__ void __launch_bounds__(kThreads)
   __syncthreads();  // the counters are zero, the starts there
 
   // Stages the entries at positions [w0, w1). Single-cell patches (a batch's small targets beside larger
-  // ones): every lane walks its items' listed cells (most items have one or two; a box of more than 64 cells is walked by the whole warp).
+  // ones, at kMostItems): every lane walks its items' listed cells (most items have one or two; a box of
+  // more than 64 cells is walked by the whole warp).
   // Larger patches: one position per lane and step; every item marks its first position, and an
   // entry's item is the last mark at or before its position (a running maximum).
   auto stageWindow = [&](uint32_t w0, uint32_t w1, uint32_t& carry, bool count) {
-    if (job.shift == 0) {
+    if (kItems == kMostItems && job.shift == 0) {
       auto put = [&](uint32_t patch, uint32_t pos, uint32_t item) {
         if (pos < w0 || pos >= w1) return;
         if (count) atomicAdd(mine + (patch >> 1), 1u << ((patch & 1u) * 16));

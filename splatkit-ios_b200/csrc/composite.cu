@@ -20,7 +20,7 @@
 // and 1/255 cutoff) is a fixed sequence of correctly rounded operations, bit-identical to the host
 // oracle's FP32 formula.
 //
-// Bound by instruction issue (73-77% of the issue slots, half of the ALU's): 1M splats at 1080p take 179M
+// Bound by instruction issue (73% of the issue slots, half of the ALU's): 1M splats at 1080p take 179M
 // warp instructions and 203 us, 26M of them the filter and the staging of records that miss the tile.
 // The exponential predicated on the coverage, no minimum where no peak is above 1, a quarter of a load
 // per entry for its place and packed row terms took the sweep's entry from 35 instructions to 31

@@ -21,19 +21,19 @@ namespace sk {
 namespace {
 
 // The workspace size of radix_sort.cu's layout for SK_NOALLOC_SORT_MAX_KEYS keys: three
-// 4-byte-per-key buffers, 2 x 4 x 256 histogram words, one 256-word status row of 8-byte words
-// per 4096-key tile, and the counters, each part rounded up to 256 bytes. The first call checks
+// 4-byte-per-key buffers, 2 x 4 x 256 histogram words, the counters, and one 256-word status row of
+// 8-byte words per 4096-key tile, each part rounded up to 256 bytes. The first call checks
 // it against sortWorkspaceBytes() and refuses to run if the layout ever outgrows it.
 constexpr size_t roundUp256(size_t v) { return (v + 255) / 256 * 256; }
 constexpr size_t kNoAllocKeys = SK_NOALLOC_SORT_MAX_KEYS;
 constexpr size_t kNoAllocScratchBytes = 3 * roundUp256(kNoAllocKeys * 4) + roundUp256(2 * 4 * 256 * 4) +
-                                        roundUp256((kNoAllocKeys + 4095) / 4096 * 256 * 8) +
-                                        roundUp256(5 * 2 * 4);
+                                        roundUp256(5 * 2 * 4) +
+                                        roundUp256((kNoAllocKeys + 4095) / 4096 * 256 * 8);
 
-// Zero when the module loads. The histogram accumulators and the tile counters must be zero
-// when a sort starts: every completed sort leaves them at zero, and each call clears them again
-// before it sorts (two small memsets on the caller's stream), so a sort cut short by an error
-// cannot poison the next one. The status words need no clearing while the 30-bit epochs are
+// Zero when the module loads. Calls of up to 32,768 keys sort in one launch (cluster_sort.cu) and do not
+// use it. The others need the histogram accumulators and the tile counters at zero when they start: every
+// completed sort leaves them so, and each call clears them again before it sorts (one memset on the
+// caller's stream), so a sort cut short by an error cannot poison the next one. The status words need no clearing while the 30-bit epochs are
 // new: each call takes four (one per pass). When the epoch counter wraps, after 2^28 calls, the
 // call that wraps it zeroes the status words first (a flag of 0 never matches), so a word left
 // by a sort 2^28 calls earlier cannot pass for one of the new epochs.
