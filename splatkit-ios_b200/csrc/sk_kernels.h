@@ -234,6 +234,8 @@ struct CompositeArgs {
   uint32_t firstTile, tiles;
   const BatchView* views;
   uint32_t viewCount;
+  uint32_t records;  // about how many records the lists before this launch were made of (0: few, or no
+                     // lists right before it)
 };
 cudaError_t launchComposite(const CompositeArgs& args, cudaStream_t stream);
 

@@ -541,6 +541,7 @@ sk_status Batch::enqueueImages(BatchLane& l) {
   c.views = static_cast<const BatchView*>(l.viewTable.ptr);
   c.patches = l.directLists ? 1u : 0u;
   c.viewCount = l.viewCount;
+  for (const BatchView& t : l.table) c.records += t.indices ? 0u : t.count;  // (a cut's length is not known here)
   const std::vector<uint32_t> ends = compositeChunks(l);
   const bool aside = ends.size() > 1;
   cudaError_t e = cudaSuccess;

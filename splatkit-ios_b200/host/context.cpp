@@ -490,6 +490,8 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
     c.countFragments = timing == 1 ? 1u : 0u;
     c.loaded = &fc->loaded;
     c.tiles = tilesX * tilesY;
+    // (a LOD frame's cut is about that of the frame before, which has finished)
+    c.records = view.bandRows ? 0u : lod ? lastCounters.lod[0] : total;
     e = view.bandRows ? enqueueBands(c, view.bandRows, s) : launchComposite(c, s);
   }
   if (timing != 0) cudaEventRecord(events[5], s);
