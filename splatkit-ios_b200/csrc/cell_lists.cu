@@ -27,8 +27,7 @@
 // the composite 193 -> 203. 3M at 3840 x 2160 (8160 cells, 510 patches): 164 us against 668 for the
 // stable sort of (cell, splat) pairs that lists per cell needed there. Small targets keep patches of one
 // cell: their cell grid is small, and many entries of a patch would miss a tile's cell (24 views of up
-// to 640 x 480: composite 1342 us, 1620 with 4 x 4 patches). The line at 320 patches: 1080p at 2 x 2
-// (510 patches) emits in 56 us and composites in 206, at 4 x 4 in 32 and 203.
+// to 640 x 480: composite 1342 us, 1620 with 4 x 4 patches). Where the lines lie stands at PatchGoals.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -71,6 +70,7 @@ struct Work {
   uint32_t viewCount;
   const uint32_t* viewFirst;
   uint8_t* base;
+  PatchGrid grid;  // a frame's patches
 };
 
 // What one block of a pass works on: its block (or patch group) within its view, the view's ranks
@@ -98,10 +98,9 @@ __device__ __forceinline__ Job jobOf(const BinArgs& a, const Work& w, uint32_t p
     j.block = index;
     j.first = 0;
     j.n = min(*a.count, a.capacity);
-    const PatchGrid g = patchGrid(a.tilesX, a.tilesY);
     j.patches = patches;
-    j.patchesX = g.x;
-    j.shift = g.shift;
+    j.patchesX = w.grid.x;
+    j.shift = w.grid.shift;
     j.blockRows = w.blockRows;
     j.ranges = ranges;
     return j;
@@ -125,8 +124,9 @@ __device__ __forceinline__ Job jobOf(const BinArgs& a, const Work& w, uint32_t p
 // nothing but look-back words), then the block rows.
 constexpr size_t kStatusBytes = size_t{kDirectMaxPatches / kGroup} * 8;
 
-Work workOf(void* workspace) {
+Work workOf(void* workspace, PatchGrid grid) {
   Work w{};
+  w.grid = grid;
   w.status = static_cast<uint64_t*>(workspace);
   w.blockRows = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(workspace) + kStatusBytes);
   return w;
@@ -373,10 +373,10 @@ __device__ __forceinline__ void slotsFromCounts(uint32_t* slots, uint32_t words)
 // Pass 3 where every patch is one cell. The warp's spans stay in registers, and a masked span's cells are
 // staged by the lane that has it (a box of more than 64 cells by the whole warp): most splats of such
 // targets list one or two cells, so that the walk costs less than finding each position's span does, and a
-// box of many cells is walked twice, where patchEmitKernel's windows each walk it again. Whole frames against
-// patchEmitKernel's single-cell branch: 200k splats at 640 x 480 from 4 m 120 us and 177, 20k from 6 m 53 and
-// 67, 30k at 517 x 389 from 15 m 52.6 and 54.5, 1M at 400 x 300 210 and 201. 24 views of up to 640 x 480:
-// count, scan and emission 84, 23 and 205 us, there (at 512 ranks) 97, 25 and 192.
+// box of many cells is walked twice, where patchEmitKernel's windows each walk it again. Whole frames of single
+// cells against patchEmitKernel's single-cell branch: 200k splats at 640 x 480 from 4 m 120 us and 177, 20k from
+// 6 m 53 and 67, 30k at 517 x 389 from 15 m 52.6 and 54.5, 1M at 400 x 300 210 and 201. 24 views of up to 640 x
+// 480: count, scan and emission 84, 23 and 205 us, there (at 512 ranks) 97, 25 and 192.
 template <uint32_t kItems>
 __global__ void __launch_bounds__(kThreads)
     cellEmitKernel(const __grid_constant__ BinArgs a, Work work, uint32_t patches) {
@@ -652,6 +652,8 @@ size_t countDynamicBytes(uint32_t patches) { return size_t{patches} * sizeof(uin
 
 }  // namespace
 
+PatchGoals patchGoalsFor(uint32_t capacity) { return capacity <= kFewRanks ? kSmallPatches : kFramePatches; }
+
 bool patchListsFit(uint32_t patches) { return patches > 0 && patches <= kDirectMaxPatches; }
 
 uint32_t patchListBlocks(uint32_t capacity, bool cells) {
@@ -697,7 +699,7 @@ cudaError_t launchPasses(uint32_t items, bool cells, const BinArgs& a, const Wor
 cudaError_t patchListsConfigure() {
   static std::atomic<uint64_t> done{0};
   return oncePerDevice(done, [] {
-    // targets of single-cell patches have at most kPatchGoal of them: within the default limit
+    // targets of single-cell patches have at most 320 of them: within the default limit
     const int most = static_cast<int>(emitDynamicBytes(kDirectMaxPatches));
     const cudaError_t e =
         cudaFuncSetAttribute(patchEmitKernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
@@ -708,10 +710,10 @@ cudaError_t patchListsConfigure() {
 }
 
 cudaError_t launchPatchLists(const BinArgs& a, const PatchLists& lists, cudaStream_t stream) {
-  const PatchGrid g = patchGrid(a.tilesX, a.tilesY);
+  const PatchGrid g = lists.grid;
   const uint32_t patches = g.x * g.y, items = itemsFor(a.capacity);
   if (!patchListsFit(patches) || a.capacity == 0) return cudaErrorInvalidValue;
-  return launchPasses(items, g.shift == 0, a, workOf(lists.workspace), patches, blocksOf(a.capacity, items),
+  return launchPasses(items, g.shift == 0, a, workOf(lists.workspace, g), patches, blocksOf(a.capacity, items),
                       groupsOf(patches), lists.ranges, lists.entryCount, lists.counters, lists.epoch, lists.error,
                       stream);
 }

@@ -257,8 +257,7 @@ __global__ void __launch_bounds__(kThreads) compositeKernel(const __grid_constan
   __shared__ std::conditional_t<kPatches, FilterSmem, uint32_t> filter;
   Target t{a.width, a.height, a.tilesX, a.firstTile + blockIdx.x, a.binsX, 0u, 0u, 0u, a.image};
   if constexpr (kPatches && !kBatch) {
-    const PatchGrid g = patchGrid(a.binsX, (a.tilesY + 1) / 2);
-    t.patchesX = g.x, t.patchShift = g.shift;
+    t.patchesX = a.grid.x, t.patchShift = a.grid.shift;
   }
   if constexpr (kBatch) {
     const uint32_t tile = a.firstTile + blockIdx.x;
@@ -271,7 +270,7 @@ __global__ void __launch_bounds__(kThreads) compositeKernel(const __grid_constan
     t.binsX = __ldg(&v->binsX);
     t.listBase = a.patches ? __ldg(&v->patchBase) : __ldg(&v->binBase);
     if constexpr (kPatches) {
-      const PatchGrid g = patchGrid(t.binsX, __ldg(&v->binsY));
+      const PatchGrid g = patchGrid(t.binsX, __ldg(&v->binsY), kSmallPatches);
       t.patchesX = g.x, t.patchShift = g.shift;
     }
     t.image = static_cast<char*>(a.image) +

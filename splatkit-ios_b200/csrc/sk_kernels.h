@@ -157,13 +157,14 @@ cudaError_t launchTileRanges(const uint32_t* sortedKeys, const uint32_t* instanc
                              uint32_t instanceCapacity, uint2* ranges, uint32_t tiles,
                              cudaStream_t stream);
 
-// Direct lists (cell_lists.cu) on targets of at most kDirectMaxPatches patches (patchGrid): per patch, the front-to-back projected indices of the survivors whose cell box touches it, each
-// with the bits of the cells it touches there. A cell's entries are those of its patch with its
+// Direct lists (cell_lists.cu) on targets of at most kDirectMaxPatches patches (patchGrid): per patch, the
+// front-to-back projected indices of the survivors whose cell box touches it, each with the bits of the cells it touches there. A cell's entries are those of its patch with its
 // bit, the same list that binning + stable tile sort + ranges produce. args.instanceValues and
 // args.instanceMasks receive the entries, args.instanceCount the number of (survivor, cell) pairs;
 // instanceKeys and blockSums are unused.
 constexpr uint32_t kDirectMaxPatches = 4096;
 struct PatchLists {
+  PatchGrid grid;        // the target's patches, by patchGoalsFor(args.capacity)
   void* workspace;       // patchListBytes(capacity, patches), the first patchListStatusBytes() zero
                          // before the first launch
   uint2* ranges;         // per patch [start, end), clamped to the instance capacity
@@ -172,6 +173,8 @@ struct PatchLists {
   uint32_t epoch;        // look-back epoch, fresh per launch
   uint32_t* error;       // SK_DEVERR_* bits
 };
+// How many patches the target of a frame of up to `capacity` ranks gets.
+PatchGoals patchGoalsFor(uint32_t capacity);
 // Whether a target of `patches` patches takes the direct path.
 bool patchListsFit(uint32_t patches);
 size_t patchListBytes(uint32_t capacity, uint32_t patches);
@@ -217,6 +220,7 @@ struct CompositeArgs {
   const Projected* projected;
   const uint32_t* values;  // list entries' projected indices, front to back
   const uint16_t* masks;   // direct lists: each entry's cells of its patch; null: lists per cell
+  PatchGrid grid;          // direct lists of a frame: the target's patches
   uint32_t patches;        // a batch: 1 when the views' lists start at their patchBase (else binBase)
   const uint2* ranges;     // per patch (direct lists) or per binning cell
   uint32_t width, height, tilesX, tilesY;  // composite tiles (kTileSize pixels)

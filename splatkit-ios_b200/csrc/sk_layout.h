@@ -137,22 +137,33 @@ constexpr uint32_t kBinSize = 2 * kTileSize;
 // lists: one entry per splat and patch it touches, with a bit for each of the patch's cells it
 // touches (bit (y % edge) * edge + x % edge of cell (x, y)).
 constexpr uint32_t kPatchShiftMost = 2;
-// The most patches a target gets while a larger edge is left. Larger patches mean fewer entries and shorter
-// rows for the lists, single cells no filter in the composite. Frames at 475 to 920 cells take the same to
-// 2% with goals of 160, 320, 512 and 1024 (1M splats at 1024 x 768: 254, 257, 257 and 257 us, at 800 x 600
-// 234, 233, 232 and 233); 1M at 1450 cells (1600 x 900) 315 with 320 and 325 with 512 or 1024, at 320 cells
-// (640 x 512) 215 with 320 and 221 with 160. So the line lies above the 300 cells of 640 x 480.
-constexpr uint32_t kPatchGoal = 320;
+// The most patches a target gets while a larger edge is left: of single cells, and of 2 x 2 cells. Larger
+// patches mean fewer entries and shorter rows for the lists, single cells no filter in the composite.
+// A frame's lists wait for the few warps with the splats nearest to the camera, whose boxes hold most of the
+// target: an entry per patch each. From amid the splats (5 to 8 m from the middle of a 20 m cube) frames of
+// 1.5M in flight take, us, with at most 320 patches of either kind, then as many as kFramePatches says: 640 x
+// 480 232 and 171, 1280 x 720 268 and 200, 800 x 600 213 and 170, 480 x 320 (150 cells) 156 and 132; from
+// outside (15 m) 172 and 173, 1024 x 768 alone 294 and 279, 480 x 320 174 and 187; 200k at 640 x 480 114 and 93
+// (5 m), 106 and 110 (15 m). At 400 x 300 (130 cells) single cells are no slower from amid the splats, and 170
+// against 176 from outside.
+// Where blocks take 256 ranks a warp has half as many such splats, and the composite's share is larger: 30k at
+// 517 x 389 (221 cells) read to floats 144 and 146. A batch's views fill the chip together: 12 views of 500k at
+// up to 640 x 480 1442 and 1480 (15 m), 1108 and 1072 (5 m). Both have kSmallPatches, above the 300 cells of
+// 640 x 480: frames at 475 to 920 cells take the same to 2% with 160, 320, 512 and 1024.
+struct PatchGoals {
+  uint32_t cells, squares;
+};
+constexpr PatchGoals kFramePatches{144, 80}, kSmallPatches{320, 320};
 struct PatchGrid {
   uint32_t shift, x, y;  // log2 of the edge; patches per row and column
 };
-// The patches of a target of binsX x binsY cells: the smallest edge with at most kPatchGoal patches.
+// The patches of a target of binsX x binsY cells: the smallest edge whose patches are within the goals.
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-inline PatchGrid patchGrid(uint32_t binsX, uint32_t binsY) {
+inline PatchGrid patchGrid(uint32_t binsX, uint32_t binsY, PatchGoals most) {
   PatchGrid g{0, binsX, binsY};
-  while (g.shift < kPatchShiftMost && g.x * g.y > kPatchGoal) {
+  while (g.shift < kPatchShiftMost && g.x * g.y > (g.shift == 0 ? most.cells : most.squares)) {
     ++g.shift;
     g.x = (binsX + (1u << g.shift) - 1) >> g.shift;
     g.y = (binsY + (1u << g.shift) - 1) >> g.shift;

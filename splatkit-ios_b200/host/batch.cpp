@@ -295,7 +295,7 @@ sk_status Batch::prepare(BatchLane& l, const sk_batch_view* views, uint32_t coun
   uint32_t mostPatches = 1;
   l.patchMasks = false;
   for (const BatchView& t : l.table) {
-    const PatchGrid g = patchGrid(t.binsX, t.binsY);
+    const PatchGrid g = patchGrid(t.binsX, t.binsY, kSmallPatches);
     mostPatches = std::max(mostPatches, g.x * g.y);
     if (g.shift) l.patchMasks = true;  // patches of one cell need no masks
   }
@@ -315,7 +315,7 @@ sk_status Batch::prepare(BatchLane& l, const sk_batch_view* views, uint32_t coun
       BatchView& t = l.table[v];
       PatchListView& c = patchViews[v];
       c.capacity = std::max(t.count, 1u);
-      const PatchGrid g = patchGrid(t.binsX, t.binsY);
+      const PatchGrid g = patchGrid(t.binsX, t.binsY, kSmallPatches);
       c.patches = g.x * g.y;
       c.patchesX = g.x;
       c.shift = g.shift;

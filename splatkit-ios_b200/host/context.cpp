@@ -185,9 +185,9 @@ sk_status Context::reserveScratch(FrameScratch& f, uint32_t sources, uint32_t in
   grab(f.instValuesSorted, size_t{instances} * 4);
   grab(f.tileSortWorkspace, sortWorkspaceBytesFor(instances, kTileSortTileKeys));
   grab(f.ranges, size_t{maxTiles} * sizeof(uint2));
-  // a target of t composite tiles has at most kPatchGoal patches, or t / 8 + 1 of the largest
-  grab(f.patchLists, patchListBytes(sources, std::min(std::max(std::max(maxTiles, f.maxTiles) / 8 + 1, kPatchGoal),
-                                                      kDirectMaxPatches)));
+  // a target of t composite tiles has at most kSmallPatches.cells patches, or t / 8 + 1 of the largest
+  grab(f.patchLists, patchListBytes(sources, std::min(std::max(std::max(maxTiles, f.maxTiles) / 8 + 1,
+                                                               kSmallPatches.cells), kDirectMaxPatches)));
   grab(f.rangeBuffer, size_t{kMaxRanges} * sizeof(Range));
   grab(f.rangeStarts, size_t{kMaxRanges + 1} * 4);
   const bool fresh = f.counters.ptr == nullptr;
@@ -343,7 +343,7 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
   uint32_t* error = &fc->error;
   const bool direct = view.direct;
   // patches of one cell are cell lists: their entries need no masks
-  uint16_t* masks = direct && view.patches().shift ? static_cast<uint16_t*>(f.instKeysSorted.ptr) : nullptr;
+  uint16_t* masks = direct && view.patches.shift ? static_cast<uint16_t*>(f.instKeysSorted.ptr) : nullptr;
   cudaError_t e = cudaMemsetAsync(fc, 0, sizeof(FrameCounters), s);
   // Direct lists write every range; the sorted path only those of non-empty cells.
   if (e == cudaSuccess && !direct) e = clearTileRanges(static_cast<uint2*>(f.ranges.ptr), binsX * binsY, s);
@@ -463,6 +463,7 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
     b.instanceCount = &fc->instances;
     b.overflow = &fc->overflow;
     PatchLists pl{};
+    pl.grid = view.patches;
     pl.workspace = f.patchLists.ptr;
     pl.ranges = static_cast<uint2*>(f.ranges.ptr);
     pl.entryCount = &fc->entries;
@@ -478,6 +479,7 @@ sk_status Context::enqueuePipeline(FrameScratch& f, const ViewTarget& view, cons
     c.projected = static_cast<const Projected*>(f.projected.ptr);
     c.values = static_cast<const uint32_t*>(f.instValuesSorted.ptr);
     c.masks = masks;
+    c.grid = view.patches;
     c.ranges = static_cast<const uint2*>(f.ranges.ptr);
     c.width = view.width, c.height = view.height, c.tilesX = tilesX, c.tilesY = tilesY;
     c.binsX = binsX;
@@ -644,7 +646,8 @@ sk_status Context::enqueueSlot(uint32_t index) {
   *static_cast<Camera*>(slot.hostCamera.ptr) = cameraFor(slot.frame, width, height);
   FrameScratch& f = scratchOf(index);
   ViewTarget view = plainView(slot);
-  const uint32_t patches = view.patches().x * view.patches().y;
+  slot.patches = view.patches = patchGrid(view.binsX(), view.binsY(), patchGoalsFor(f.sources));
+  const uint32_t patches = view.patches.x * view.patches.y;
   view.direct = binningMode == SK_BINNING_AUTO && patchListsFit(patches) &&
                 f.patchLists.bytes >= patchListBytes(f.sources, patches);
   slot.direct = view.direct;

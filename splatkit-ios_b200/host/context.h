@@ -114,13 +114,13 @@ struct ViewTarget {
   FrameCounters* hostCounters = nullptr;   // pinned; null: no readback
   const Camera* camera = nullptr;          // device, written before the pipeline runs (LOD worlds)
   const Camera* hostCamera = nullptr;      // the same on the host
+  PatchGrid patches{};                     // of the target
   bool direct = false;                     // lists per patch, written in place
   uint32_t bandRows = 0;                   // rows of tiles per band (Context::Bands); 0: one launch
   uint32_t tilesX() const { return (width + kTileSize - 1) / kTileSize; }
   uint32_t tilesY() const { return (height + kTileSize - 1) / kTileSize; }
   uint32_t binsX() const { return (width + kBinSize - 1) / kBinSize; }
   uint32_t binsY() const { return (height + kBinSize - 1) / kBinSize; }
-  PatchGrid patches() const { return patchGrid(binsX(), binsY()); }
 };
 
 // The per-view camera block of a frame on a width x height target.
@@ -169,6 +169,7 @@ struct Context {
     uint32_t total = 0, image = 0;
     uint32_t width = 0, height = 0;  // target it was drawn on
     uint32_t sources = 0;            // of its scratch when it was drawn
+    PatchGrid patches{};
     bool direct = false;             // its lists are per patch (csrc/cell_lists.cu)
     uint32_t bandRows = 0;           // rows of tiles per band it was drawn in; 0: one launch
     uint64_t number = 0;  // the submitted-frame count it was drawn as

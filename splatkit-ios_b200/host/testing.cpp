@@ -40,8 +40,7 @@ sk_status sk_testing_read_patch_lists(sk_context* handle, uint32_t* grid, uint32
   const sk::Context::Slot& slot = ctx->slots[ctx->lastSlot];
   const sk::FrameScratch& f = ctx->scratchOf(ctx->lastSlot);
   if (!slot.direct || ctx->listsPerCell || !f.spansKept) return SK_E_INVALID;
-  const sk::PatchGrid g = sk::patchGrid((slot.width + sk::kBinSize - 1) / sk::kBinSize,
-                                        (slot.height + sk::kBinSize - 1) / sk::kBinSize);
+  const sk::PatchGrid g = slot.patches;
   grid[0] = g.shift, grid[1] = g.x, grid[2] = g.y;
   *count = ctx->lastCounters.entries;
   const size_t copy = std::min({*count, capacity, f.instanceCapacity});

@@ -39,7 +39,12 @@ def cell_lists(lists, w, h):
     (80_000, 1920, 1080, -2.5, 2),
     (3_000, 1920, 1080, 0.7, 2),     # boxes of hundreds of cells
     (200_000, 3840, 2160, -2.0, 2),  # more than 151,552 sources: blocks of 512 ranks
-    (160_000, 640, 480, -3.0, 0),
+    (160_000, 400, 300, -3.0, 0),
+    (160_000, 640, 480, -3.0, 1),    # larger patches from 145 cells, and from 81 patches of 2 x 2, up
+    (151_553, 384, 384, -2.5, 0),    # 144 cells
+    (151_553, 385, 384, -2.0, 1),
+    (151_553, 640, 512, -1.0, 1),    # 80 patches; several windows
+    (151_553, 641, 512, -2.5, 2),
     (1, 33, 17, -1.0, 0),
 ])
 def test_patch_lists_hold_the_cells_lists(cuda_device, n, w, h, log_scale, shift):
