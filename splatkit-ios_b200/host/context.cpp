@@ -272,7 +272,8 @@ sk_status Context::reserveView(uint32_t w, uint32_t h) {
     if (e == cudaSuccess) e = sl.hostCamera.allocate(sizeof(Camera));
   }
   // Made with the view (0.23 ms of its 2.8) and not by the first frame in bands: behind its lists the larger
-  // frames hide that, but a first one of 100k splats at 720p was read in 320 us instead of 220.
+  // frames hide that, but a first one of 100k splats at 720p was read in 320 us instead of 220. (A first frame
+  // in one launch instead: 1M splats at 1080p read in 561 us, in bands in 440; 1M at 3840 x 2160 1417 and 967.)
   if (bandRowsFor(w, h)) {
     for (cudaStream_t* st : {&bands.side, &bands.copies})
       if (e == cudaSuccess && !*st) e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
@@ -1118,6 +1119,23 @@ sk_status sk_wait_idle(sk_context* handle) {
   return ctx->check(ctx->syncStreams(), "wait");
 }
 
+// Smaller images are copied to pageable memory in one piece: such a copy goes through the driver's staging
+// buffer and holds the calling thread, and each costs 20 to 40 us. Read there, in one launch and in bands, us,
+// over separate boxes: 100k splats at 720p 369 to 436 and 415 to 477, at 1080p 620 to 739 and 738 to 840, at 2560
+// x 1440 983 to 1183 and 1122 to 1333; 1M at 1080p 801 to 965 and 840 to 939, at 3840 x 2160 2475 to 3002 and
+// 2398 to 2724.
+constexpr size_t kPageablePixels = 5'000'000;
+
+// Whether copies to `host` run beside the calling thread (memory of cudaMallocHost or cudaHostRegister).
+static bool isPinned(const void* host) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeHost;
+}
+
 sk_status sk_read_image(sk_context* handle, void* host, size_t bytes, int32_t format) {
   SK_CTX(handle);
   if (!host) return SK_E_INVALID;
@@ -1131,10 +1149,14 @@ sk_status sk_read_image(sk_context* handle, void* host, size_t bytes, int32_t fo
     const uint32_t newest = ctx->inFlight.back();
     const uint64_t redraws = ctx->redraws;
     const sk::Context::Slot& slot = ctx->slots[newest];
-    const cudaStream_t copies = slot.bandRows ? ctx->bands.copies : ctx->streamOf(newest);
-    if (ctx->inFlight.size() == 1) ctx->bands.wanted = true;
-    cudaError_t e = slot.bandRows ? ctx->copyBands(host, slot)
-                                  : cudaMemcpyAsync(host, ctx->imageOf(slot.image), need, cudaMemcpyDeviceToHost, copies);
+    // (the frame's own stream waits for all of its bands)
+    const bool large = ctx->bandRowsFor(ctx->width, ctx->height) != 0;
+    const bool suits = large && (pixels >= kPageablePixels || isPinned(host));
+    const bool inBands = slot.bandRows && suits;
+    if (large && ctx->inFlight.size() == 1) ctx->bands.wanted = suits;
+    const cudaStream_t copies = inBands ? ctx->bands.copies : ctx->streamOf(newest);
+    cudaError_t e = inBands ? ctx->copyBands(host, slot)
+                            : cudaMemcpyAsync(host, ctx->imageOf(slot.image), need, cudaMemcpyDeviceToHost, copies);
     // (also after a failure: the buffer is the caller's again when the call returns)
     const cudaError_t landed = cudaStreamSynchronize(copies);
     if (e == cudaSuccess) e = landed;

@@ -176,17 +176,17 @@ struct Context {
   };
   Slot slots[kFrameSlots];
   std::deque<uint32_t> inFlight;  // slots of the frames in flight, oldest first
-  // A frame that is read as soon as it is drawn (sk_read_image with no other frame in flight) is drawn in
-  // bands, launches of some rows of tiles each, and the image of one band crosses to the host while the
-  // next ones are drawn. The bands take turns on the frame's stream and a side stream, so that a band's
-  // blocks fill the chip as the one before it drains.
+  // A frame that is read as soon as it is drawn (sk_read_image with no other frame in flight, into pinned memory
+  // or of a very large target) is drawn in bands, launches of some rows of tiles each, and the image of one band
+  // crosses to the host while the next ones are drawn. The bands take turns on the frame's stream and a side
+  // stream, so that a band's blocks fill the chip as the one before it drains.
   static constexpr uint32_t kMaxBands = 8;
   struct Bands {
     cudaStream_t side = nullptr, copies = nullptr;
     cudaEvent_t listed = nullptr, drawn[kMaxBands] = {};
-    // Whether the last frame drawn in bands was read while it was the only one in flight. A program that
-    // draws without reading goes without them after one frame: short bands wait for their deepest tiles
-    // one after the other (a LOD frame at 1080p, not read: 277 us in one launch, 340 in six).
+    // Whether the last frame was read so (the first frame: true). A program that draws without reading goes
+    // without bands after one frame: short ones wait for their deepest tiles one after the other (a LOD frame at
+    // 1080p, not read: 277 us in one launch, 340 in six).
     bool wanted = true;
   } bands;
   uint32_t bandRowsFor(uint32_t width, uint32_t height) const;
