@@ -73,6 +73,13 @@ uint32_t Batch::nextEpoch(uint32_t n) {
   return e;
 }
 
+cudaError_t BatchLane::makeCopyStream() {
+  cudaError_t e = cudaSuccess;
+  if (!copyStream) e = cudaStreamCreateWithFlags(&copyStream, cudaStreamNonBlocking);
+  if (e == cudaSuccess && !copied) e = cudaEventCreateWithFlags(&copied, cudaEventDisableTiming);
+  return e;
+}
+
 namespace {
 uint32_t bitsFor(uint64_t values) {  // key bits, a multiple of 8, for keys < values
   uint32_t b = 8;
@@ -544,9 +551,7 @@ sk_status Batch::enqueueImages(BatchLane& l) {
   for (const BatchView& t : l.table) c.records += t.indices ? 0u : t.count;  // (a cut's length is not known here)
   const std::vector<uint32_t> ends = compositeChunks(l);
   const bool aside = ends.size() > 1;
-  cudaError_t e = cudaSuccess;
-  if (aside && !l.copyStream) e = cudaStreamCreateWithFlags(&l.copyStream, cudaStreamNonBlocking);
-  if (aside && !l.copied && e == cudaSuccess) e = cudaEventCreateWithFlags(&l.copied, cudaEventDisableTiming);
+  cudaError_t e = aside ? l.makeCopyStream() : cudaSuccess;
   while (aside && e == cudaSuccess && l.composited.size() < ends.size()) {
     cudaEvent_t ev = nullptr;
     e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);

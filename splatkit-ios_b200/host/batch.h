@@ -94,6 +94,7 @@ struct BatchLane {
   // captured stage sequence and the shape it was captured for
   cudaGraphExec_t graph = nullptr;
   std::vector<uint64_t> graphShape;
+  cudaError_t makeCopyStream();
   ~BatchLane();
 };
 

@@ -263,6 +263,12 @@ sk_status sk_server_create(const sk_server_config* config, sk_server** out) {
         cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreate(&l.start) != cudaSuccess || cudaEventCreate(&l.end) != cudaSuccess)
       return SK_E_DEVICE;
+    // what a large batch needs beside its buffers, and the lists' view table (pinning memory can wait for
+    // the device): made here, not while requests wait
+    if (l.makeCopyStream() != cudaSuccess) return SK_E_DEVICE;
+    if (l.hostPatchViews.allocate(size_t{std::min(config->max_batch_views, 1024u)} * sizeof(sk::PatchListView)) !=
+        cudaSuccess)
+      cudaGetLastError();  // a batch that needs it says so
   }
   s->work = std::vector<sk::LaneWork>(config->lanes);
   sk::holdPooledMemory(config->device);
